@@ -63,7 +63,7 @@ uint64_t scene_key(const DevScene& S)
     return key_of({key_of(S.patches), key_of(S.nodes), key_of(S.indices), key_of(S.tables), key_of(S.disps),
                    key_of(S.bvhs), key_of(S.patchBase), key_of(S.objects), key_of(S.materials),
                    key_of(S.patchMaterial), key_of(S.lights), key_of(S.groupTop), key_of(S.groupLights),
-                   key_of(S.groupEnv), S.nobjects, S.nsurfaces, S.ngroups});
+                   key_of(S.groupEnv), key_of(S.qnodes), key_of(S.leafKeys), S.nobjects, S.nsurfaces, S.ngroups});
 }
 
 uint64_t query_key(const Query& q)

@@ -30,7 +30,12 @@ struct DevBVH
     uint32_t nodeBase, indexBase, tableBase, dispBase;
     uint32_t A, B, N, mask;  // h(k) = (A k + B + disp[k & mask]) mod N, src/rt/PerfectHashFunction.h:58-63
     unsigned long long Nmagic;  // ceil(2^64 / N): x mod N by multiplication (fastmod_u32)
-    uint32_t compressed;        // 1: every node has a record in the compressed mirror
+    uint32_t compressed;        // 1: every node of the walked tree has a record in the compressed mirror
+    uint32_t qnodeBase;         // the walked tree's first record there
+    // A patch BVH's walk tree (build_walk_bvh in scene.cu): a second tree over the same leaf boxes,
+    // split on the longest axis, whose nodes have the same heap keys at the same positions, so
+    // that both share one hash table.  EMPTY: none, the query engine walks the tree above.
+    uint32_t walkBase;
 };
 
 // x mod N for 32-bit x and N >= 1 with M = ceil(2^64 / N) (Lemire, Kaser,
@@ -72,6 +77,7 @@ struct DevScene
     const uint32_t* disps;
     const DevBVH* bvhs;        // [nsurfaces] patch BVHs, then the object-level BVH
     const uint32_t* patchBase; // first global patch of each surface
+    const uint32_t* leafKeys;  // per global patch: the heap key of its leaf (surfaces with a walk tree)
     const DevObject* objects;
     const DevMaterial* materials;
     const uint32_t* patchMaterial;

@@ -119,9 +119,8 @@ DevMaterial to_dev(const cgs_material& m)
 }
 
 // BezierSurface::buildBVH (src/rt/Primitive.cu:199-220): per-patch bounds of
-// the 16 projected points and their mean as the centroid; `out` takes the
-// tree (its split_mode set by the caller).
-void build_surface_bvh(const Surface& s, HostBVH& out)
+// the 16 projected points and their mean as the centroid.
+std::vector<Element> surface_elements(const Surface& s)
 {
     std::vector<Element> el(s.patchCount());
     for (uint32_t i = 0; i < el.size(); i++)
@@ -139,6 +138,13 @@ void build_surface_bvh(const Surface& s, HostBVH& out)
             for (int k = 0; k < 3; k++) e.centroid[k] = e.centroid[k] + inv * p[k];
         }
     }
+    return el;
+}
+
+// `out` takes the tree (its split_mode set by the caller).
+void build_surface_bvh(const Surface& s, HostBVH& out)
+{
+    std::vector<Element> el = surface_elements(s);
     out.build(el);
 }
 
@@ -319,16 +325,71 @@ int upload_lights(cgs_scene* sc)
 
 }  // namespace
 
+// A second tree over a surface's patches for the query engine to walk: the
+// same median halves, split on the longest axis.  Halving n elements gives
+// the same heap keys in the same pre-order whatever the axis, so a hash table
+// of the one tree's keys finds the other's nodes.
+void cgs::build_walk_bvh(const Surface& s, HostBVH& out)
+{
+    std::vector<Element> el = surface_elements(s);
+    out = HostBVH {};
+    for (const Element& e : el)
+        for (int k = 0; k < 3; k++)
+            if (!std::isfinite(e.bounds.lo[k]) || !std::isfinite(e.bounds.hi[k])) return;
+    out.split_mode = CGS_SPLIT_LONGEST;
+    out.build(el);
+    for (Node& n : out.nodes)
+        if (n.left == EMPTY) n.right = out.indices[n.right];  // a leaf names its patch
+    out.indices.clear();
+}
+
+// What the walk relies on: both trees have the same keys in the same order and
+// one leaf per patch, a patch's leaf box is the same in both, and every inner
+// box of the reference tree contains its children (the walk tree's do by
+// construction).  Trees built here have it; one read from a blob may not.
+void cgs::check_walk_bvh(Surface& s)
+{
+    const HostBVH &b = s.bvh, &w = s.walk;
+    if (w.nodes.empty()) return;
+    auto contains = [](const Box& outer, const Box& inner) {
+        for (int k = 0; k < 3; k++)
+            if (!(outer.lo[k] <= inner.lo[k] && outer.hi[k] >= inner.hi[k])) return false;
+        return true;
+    };
+    bool ok = b.keys == w.keys && b.nodes.size() == 2ull * s.patchCount() - 1;
+    std::vector<const Box*> box(s.patchCount(), nullptr);
+    for (const Node& n : w.nodes)
+        if (n.left == EMPTY) box[n.right] = &n.leftBox;
+    for (size_t i = 0; ok && i < b.nodes.size(); i++)
+    {
+        const Node& n = b.nodes[i];
+        if (n.left == EMPTY)
+        {
+            // one element, not seen before, with its own box
+            const uint32_t e = b.indices[n.right];
+            ok = e < box.size() && b.indices[n.right + 1] == EMPTY && box[e] &&
+                 std::memcmp(box[e], &n.leftBox, sizeof(Box)) == 0;
+            if (ok) box[e] = nullptr;
+            continue;
+        }
+        const Node &l = b.nodes[n.left], &r = b.nodes[n.right];
+        ok = contains(n.leftBox, l.leftBox) && (l.left == EMPTY || contains(n.leftBox, l.rightBox)) &&
+             contains(n.rightBox, r.leftBox) && (r.left == EMPTY || contains(n.rightBox, r.rightBox));
+    }
+    if (!ok) s.walk = HostBVH {};
+}
+
 // Device copy of the store's host state (everything but the hash tables).
 int cgs::upload_store(cgs_scene* sc)
 {
     const uint32_t nb = sc->nbvh();
     std::vector<float4> hp, hn;
     std::vector<uint4> hq;
-    std::vector<uint32_t> hi, pbase, pmat, gtop;
+    std::vector<uint32_t> hi, pbase, pmat, gtop, lkeys;
     std::vector<DevMaterial> hm;
     std::vector<DevObject> ho;
     sc->hbvh.assign(nb, DevBVH {});
+    sc->walkTrees = false;
     sc->tableCap.assign(nb, 0);
     uint32_t patchCursor = 0, tableCursor = 0, dispCursor = 0;
     for (uint32_t k = 0; k < nb; k++)
@@ -337,8 +398,19 @@ int cgs::upload_store(cgs_scene* sc)
         DevBVH& d = sc->hbvh[k];
         d.nodeBase = uint32_t(hn.size() / 4);
         d.indexBase = uint32_t(hi.size());
+        d.qnodeBase = uint32_t(hq.size() / 2);
+        d.walkBase = EMPTY;
         pack_nodes(b, hn);
-        d.compressed = pack_qnodes(b, hq) ? 1u : 0u;
+        if (k < sc->surfaces.size() && !sc->surfaces[k].walk.nodes.empty())
+        {
+            const HostBVH& w = sc->surfaces[k].walk;
+            d.walkBase = uint32_t(hn.size() / 4);
+            pack_nodes(w, hn);
+            d.compressed = pack_qnodes(w, hq) ? 1u : 0u;
+            sc->walkTrees = true;
+        }
+        else
+            d.compressed = pack_qnodes(b, hq) ? 1u : 0u;
         hi.insert(hi.end(), b.indices.begin(), b.indices.end());
         uint32_t n = uint32_t(b.keys.size());
         d.tableBase = tableCursor;
@@ -360,6 +432,14 @@ int cgs::upload_store(cgs_scene* sc)
                 const float* w = &s.points[4ull * s.indices[16ull * p + j]];
                 hp.push_back(make_float4(w[0], w[1], w[2], w[3]));
             }
+        if (sc->walkTrees)
+        {
+            lkeys.resize(size_t(patchCursor) + s.patchCount(), 0);
+            if (!s.walk.nodes.empty())
+                for (size_t i = 0; i < s.bvh.nodes.size(); i++)
+                    if (s.bvh.nodes[i].left == EMPTY)
+                        lkeys[patchCursor + s.bvh.indices[s.bvh.nodes[i].right]] = s.bvh.keys[i];
+        }
         patchCursor += s.patchCount();
     }
     for (const Object& ob : sc->objects)
@@ -393,6 +473,11 @@ int cgs::upload_store(cgs_scene* sc)
     CGS_TRY(sc->dobjects.reserve(ho.size()));
     CGS_TRY(sc->materials.reserve(hm.size()));
     CGS_TRY(sc->counters.reserve(1));
+    if (sc->walkTrees)
+    {
+        CGS_TRY(sc->leafKeys.reserve(lkeys.size()));
+        CGS_TRY(cudaMemcpy(sc->leafKeys.p, lkeys.data(), lkeys.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    }
     CGS_TRY(cudaMemcpy(sc->patches.p, hp.data(), hp.size() * sizeof(float4), cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->nodes.p, hn.data(), hn.size() * sizeof(float4), cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->qnodes.p, hq.data(), hq.size() * sizeof(uint4), cudaMemcpyHostToDevice));
@@ -406,6 +491,7 @@ int cgs::upload_store(cgs_scene* sc)
     CGS_TRY(cudaMemcpy(sc->bvhs.p, sc->hbvh.data(), nb * sizeof(DevBVH), cudaMemcpyHostToDevice));
     int r = upload_lights(sc);
     if (r) return r;
+    for (Surface& s : sc->surfaces) s.walk = HostBVH {};  // only the device needs it
     sc->uploaded = true;
     return CGS_OK;
 }
@@ -595,7 +681,7 @@ cgs::DevScene cgs_scene::dev() const
 {
     DevScene S {};
     S.patches = patches.p; S.nodes = nodes.p; S.qnodes = qnodes.p; S.indices = indices.p; S.tables = tables.p; S.disps = disps.p;
-    S.bvhs = bvhs.p; S.patchBase = patchBase.p; S.objects = dobjects.p; S.materials = materials.p;
+    S.bvhs = bvhs.p; S.patchBase = patchBase.p; S.leafKeys = walkTrees ? leafKeys.p : nullptr; S.objects = dobjects.p; S.materials = materials.p;
     S.patchMaterial = patchMaterial.p; S.lights = dlights.p;
     S.groupTop = groupTop.p; S.groupLights = groupLights.p; S.groupEnv = groupEnv.p;
     S.nobjects = uint32_t(objects.size()); S.nsurfaces = uint32_t(surfaces.size());
@@ -608,7 +694,7 @@ cgs_scene::~cgs_scene()
     cudaSetDevice(device);
     patches.release(); nodes.release(); qnodes.release();
     for (auto* b : {&indices, &tables, &disps, &patchBase, &patchMaterial, &keys, &groupTop, &scratch32, &groupStage,
-                    &hashJobs,
+                    &hashJobs, &leafKeys,
                     &engine, &fbStage})
         b->release();
     rayStage.release(); hitF.release(); linStage.release(); groupEnv.release();
@@ -777,7 +863,13 @@ int cgs_bvh_build(cgs_scene* s)
     // cores, largest first, each by one thread (the same result as in order)
     const size_t ns = s->surfaces.size(), ng = s->groups.size();
     std::vector<std::pair<uint64_t, size_t>> work;
-    for (size_t i = 0; i < ns; i++) work.push_back({s->surfaces[i].patchCount(), i});
+    const bool walk = s->splitMode == CGS_SPLIT_REFERENCE;
+    for (size_t i = 0; i < ns; i++)
+    {
+        work.push_back({s->surfaces[i].patchCount(), i});
+        if (walk) work.push_back({s->surfaces[i].patchCount(), ns + ng + i});
+        s->surfaces[i].walk = HostBVH {};
+    }
     for (size_t g = 0; g < ng; g++)
     {
         uint64_t cost = 0;
@@ -797,6 +889,8 @@ int cgs_bvh_build(cgs_scene* s)
                 s->surfaces[i].bvh.split_mode = mode;
                 build_surface_bvh(s->surfaces[i], s->surfaces[i].bvh);
             }
+            else if (i >= ns + ng)
+                build_walk_bvh(s->surfaces[i - ns - ng], s->surfaces[i - ns - ng].walk);
             else
             {
                 s->groups[i - ns].top.split_mode = mode;
@@ -846,7 +940,7 @@ int cgs_scene_footprint(const cgs_scene* s, uint64_t* bytes)
     b += s->patches.bytes() + s->nodes.bytes() + s->qnodes.bytes() + s->indices.bytes() + s->tables.bytes() + s->disps.bytes();
     b += s->patchBase.bytes() + s->patchMaterial.bytes() + s->bvhs.bytes() + s->dobjects.bytes();
     b += s->materials.bytes() + s->dlights.bytes() + s->groupTop.bytes() + s->groupLights.bytes();
-    b += s->groupEnv.bytes();
+    b += s->groupEnv.bytes() + s->leafKeys.bytes();
     *bytes = b;
     return CGS_OK;
 }

@@ -52,6 +52,7 @@ struct Surface
     std::vector<float> points;   // 4 per point
     std::vector<uint32_t> indices;
     HostBVH bvh;
+    HostBVH walk;  // the query engine's tree over the same leaves; no nodes where there is none
     uint32_t patchCount() const { return uint32_t(indices.size() / 16); }
 };
 
@@ -187,7 +188,8 @@ struct cgs_scene
     // device side
     cgs::DBuf<float4> patches, nodes;
     cgs::DBuf<uint4> qnodes;  // the compressed mirror of nodes (32 bytes per node)
-    cgs::DBuf<uint32_t> indices, tables, disps, patchBase, patchMaterial, keys, groupTop;
+    cgs::DBuf<uint32_t> indices, tables, disps, patchBase, patchMaterial, keys, groupTop, leafKeys;
+    bool walkTrees = false;  // some surface has a walk tree (and leafKeys its leaves' keys)
     cgs::DBuf<uint2> groupLights;
     cgs::DBuf<float> groupEnv;
     cgs::DBuf<cgs::DevBVH> bvhs;
@@ -242,6 +244,11 @@ namespace cgs {
 
 void camera_setup(const cgs_camera& c, uint32_t w, uint32_t h, int flip, CameraSetup& s);
 int upload_store(cgs_scene* sc);
+// The walk tree of a surface (Surface::walk), for stores of the reference split.
+void build_walk_bvh(const Surface& s, HostBVH& out);
+// Drops s.walk unless the leaves and keys of s.bvh, read from a blob, are those of the walk tree and its
+// boxes nest.
+void check_walk_bvh(Surface& s);
 uint32_t table_capacity(uint32_t n);
 uint32_t displ_size(uint32_t n);
 void hash_coefficients(uint32_t n, uint32_t A[16], uint32_t B[16]);
