@@ -746,7 +746,7 @@ int cgs_perfect_hash_build(const uint32_t* keys, uint32_t n, uint32_t* disp, uin
     cudaStream_t st = (cudaStream_t)stream;
     if (n <= kHashGlobalBlockMaxKeys)
     {
-        // one CTA builds the table, its scratch in shared memory up to
+        // one CTA or cluster builds the table, its buckets in shared memory up to
         // kHashBlockMaxKeys keys, else in global memory (hash_build_blocks)
         HashJob J {};
         J.n = n; J.tableCap = tcap; J.mask = displ_size(n) - 1;

@@ -13,13 +13,16 @@
 // placed, the others add rank+1 to their displacement -- which makes the table
 // a pure function of the keys.  Each round is two kernel launches (bid,
 // commit); there is no device-wide barrier and no spin-wait.
-#include <atomic>
-#include <type_traits>
 #include <algorithm>
+#include <atomic>
+
+#include <cooperative_groups.h>
 
 #include "kernels.h"
 
 namespace cgs {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -31,7 +34,7 @@ constexpr int kRankChunk = 4096;  // buckets per rank block (counts fit 16 bits)
 enum : uint32_t { kActive = 1u, kFeasible = 2u };
 enum : uint32_t { kErrOverflow = 1u, kErrDuplicate = 2u };
 
-// misc layout
+// misc layout; M_FAIL: buckets of each class that the trial did not place
 enum { M_ERR = 0, M_CLASS = 1, M_REMAIN = 5, M_FAIL = 9 };
 
 __global__ void k_bucket(const uint32_t* __restrict__ keys, uint32_t n, uint32_t mask, uint32_t* bsize,
@@ -136,13 +139,24 @@ __global__ void k_trial_init(const uint32_t* bsize, uint32_t nb, uint32_t* dcur,
         disp[b] = 0;
         state[b] = (bsize[b] >= 1 && bsize[b] <= kCap) ? kActive : 0u;
     }
-    if (blockIdx.x == 0 && threadIdx.x < 4) misc[M_REMAIN + threadIdx.x] = misc[M_CLASS + threadIdx.x];
-    if (blockIdx.x == 0 && threadIdx.x == 0) misc[M_FAIL] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < 4)
+    {
+        misc[M_REMAIN + threadIdx.x] = misc[M_CLASS + threadIdx.x];
+        misc[M_FAIL + threadIdx.x] = 0;
+    }
 }
 
 __device__ __forceinline__ unsigned long long owner_tag(uint32_t round, uint32_t rank)
 {
     return ((unsigned long long)(0xFFFFFFFFu - round) << 32) | rank;
+}
+
+// Nothing left to place in class cls: all of it is, or a class before it was not and the trial has failed.
+__device__ __forceinline__ bool class_over(const uint32_t* misc, uint32_t cls)
+{
+    bool over = misc[M_REMAIN + cls - 1] == 0;
+    for (uint32_t c = cls; c < kCap; c++) over = over || misc[M_FAIL + c] != 0;
+    return over;
 }
 
 __global__ void __launch_bounds__(kThreads) k_bid(const uint32_t* bsize, const uint32_t* bkeys, const uint32_t* rank,
@@ -151,7 +165,7 @@ __global__ void __launch_bounds__(kThreads) k_bid(const uint32_t* bsize, const u
                                                   uint32_t cls, uint32_t A, uint32_t B, uint32_t N, uint32_t round,
                                                   const uint32_t* misc)
 {
-    if (misc[M_REMAIN + cls - 1] == 0) return;
+    if (class_over(misc, cls)) return;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
     {
         if (bsize[b] != cls) continue;
@@ -181,7 +195,7 @@ __global__ void __launch_bounds__(kThreads) k_commit(const uint32_t* bsize, cons
                                                      const unsigned long long* owner, uint32_t* disp, uint32_t nb,
                                                      uint32_t cls, uint32_t round, bool last, uint32_t* misc)
 {
-    if (misc[M_REMAIN + cls - 1] == 0) return;
+    if (class_over(misc, cls)) return;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
     {
         if (bsize[b] != cls) continue;
@@ -207,7 +221,7 @@ __global__ void __launch_bounds__(kThreads) k_commit(const uint32_t* bsize, cons
         else
         {
             dcur[b] += rank[b] + 1;
-            if (last) atomicAdd(misc + M_FAIL, 1u);
+            if (last) atomicAdd(misc + M_FAIL + cls - 1, 1u);
         }
     }
 }
@@ -247,34 +261,29 @@ int device_sms()
     return sms;
 }
 
-// ------------------------------------------------------- one CTA per BVH --
-// The same build for one BVH run entirely by one CTA: the bid and commit
-// phases of a round are separated by __syncthreads instead of kernel
-// launches, and a whole store's BVHs are built by one launch, one CTA each,
-// with no host round trip between trials.  Up to kHashBlockMaxKeys keys the
-// buckets, ranks, displacements, slot owners and occupancy bitmap live in
-// shared memory (kShared); up to kHashGlobalBlockMaxKeys in a global scratch
-// area per BVH (mostly L2-resident).  The rounds, ranks, tie rule (lowest
-// rank wins a slot) and displacement steps are those of k_bid / k_commit,
-// so the tables are the same.  Slot owners are tags with the round in the
-// high half and the rank in the low half: 16 + 16 bits in shared memory
-// (rounds < 2^11, ranks < 2^16 there), 32 + 32 bits in global memory.
-struct BlockScratchLayout
-{
-    uint32_t* bkeys;  // [4 nb]
-    uint32_t* dcur;   // [nb]
-    uint32_t* bsize;  // [nb]
-    uint32_t* rank;   // [nb]
-    uint32_t* state;  // [nb]: bit 0 active, bit 1 feasible
-    uint32_t* occ;    // [ceil(nmax / 32)]
-    void* owner;      // [nmax] tags
-};
-
-// Words of a global scratch area for a BVH of n keys (owner tags 64-bit).
-__host__ __device__ inline uint64_t block_scratch_words(uint32_t nb, uint32_t nmax)
-{
-    return 8ull * nb + (nmax + 31) / 32 + 1 + 2ull * nmax;  // +1: 8-byte alignment of the tags
-}
+// ------------------------------------------ one CTA or cluster per BVH --
+// The same build for one BVH run entirely on the device by one CTA (kShared:
+// up to kHashBlockMaxKeys keys) or one cluster of kHashCluster CTAs (up to
+// kHashGlobalBlockMaxKeys): the bid and commit phases of a round are separated
+// by a CTA or cluster barrier instead of kernel launches, and a whole store's
+// BVHs are built by one launch of each kind, with no host round trip between
+// trials.  The rounds, ranks, tie rule (lowest rank wins a slot) and
+// displacement steps are those of k_bid / k_commit, so the tables are the same.
+//
+// What bounds it is the chain of a round: two barriers, a slot read, a bid
+// and its read-back, up to 128 rounds per trial.  So a thread keeps its buckets
+// (at most kItems of the class in hand, in rank order) in registers and a
+// round touches only the slots' owner tags, which are in the CTA's shared
+// memory or spread over the cluster's, slot s in CTA s % kHashCluster; a slot's
+// tag is (round, rank) in 16 + 16 bits (rounds < 2^11, ranks < 2^16), lower
+// for later rounds, and 0 once a bucket is placed there.  A trial ends at the
+// first class that does not place all of its buckets: it has failed then.
+// 39,199 keys (15 trials): 1.60 ms; 15.8 ms as one CTA that swept all buckets
+// of a global scratch area in every round and ran failed trials to their end.
+// The 25 BVHs of a 30,000-patch store, largest 4,800 keys: 0.257 ms, before 0.707 ms.
+// The cluster's rounds are bound by their scattered reads of other CTAs' memory
+// (about 3.3 us a round at 39,199 keys).
+constexpr int kHashCluster = 8;
 
 __device__ __forceinline__ uint4 warp_incl_scan4(uint4 v)
 {
@@ -290,63 +299,69 @@ __device__ __forceinline__ uint4 warp_incl_scan4(uint4 v)
     return v;
 }
 
+// Words of the bucket arrays: bkeys [4 nb], bsize, ord, dcur [nb] each.
+__host__ __device__ inline uint64_t bucket_words(uint32_t nb) { return 7ull * nb; }
+
 template<bool kShared>
 __global__ void __launch_bounds__(kBlockThreads) k_hash_block(const uint32_t* __restrict__ keys,
                                                               const HashJob* __restrict__ jobs, uint32_t* disps,
-                                                              uint32_t* tables, uint32_t* out, uint32_t nbMax,
-                                                              uint32_t nmaxMax, uint32_t* gscratch)
+                                                              uint32_t* tables, uint32_t* out, uint32_t* gscratch)
 {
-    using Tag = typename std::conditional<kShared, uint32_t, unsigned long long>::type;
+    constexpr uint32_t C = kShared ? 1u : uint32_t(kHashCluster);
+    constexpr int kItems = kShared ? 2 : 4;  // nb <= kItems * C * bd below
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t sErr, sFail, sCount[4], sRemain[4];
+    __shared__ uint32_t sErr, sCount[4], sPlaced[64];  // sPlaced: the first CTA's is the cluster's
     __shared__ uint4 sWarp[kBlockThreads / 32];
-    const HashJob& J = jobs[blockIdx.x];
+    const cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t crank = kShared ? 0u : cluster.block_rank();
+    const uint32_t job = kShared ? blockIdx.x : blockIdx.x / C;
+    const HashJob& J = jobs[job];
     const uint32_t n = J.n, mask = J.mask, nb = mask + 1;
     const uint32_t step = max(4u, uint32_t(0.05f * float(n)));
-    BlockScratchLayout L;
-    {
-        const uint32_t nbs = kShared ? nbMax : nb;
-        const uint32_t nms = kShared ? nmaxMax : n + 16u * step;
-        uint32_t* p = kShared ? sm : gscratch + J.scratchOff;
-        L.bkeys = p; p += 4ull * nbs;
-        L.dcur = p; p += nbs;
-        L.bsize = p; p += nbs;
-        L.rank = p; p += nbs;
-        L.state = p; p += nbs;
-        L.occ = p; p += (nms + 31) / 32;
-        if (!kShared && (reinterpret_cast<uintptr_t>(p) & 7u)) p++;
-        L.owner = p;
-    }
-    uint32_t *bkeys = L.bkeys, *dcur = L.dcur, *bsize = L.bsize, *rank = L.rank, *state = L.state, *occ = L.occ;
-    Tag* owner = static_cast<Tag*>(L.owner);
-    const uint32_t tid = threadIdx.x, bd = blockDim.x;
-    uint32_t* res = out + 8ull * blockIdx.x;
+    const uint32_t tid = threadIdx.x;
+    // a small BVH keeps only the warps that hold its buckets: barriers cost by the warp
+    const uint32_t bd = kShared ? min(blockDim.x, max(64u, nb / 2)) : blockDim.x;
+    if (tid >= bd) return;
+    auto sync = [&]() { if constexpr (kShared) __syncthreads(); else cluster.sync(); };
+    auto first = [&](uint32_t* p) { return kShared ? p : cluster.map_shared_rank(p, 0u); };
+    uint32_t* bk = kShared ? sm : gscratch + J.scratchOff;
+    uint32_t *bkeys = bk, *bsize = bk + 4ull * nb, *ord = bsize + nb, *dcur = ord + nb;
+    uint32_t* mine = kShared ? sm + bucket_words(nb) : sm;  // this CTA's owner tags
+    auto owner = [&](uint32_t s) -> volatile uint32_t* {
+        return kShared ? mine + s : cluster.map_shared_rank(mine, s % C) + s / C;
+    };
+    uint32_t* res = out + 8ull * job;
+    const uint32_t g = crank * bd + tid, G = C * bd;  // this thread among the BVH's
 
-    for (uint32_t b = tid; b < nb; b += bd) bsize[b] = 0;
-    if (tid == 0) { sErr = 0; sFail = 0; }
-    __syncthreads();
-    for (uint32_t i = tid; i < n; i += bd)
+    for (uint32_t b = g; b < nb; b += G) { bsize[b] = 0; dcur[b] = 0; }
+    for (uint32_t k = tid; k < 64; k += bd) sPlaced[k] = 0;
+    if (tid == 0) sErr = 0;
+    sync();
+    for (uint32_t i = g; i < n; i += G)
     {
         const uint32_t key = keys[J.keyOff + i], j = key & mask;
         const uint32_t s = atomicAdd(bsize + j, 1u);
-        if (s >= kCap) atomicOr(&sErr, kErrOverflow);  // reference: __trap()
+        if (s >= kCap) atomicOr(first(&sErr), kErrOverflow);  // reference: __trap()
         else bkeys[kCap * j + s] = key;
     }
-    __syncthreads();
-    if (sErr)
+    sync();
+    if (*(volatile uint32_t*)first(&sErr))
     {
         // as hash_build_device reports a bucket overflow (found in trial 0)
-        if (tid == 0) { res[0] = 4; res[1] = J.A[0]; res[2] = J.B[0]; res[3] = n; res[4] = mask; res[5] = 0; }
+        if (g == 0) { res[0] = 4; res[1] = J.A[0]; res[2] = J.B[0]; res[3] = n; res[4] = mask; res[5] = 0; }
+        sync();  // the first CTA's memory is read until here
         return;
     }
 
-    // rank[b]: buckets b' < b of the same size; contiguous buckets per thread,
-    // the four classes' counts scanned block-wide
-    const uint32_t per = (nb + bd - 1) / bd, b0 = tid * per;
+    // ord: the buckets of size 4, then 3, 2, 1, each class in ascending bucket
+    // order: a bucket's place in its class is its rank.  Contiguous buckets per
+    // thread, the four classes' counts scanned over the CTA and the cluster.
+    const uint32_t chunk = (nb + C - 1) / C, per = (chunk + bd - 1) / bd;
+    const uint32_t b0 = crank * chunk + tid * per, b1 = min(min(b0 + per, (crank + 1) * chunk), nb);
     uint4 local = make_uint4(0, 0, 0, 0);
-    for (uint32_t k = 0; k < per && b0 + k < nb; k++)
+    for (uint32_t b = b0; b < b1; b++)
     {
-        const uint32_t sz = bsize[b0 + k];
+        const uint32_t sz = kShared ? bsize[b] : __ldcg(bsize + b);
         local.x += sz == 1; local.y += sz == 2; local.z += sz == 3; local.w += sz == 4;
     }
     const uint4 incl = warp_incl_scan4(local);
@@ -360,113 +375,150 @@ __global__ void __launch_bounds__(kBlockThreads) k_hash_block(const uint32_t* __
         if (tid < nw) sWarp[tid] = make_uint4(wi.x - w.x, wi.y - w.y, wi.z - w.z, wi.w - w.w);
         if (tid == 31) { sCount[0] = wi.x; sCount[1] = wi.y; sCount[2] = wi.z; sCount[3] = wi.w; }
     }
-    __syncthreads();
+    sync();
+    uint32_t count[4] = {0, 0, 0, 0}, before[4] = {0, 0, 0, 0};  // of all CTAs, of the CTAs before this one
+    for (uint32_t c = 0; c < C; c++)
+    {
+        const uint32_t* sc = kShared ? sCount : cluster.map_shared_rank(sCount, c);
+        for (int k = 0; k < 4; k++)
+        {
+            const uint32_t v = sc[k];
+            count[k] += v;
+            before[k] += c + 1u <= crank ? v : 0u;
+        }
+    }
     {
         const uint4 wb = sWarp[tid >> 5];
-        uint32_t run[4] = {wb.x + incl.x - local.x, wb.y + incl.y - local.y, wb.z + incl.z - local.z,
-                           wb.w + incl.w - local.w};
-        for (uint32_t k = 0; k < per && b0 + k < nb; k++)
+        uint32_t run[4] = {before[0] + wb.x + incl.x - local.x + count[3] + count[2] + count[1],
+                           before[1] + wb.y + incl.y - local.y + count[3] + count[2],
+                           before[2] + wb.z + incl.z - local.z + count[3], before[3] + wb.w + incl.w - local.w};
+        for (uint32_t b = b0; b < b1; b++)
         {
-            const uint32_t b = b0 + k, sz = bsize[b];
-            rank[b] = (sz >= 1 && sz <= kCap) ? run[sz - 1]++ : 0u;
+            const uint32_t sz = kShared ? bsize[b] : __ldcg(bsize + b);
+            if (sz >= 1 && sz <= kCap) ord[run[sz - 1]++] = b;
         }
     }
 
     uint32_t N = n, trial = 0, A = 0, B = 0;
+    unsigned long long M = 0;
     bool ok = false;
-    for (trial = 0; trial < 16; trial++)
+    for (trial = 0; trial < 16 && !ok; trial++)
     {
         A = J.A[trial];
         B = J.B[trial];
-        for (uint32_t w = tid; w < (N + 31) / 32; w += bd) occ[w] = 0;
-        for (uint32_t w = tid; w < N; w += bd) owner[w] = Tag(~Tag(0));
-        for (uint32_t b = tid; b < nb; b += bd)
+        M = fastmod_magic(N);
+        for (uint32_t w = tid; w * C + crank < N; w += bd) mine[w] = EMPTY;
+        sync();
+        ok = true;
+        uint32_t base = 0;  // the class's first place in ord
+        for (uint32_t cls = kCap; cls >= 1 && ok; base += count[cls - 1], cls--)
         {
-            dcur[b] = 0;
-            state[b] = (bsize[b] >= 1 && bsize[b] <= kCap) ? kActive : 0u;
-        }
-        if (tid == 0)
-        {
-            sFail = 0;
-            for (int c = 0; c < 4; c++) sRemain[c] = sCount[c];
-        }
-        __syncthreads();
-        for (uint32_t cls = kCap; cls >= 1; cls--)
-        {
-            if (sCount[cls - 1] == 0) continue;
-            for (uint32_t r = 0; r < 32; r++)
+            const uint32_t cnt = count[cls - 1];
+            if (cnt == 0) continue;
+            uint32_t bucket[kItems], key[kItems][kCap], dc[kItems];
+            bool active[kItems];
+#pragma unroll
+            for (int i = 0; i < kItems; i++)
             {
-                const uint32_t round = trial * 128u + (kCap - cls) * 32u + r;
-                const Tag tagHi = kShared ? Tag(0xFFFFu - round) << 16 : Tag(0xFFFFFFFFu - round) << 32;
-                for (uint32_t b = tid; b < nb; b += bd)
+                const uint32_t r = g + uint32_t(i) * G;
+                active[i] = r < cnt;
+                dc[i] = 0;
+                bucket[i] = active[i] ? (kShared ? ord[base + r] : __ldcg(ord + base + r)) : 0u;
+#pragma unroll
+                for (int k = 0; k < int(kCap); k++)
                 {
-                    if (bsize[b] != cls || !(state[b] & kActive)) continue;
-                    uint32_t sl[kCap];
-                    bool f = true;
-                    for (uint32_t k = 0; k < cls; k++)
-                    {
-                        sl[k] = (A * bkeys[kCap * b + k] + B + dcur[b]) % N;
-                        if (occ[sl[k] >> 5] & (1u << (sl[k] & 31))) f = false;
-                        for (uint32_t m = 0; m < k; m++) if (sl[m] == sl[k]) f = false;
-                    }
-                    state[b] = f ? (kActive | kFeasible) : kActive;
-                    if (f)
-                        for (uint32_t k = 0; k < cls; k++) atomicMin(owner + sl[k], tagHi | Tag(rank[b]));
+                    const uint32_t* p = bkeys + kCap * bucket[i] + k;
+                    key[i][k] = active[i] && k < int(cls) ? A * (kShared ? *p : __ldcg(p)) + B : 0u;
                 }
-                __syncthreads();
-                for (uint32_t b = tid; b < nb; b += bd)
+            }
+            uint32_t* placed = first(sPlaced + 4 * trial + cls - 1);
+            bool all = false;
+            for (uint32_t r = 0; r < 32 && !all; r++)
+            {
+                const uint32_t tagHi = (0xFFFFu - (trial * 128u + (kCap - cls) * 32u + r)) << 16;
+                // a cluster learns that the last round placed everything while it bids again (nobody does then)
+                const uint32_t done = kShared ? 0u : *(volatile uint32_t*)placed;
+                uint32_t sl[kItems][kCap];
+                bool feasible[kItems];
+#pragma unroll
+                for (int i = 0; i < kItems; i++)
                 {
-                    if (bsize[b] != cls || !(state[b] & kActive)) continue;
-                    bool win = (state[b] & kFeasible) != 0;
-                    uint32_t sl[kCap];
-                    for (uint32_t k = 0; k < cls; k++)
+                    feasible[i] = active[i];
+                    if (!active[i]) continue;
+#pragma unroll
+                    for (int k = 0; k < int(kCap); k++)
                     {
-                        sl[k] = (A * bkeys[kCap * b + k] + B + dcur[b]) % N;
-                        if (win && owner[sl[k]] != (tagHi | Tag(rank[b]))) win = false;
+                        if (k >= int(cls)) break;
+                        sl[i][k] = fastmod(key[i][k] + dc[i], N, M);
+                        if (*owner(sl[i][k]) == 0u) feasible[i] = false;
+#pragma unroll
+                        for (int m = 0; m < k; m++) if (sl[i][m] == sl[i][k]) feasible[i] = false;
                     }
+                    if (feasible[i])
+#pragma unroll
+                        for (int k = 0; k < int(kCap); k++)
+                            if (k < int(cls)) atomicMin((uint32_t*)owner(sl[i][k]), tagHi | (g + uint32_t(i) * G));
+                }
+                sync();
+                if (!kShared && done == cnt) { all = true; break; }
+                uint32_t wins = 0;
+                bool left = false;
+#pragma unroll
+                for (int i = 0; i < kItems; i++)
+                {
+                    if (!active[i]) continue;
+                    bool win = feasible[i];
+#pragma unroll
+                    for (int k = 0; k < int(kCap); k++)
+                        if (k < int(cls) && win && *owner(sl[i][k]) != (tagHi | (g + uint32_t(i) * G))) win = false;
                     if (win)
                     {
-                        for (uint32_t k = 0; k < cls; k++) atomicOr(occ + (sl[k] >> 5), 1u << (sl[k] & 31));
-                        state[b] = 0;
-                        atomicSub(sRemain + cls - 1, 1u);
+#pragma unroll
+                        for (int k = 0; k < int(kCap); k++) if (k < int(cls)) *owner(sl[i][k]) = 0u;
+                        dcur[bucket[i]] = dc[i];
+                        active[i] = false;
+                        wins++;
                     }
                     else
                     {
-                        dcur[b] += rank[b] + 1;
-                        if (r == 31) atomicAdd(&sFail, 1u);
+                        dc[i] += g + uint32_t(i) * G + 1;
+                        left = true;
                     }
                 }
-                __syncthreads();
-                if (sRemain[cls - 1] == 0) break;
+                if constexpr (kShared)
+                    all = __syncthreads_or(left) == 0;
+                else
+                {
+                    wins = __reduce_add_sync(0xFFFFFFFFu, wins);
+                    if (wins && (tid & 31) == 0) atomicAdd(placed, wins);
+                    sync();
+                }
             }
+            ok = kShared ? all : all || *(volatile uint32_t*)placed == cnt;
         }
-        __syncthreads();
-        if (sFail == 0) { ok = true; break; }
+        if (ok) break;
         N += step;
-        __syncthreads();
+        sync();  // the slots' tags are reset next
     }
     if (!ok)
     {
         // as hash_build_device reports a failed build: the last trial's
         // coefficients and the table size grown past it
-        if (tid == 0)
-        {
-            res[0] = 3; res[1] = J.A[15]; res[2] = J.B[15]; res[3] = N; res[4] = mask; res[5] = 16;
-        }
+        if (g == 0) { res[0] = 3; res[1] = J.A[15]; res[2] = J.B[15]; res[3] = N; res[4] = mask; res[5] = 16; }
         return;
     }
     uint32_t* table = tables + J.tableOff;
-    for (uint32_t b = tid; b < nb; b += bd) disps[J.dispOff + b] = dcur[b];
-    for (uint32_t w = tid; w < N; w += bd) table[w] = EMPTY;
-    __syncthreads();
-    for (uint32_t i = tid; i < n; i += bd)
+    for (uint32_t w = g; w < N; w += G) table[w] = EMPTY;
+    sync();
+    for (uint32_t b = g; b < nb; b += G) disps[J.dispOff + b] = kShared ? dcur[b] : __ldcg(dcur + b);
+    for (uint32_t i = g; i < n; i += G)
     {
         const uint32_t key = keys[J.keyOff + i];
-        const uint32_t h = (A * key + B + dcur[key & mask]) % N;
-        if (atomicCAS(table + h, EMPTY, i) != EMPTY) atomicOr(&sErr, kErrDuplicate);
+        const uint32_t d = kShared ? dcur[key & mask] : __ldcg(dcur + (key & mask));
+        if (atomicCAS(table + fastmod(A * key + B + d, N, M), EMPTY, i) != EMPTY) atomicOr(first(&sErr), kErrDuplicate);
     }
-    __syncthreads();
-    if (tid == 0)
+    sync();
+    if (g == 0)
     {
         res[0] = sErr ? 5u : 0u; res[1] = A; res[2] = B; res[3] = N; res[4] = mask; res[5] = trial;
     }
@@ -560,7 +612,7 @@ int hash_build_device(const uint32_t* keys, uint32_t n, const uint32_t A[16], co
         if (cudaMemcpyAsync(host, sc.misc, sizeof host, cudaMemcpyDeviceToHost, stream) != cudaSuccess) return -1;
         if (cudaStreamSynchronize(stream) != cudaSuccess) return -1;
         if (host[M_ERR] & kErrOverflow) { result = 4; break; }
-        if (host[M_FAIL] == 0) { result = 0; break; }
+        if ((host[M_FAIL] | host[M_FAIL + 1] | host[M_FAIL + 2] | host[M_FAIL + 3]) == 0) { result = 0; break; }
         N = N + step;
     }
     if (launches) *launches += nl;
@@ -591,18 +643,11 @@ void block_sizes(uint32_t n, uint32_t& nb, uint32_t& nmax)
 
 }  // namespace
 
-size_t hash_block_smem(uint32_t maxKeys)
-{
-    uint32_t nb = 0, nmax = 0;
-    block_sizes(maxKeys, nb, nmax);
-    return sizeof(uint32_t) * (8ull * nb + nmax + (nmax + 31) / 32);
-}
-
 uint64_t hash_block_scratch_words(uint32_t n)
 {
     uint32_t nb = 0, nmax = 0;
     block_sizes(n, nb, nmax);
-    return block_scratch_words(nb, nmax);
+    return bucket_words(nb);
 }
 
 cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_t njobs, uint32_t maxKeys,
@@ -611,18 +656,26 @@ cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_
 {
     if (njobs == 0) return cudaSuccess;
     if (maxKeys > kHashGlobalBlockMaxKeys || (maxKeys > kHashBlockMaxKeys && !gscratch)) return cudaErrorInvalidValue;
-    if (maxKeys > kHashBlockMaxKeys)
-    {
-        k_hash_block<false><<<njobs, kBlockThreads, 0, stream>>>(keys, jobs, disps, tables, out, 0, 0, gscratch);
-        return cudaGetLastError();
-    }
     uint32_t nb = 0, nmax = 0;
     block_sizes(maxKeys, nb, nmax);
-    const size_t smem = hash_block_smem(maxKeys);
-    cudaError_t e = cudaFuncSetAttribute(k_hash_block<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const bool shared = maxKeys <= kHashBlockMaxKeys;
+    const size_t smem = sizeof(uint32_t) *
+                        (shared ? size_t(bucket_words(nb)) + nmax : size_t(nmax + kHashCluster - 1) / kHashCluster);
+    auto* k = shared ? k_hash_block<true> : k_hash_block<false>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
-    k_hash_block<true><<<njobs, kBlockThreads, smem, stream>>>(keys, jobs, disps, tables, out, nb, nmax, nullptr);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg {};
+    cfg.gridDim = dim3(shared ? njobs : njobs * kHashCluster);
+    cfg.blockDim = dim3(kBlockThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = shared ? 1 : kHashCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, keys, jobs, disps, tables, out, gscratch);
 }
 
 }  // namespace cgs

@@ -197,14 +197,12 @@ struct HashJob
     uint32_t keyOff, n, dispOff, tableOff, tableCap, mask, scratchOff, pad;
     uint32_t A[16], B[16];
 };
-constexpr uint32_t kHashBlockMaxKeys = 8192;          // one CTA, scratch in shared memory
-constexpr uint32_t kHashGlobalBlockMaxKeys = 131072;  // one CTA, scratch in global memory
-// Dynamic shared memory of the CTA that builds a BVH of maxKeys keys.
-size_t hash_block_smem(uint32_t maxKeys);
-// Global scratch words of the CTA that builds a BVH of n keys (above kHashBlockMaxKeys).
+constexpr uint32_t kHashBlockMaxKeys = 8192;          // one CTA, everything in its shared memory
+constexpr uint32_t kHashGlobalBlockMaxKeys = 131072;  // a cluster of CTAs, buckets in global memory
+// Global scratch words of a BVH of n keys (above kHashBlockMaxKeys).
 uint64_t hash_block_scratch_words(uint32_t n);
-// Builds every job's table, one CTA each, in one launch (asynchronous):
-// all jobs at most kHashBlockMaxKeys keys (shared-memory scratch), or all in
+// Builds every job's table, one CTA or cluster each, in one launch (asynchronous):
+// all jobs at most kHashBlockMaxKeys keys, or all in
 // (kHashBlockMaxKeys, kHashGlobalBlockMaxKeys] with gscratch.  out[8 j ..]:
 // status (0 ok, 3 no trial found a table, 4 bucket overflow, 5 duplicate
 // slot), A, B, N, mask, trial -- the values hash_build_device returns.

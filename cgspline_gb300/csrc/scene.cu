@@ -502,9 +502,9 @@ int upload(cgs_scene* sc) { return upload_store(sc); }
 
 // BVH::buildHashTable (src/rt/BVH.cpp:24-39) for every BVH of the store.
 // BVHs of at most kHashBlockMaxKeys keys (most: one per surface) are built
-// together, one CTA each with its scratch in shared memory, in one launch;
-// those of at most kHashGlobalBlockMaxKeys likewise with a global scratch
-// area each, in a second launch; one host round trip reads both launches'
+// together, one CTA each, in one launch; those of at most
+// kHashGlobalBlockMaxKeys by a cluster of CTAs and a global scratch area each,
+// in a second launch; one host round trip reads both launches'
 // results.  Larger BVHs run the multi-launch build one at a time.
 int hash_all(cgs_scene* sc, cudaStream_t stream)
 {

@@ -398,9 +398,9 @@ int cgs_debug_fail_allocation(uint32_t nth);
  * Outputs (device): disp[displ_capacity], table[table_capacity] with
  * table[h(keys[i])] = i; params (host) = A, B, N, mask, trials.
  * displacement size = bit_floor(max(2, (n-1)>>1)); table_capacity must be at
- * least n + 15*max(4, 0.05n).  Up to 131,072 keys one thread block builds the
- * table in one launch (its scratch in shared memory up to 8,192 keys);
- * larger inputs run the multi-launch build (two launches per round).  All
+ * least n + 15*max(4, 0.05n).  Up to 8,192 keys one thread block and up to
+ * 131,072 keys one cluster of them builds the table in one launch; larger
+ * inputs run the multi-launch build (two launches per round).  All
  * give the same tables.  Synchronises `stream`. */
 int cgs_perfect_hash_build(const uint32_t* keys, uint32_t n, uint32_t* disp, uint32_t displ_capacity,
                            uint32_t* table, uint32_t table_capacity, uint32_t params[5], void* stream);
