@@ -596,9 +596,9 @@ __device__ __forceinline__ bool near_grazing(const float4* __restrict__ P, float
 // from the patch so that it need not stay in registers.  Stack overflow and
 // the iteration cap end the search with an error bit instead of __trap().
 //
-// The search is resumable: clip_begin sets up the state, each clip_step runs
-// one iteration of the reference loop and returns false when the search is
-// over, so a persistent kernel can interleave candidates lane by lane.
+// The search is resumable: clip_begin sets up the state, and the parts of a
+// step below take it on, so a persistent kernel can interleave candidates lane
+// by lane.
 struct ClipState
 {
     float2 buf[16];
@@ -606,7 +606,7 @@ struct ClipState
     int cutsideStack, sl, it;
     float tol;
     bool found, b64;  // b64: FP64 projection and fat-line bounds (near-grazing)
-    bool fresh;       // the net is still to be projected (the search's first step)
+    bool fresh;       // the next projection is the search's first
     bool tposed;      // buf holds the transposed net (left so by a cut along v)
     // The resumable subdivision search (subdiv_step) keeps its walk in the
     // same state: the bit trail in cutsideStack, the level in sl, the
@@ -639,7 +639,7 @@ __device__ __forceinline__ void clip_begin(ClipState& c, const HitSink& sink, fl
         ray64[0] = r.o.x; ray64[1] = r.o.y; ray64[2] = r.o.z;
         ray64[3] = r.d.x; ray64[4] = r.d.y; ray64[5] = r.d.z;
     }
-    c.fresh = true;  // the first clip_step projects the net
+    c.fresh = true;
     c.tposed = false;
     c.emin = make_float2(0.0f, 0.0f);
     c.emax = make_float2(1.0f, 1.0f);
@@ -666,92 +666,111 @@ __device__ __forceinline__ void transpose_if(float2* p, bool t)
         }
 }
 
-// One step of the search.  The first step of a search only projects the net
-// (clip_begin leaves that to it), at the same place in the code as the
-// re-projection after a pop, so lanes starting a search and lanes popping a
-// sub-net share those instructions; it is not counted as an iteration.
-// A cut along v leaves the net transposed (c.tposed); the next step
-// transposes it only if its own cut needs the other orientation, so a step
-// moves the net at most once, and the sub-net of a pop is derived in the
-// natural orientation.  A loop iteration costs the union of the paths its
-// lanes take, so the transposes are kept off the paths that differ.
-template<bool kG64 = true>
-__device__ __forceinline__ bool clip_step(ClipState& c, float4* st, HitSink& sink, LocalCounters& lc,
-                                          const volatile double* ray64)
+// The parts of a step.  A search alternates projections (of the net at its
+// start, of the net and a sub-domain's slices after a pop) and tests of the net
+// in hand, which end in a cut or, below the tolerance, in a root and a pop.
+// clip_patch runs them in order for one thread's search; k_clip interleaves
+// those of a warp's searches, a part at a time.
+enum ClipNext : int { kClipOver, kClipProject, kClipCut, kClipRoot };
+
+// The largest float whose square root is below tol: sqrtf(x) < tol as x <= bound.
+__device__ __forceinline__ float below_sqrt(float tol)
 {
-    const bool b64 = kG64 && c.b64;
-    const bool fresh = c.fresh;
-    bool pop = false, tr = false;
-    float a = 0.0f, b = 1.0f;  // the cut, on the (transposed) net's u axis
-    if (!fresh)
+    float x = tol * tol;
+    while (sqrtf(x) >= tol) x = __uint_as_float(__float_as_uint(x) - 1u);
+    while (sqrtf(__uint_as_float(__float_as_uint(x) + 1u)) < tol) x = __uint_as_float(__float_as_uint(x) + 1u);
+    return x;
+}
+
+// The net in hand counts as one iteration: whether it is small enough for a
+// root, is to be cut, or ends the search at its limit.  tol2 is below_sqrt of
+// the search's tolerance.
+template<bool kG64> __device__ __forceinline__ ClipNext clip_test(ClipState& c, float tol2, LocalCounters& lc)
+{
+    if (kG64 && c.b64 && c.it >= kGrazeIterations) return kClipOver;
+    if (c.it++ >= kMaxClipIterations) { lc.errors |= kErrClipIterations; return kClipOver; }
+    lc.iterations++;
+    // the diagonals (the corners p3 and p12 swapped where the net is transposed: the same length)
+    const float2 e = c.buf[3] - c.buf[12], f = c.buf[15] - c.buf[0];
+    return dot2(e, e) <= tol2 && dot2(f, f) <= tol2 ? kClipRoot : kClipCut;
+}
+
+// The interval pushed last, or the search's end.
+__device__ __forceinline__ ClipNext clip_pop(ClipState& c, const float4* st)
+{
+    c.cutsideStack >>= 1;
+    if (--c.sl < 0) return kClipOver;
+    const float4 e = st[c.sl];
+    c.emin = make_float2(e.x, e.y);
+    c.emax = make_float2(e.z, e.w);
+    return kClipProject;
+}
+
+// Projects the patch; after a pop also derives the popped interval's sub-net
+// (in the natural orientation).
+template<bool kG64> __device__ __forceinline__ void clip_project(ClipState& c, const HitSink& sink,
+                                                                 const volatile double* ray64)
+{
+    if (kG64 && c.b64)
+        project_net64(c.buf, sink.P, make_double3(ray64[0], ray64[1], ray64[2]),
+                      make_double3(ray64[3], ray64[4], ray64[5]));
+    else project_net(c.buf, sink.P, sink.o, sink.d);
+    c.tposed = false;
+    if (!c.fresh)
     {
-        if (b64 && c.it >= kGrazeIterations) return false;
-        if (c.it++ >= kMaxClipIterations) { lc.errors |= kErrClipIterations; return false; }
-        lc.iterations++;
-        tr = (c.cutsideStack & 1) != 0;  // this step cuts along v
-        pop = true;
-        // the corners in the natural orientation (a transpose swaps p3 and p12)
-        const float2 p3 = c.tposed ? c.buf[12] : c.buf[3], p12 = c.tposed ? c.buf[3] : c.buf[12];
-        if (len2(p3 - p12) < c.tol && len2(c.buf[15] - c.buf[0]) < c.tol)
-            c.found |= approximateIntersection(sink, c.buf[0], p3, p12, c.buf[15], c.emin, c.emax);
-        else
-        {
-            transpose_if(c.buf, tr != c.tposed);
-            c.tposed = tr;
-            float lower, upper;
-            if (b64) clip_range64(c.buf, 0, lower, upper);
-            else clip_range(c.buf, 0, lower, upper);
-            const float delta = upper - lower;
-            const float lo = tr ? c.emin.y : c.emin.x, hi = tr ? c.emax.y : c.emax.x;
-            if (delta > 0.8f)
-            {
-                // split in halves: keep the upper half, push the lower
-                const float h = 0.5f * (lo + hi);
-                const float4 pushed = tr ? make_float4(c.emin.x, c.emin.y, c.emax.x, h)
-                                         : make_float4(c.emin.x, c.emin.y, h, c.emax.y);
-                if (tr) c.emin.y = h; else c.emin.x = h;
-                c.cutsideStack = tr ? ((c.cutsideStack << 1) & ~3) : ((c.cutsideStack << 1) | 3);
-                if (c.sl >= kClipStack) { lc.errors |= kErrClipStack; return false; }
-                st[c.sl++] = pushed;
-                a = 0.5f; b = 1.0f;
-                pop = false;
-            }
-            else if (delta > 0.0f)
-            {
-                const float sz = hi - lo;
-                const float n0 = lo + sz * lower, n1 = hi - sz * (1.0f - upper);
-                if (tr) { c.emin.y = n0; c.emax.y = n1; } else { c.emin.x = n0; c.emax.x = n1; }
-                c.cutsideStack ^= 1;
-                a = lower; b = upper;
-                pop = false;
-            }
-        }
-        if (pop)
-        {
-            c.cutsideStack >>= 1;
-            if (--c.sl < 0) return false;
-            const float4 e = st[c.sl];
-            c.emin = make_float2(e.x, e.y);
-            c.emax = make_float2(e.z, e.w);
-            a = c.emin.x; b = c.emax.x;
-        }
+        subpatchU(c.buf, c.emin.x, c.emax.x);
+        subpatchV(c.buf, c.emin.y, c.emax.y);
     }
-    if (fresh || pop)
+    c.fresh = false;
+}
+
+// Cuts the net along u or v to its fat line's range, halves it where the range
+// is wide, drops it where it is empty.  kClipCut: the net in hand is new.
+// A cut along v leaves the net transposed (c.tposed); the next cut transposes
+// it only if it needs the other orientation.
+template<bool kG64> __device__ __forceinline__ ClipNext clip_cut(ClipState& c, float4* st, LocalCounters& lc)
+{
+    const bool tr = (c.cutsideStack & 1) != 0;  // this cut is along v
+    transpose_if(c.buf, tr != c.tposed);
+    c.tposed = tr;
+    float lower, upper;
+    if (kG64 && c.b64) clip_range64(c.buf, 0, lower, upper);
+    else clip_range(c.buf, 0, lower, upper);
+    const float delta = upper - lower;
+    const float lo = tr ? c.emin.y : c.emin.x, hi = tr ? c.emax.y : c.emax.x;
+    float a = lower, b = upper;
+    if (delta > 0.8f)
     {
-        if (b64)
-            project_net64(c.buf, sink.P, make_double3(ray64[0], ray64[1], ray64[2]),
-                          make_double3(ray64[3], ray64[4], ray64[5]));
-        else project_net(c.buf, sink.P, sink.o, sink.d);
-        c.tposed = false;
+        // split in halves: keep the upper half, push the lower
+        const float h = 0.5f * (lo + hi);
+        const float4 pushed = tr ? make_float4(c.emin.x, c.emin.y, c.emax.x, h)
+                                 : make_float4(c.emin.x, c.emin.y, h, c.emax.y);
+        if (tr) c.emin.y = h; else c.emin.x = h;
+        c.cutsideStack = tr ? ((c.cutsideStack << 1) & ~3) : ((c.cutsideStack << 1) | 3);
+        if (c.sl >= kClipStack) { lc.errors |= kErrClipStack; return kClipOver; }
+        st[c.sl++] = pushed;
+        a = 0.5f; b = 1.0f;
     }
-    if (fresh)
+    else if (delta > 0.0f)
     {
-        c.fresh = false;
-        return true;
+        const float sz = hi - lo;
+        const float n0 = lo + sz * lower, n1 = hi - sz * (1.0f - upper);
+        if (tr) { c.emin.y = n0; c.emax.y = n1; } else { c.emin.x = n0; c.emax.x = n1; }
+        c.cutsideStack ^= 1;
     }
-    subpatchU(c.buf, a, b);  // every lane: the cut, or the u range of the popped sub-net
-    if (pop) subpatchV(c.buf, c.emin.y, c.emax.y);
-    return true;
+    else
+        return clip_pop(c, st);
+    subpatchU(c.buf, a, b);
+    return kClipCut;
+}
+
+// The net is below the tolerance: its roots, then the next interval.
+__device__ __forceinline__ ClipNext clip_root(ClipState& c, const float4* st, HitSink& sink)
+{
+    // the corners in the natural orientation (a transpose swaps p3 and p12)
+    const float2 p3 = c.tposed ? c.buf[12] : c.buf[3], p12 = c.tposed ? c.buf[3] : c.buf[12];
+    c.found |= approximateIntersection(sink, c.buf[0], p3, p12, c.buf[15], c.emin, c.emax);
+    return clip_pop(c, st);
 }
 
 // anyHit: stop at the first root found.  An any-hit query only asks whether
@@ -765,7 +784,18 @@ static __device__ __noinline__ bool clip_patch(HitSink& sink, float tol, float g
     ClipState c;
     volatile double ray64[6];
     clip_begin(c, sink, tol, grazeSin, ray64, ob, wo, wd);
-    while (clip_step(c, st, sink, lc, ray64) && !(anyHit && c.found)) {}
+    const float tol2 = below_sqrt(c.tol);
+    ClipNext next = kClipProject;
+    while (next != kClipOver && !(anyHit && c.found))
+    {
+        if (next == kClipRoot) next = clip_root(c, st, sink);
+        else
+        {
+            if (next == kClipCut) next = clip_cut<true>(c, st, lc);
+            if (next == kClipProject) { clip_project<true>(c, sink, ray64); next = kClipCut; }
+            if (next == kClipCut) next = clip_test<true>(c, tol2, lc);
+        }
+    }
     return c.found;
 }
 

@@ -14,7 +14,7 @@
 // the ray parks: its key, postponed bits and node are saved and the next
 // pass resumes it.
 //
-// k_resolve replays the reference's leaf callbacks over the chunk in order: a
+// k_clip and k_subdivide replay the reference's leaf callbacks over the chunk in order: a
 // patch whose leaf box starts at or beyond the object's current best t is
 // skipped (the reference's `L0 < hit.t` test), any other runs the
 // Bezier-clipping search with the current best as hit.distance
@@ -48,7 +48,7 @@
 //     reference tree, which parks the ray exactly where it would have parked.
 //
 // Both kernels refill lanes one ray (k_collect) or one clip iteration
-// (k_resolve) at a time, so heavy-tailed per-ray work does not idle the other
+// (the search kernels) at a time, so heavy-tailed per-ray work does not idle the other
 // lanes of a warp, and take rays in id order so a warp's rays stay coherent.
 // Rays still unfinished after the configured number of passes are completed
 // by k_rest, the inline version of the same search.  Block sizes, grid
@@ -547,132 +547,41 @@ __global__ void __launch_bounds__(kOrderThreads) k_order(DevScene S, RaysSoA ray
 }
 
 // ------------------------------------------------------------ resolve --
-// kG64: the search may take the FP64 grazing path (precision levels 3 and 5);
-// the other levels run an instance without that code.  kSub: the searches
-// are the subdivision method's (a separate instance, so that the clipping
-// instances' loop holds no subdivision code; at the grazing levels the kG64
-// instance runs subdivision searches whole instead).  The FP32 clipping
-// instances are held to 128 registers, four 128-thread blocks per SM.
-template<bool kAny, bool kG64, bool kSub = false>
-__global__ void __launch_bounds__(kResolveThreads, (!kG64 && !kSub) ? 4 : 3) k_resolve(DevScene S, RaysSoA rays, uint32_t n0,
-                                                             const uint32_t* nDev, Eng E, int pass, Query q,
-                                                             HitsSoA hits, int32_t* occluded, Counters* cnt)
+// One lane's ray: where it is in its list, and the best hit so far.  Shared by
+// the two search kernels below.
+template<bool kAny> struct ListWalk
 {
-    const uint32_t n = nDev ? *nDev : n0;
-    LocalCounters lc;
-    float4 stack[kClipStack];
-    volatile double ray64[6];  // kG64: a near-grazing search's ray in double
-    ClipState c;
-    HitSink sink {nullptr, f3(0, 0, 0), f3(0, 0, 1), 0.0f, make_float2(0, 0)};
-    bool active = false, exhausted = false, clipping = false;
-    bool thief = false;  // any hit: the lane searches an interval taken from another lane's search
+    uint32_t rid = 0, k = 0, count = 0, patch = 0;
+    int32_t obj = -1, lpatch = -1;
     // any hit with E.originLast: sweep 0 searches the candidates whose leaf box
     // holds the ray's origin (entry <= 0) not, sweep 1 only those
     bool sweep = false;
-    uint32_t rid = 0, k = 0, count = 0, patch = 0;
-    int32_t obj = -1, lpatch = -1;
     float3 o = f3(0, 0, 0), d = f3(0, 0, 1);
     float tmax = 0, lmax = 0, sinv = 1, lt = 0, lu = 0, lv = 0, limit = 0;
     const uint2* list = nullptr;
-    // pass 0 resolves every ray; a later pass the rays its traversal walked
-    const uint32_t m = pass == 0 ? n : E.ctl[4 * pass + 2];
-    const uint32_t* queue = E.queue[pass & 1];
-    for (;;)
-    {
-        const bool need = !active && !exhausted;
-        const uint32_t idx = warp_fetch(E.ctl + 4 * pass + 1, need);
-        if (need)
-        {
-            if (idx >= m)
-                exhausted = true;
-            else
-            {
-                const uint32_t r = pass == 0 ? idx : queue[idx];
-                const uint32_t st = E.status[r];
-                count = E.count[r];
-                if (count > 0 && st != kFinished)
-                {
-                    rid = r;
-                    active = true;
-                    k = 0;
-                    obj = -1;
-                    clipping = false;
-                    sweep = false;
-                    load_ray(rays, rid, o, d, tmax);
-                    limit = kAny ? tmax : (pass == 0 ? tmax : E.limit[rid]);
-                    list = E.list + size_t(rid) * kChunk;
-                }
-            }
-        }
-        if (__ballot_sync(0xFFFFFFFFu, active || !exhausted) == 0) break;
-        if constexpr (kAny && !kSub && !kG64)
-        {
-            // The tail of an any-hit launch is a few long searches.  A lane
-            // left without rays takes the bottom (largest) pending interval of
-            // a search in its warp that holds one or more, and searches it as
-            // that search would after popping it: the same sub-net, derived
-            // from the projected net, and the same cut side.  The searched
-            // intervals are the same, so the roots found are; an any-hit
-            // answer needs one of them, and whichever lane finds it marks
-            // the ray occluded (writes of "occluded" never clear it).
-            const unsigned idleM = __ballot_sync(0xFFFFFFFFu, exhausted && !active);
-            const unsigned richM = __ballot_sync(0xFFFFFFFFu, clipping && !c.fresh && c.sl >= 1 && c.sl <= 30);
-            if (idleM && richM)
-            {
-                const unsigned lane = lane_id(), below = (1u << lane) - 1u;
-                const int pairs = min(__popc(idleM), __popc(richM));
-                const int idleRank = __popc(idleM & below), richRank = __popc(richM & below);
-                const bool isThief = ((idleM >> lane) & 1u) && idleRank < pairs;
-                const bool isVictim = ((richM >> lane) & 1u) && richRank < pairs;
-                const int src = isThief ? int(__fns(richM, 0, idleRank + 1)) : int(lane);
-                float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                int bit = 0;
-                if (isVictim)
-                {
-                    // entry i's cut side is bit (sl - i) of the bit stack; the
-                    // bits above the bottom entry's are clear
-                    e = stack[0];
-                    bit = (c.cutsideStack >> c.sl) & 1;
-                    c.cutsideStack &= ~(1 << c.sl);
-                    for (int i = 1; i < c.sl; i++) stack[i - 1] = stack[i];
-                    c.sl--;
-                }
-                const float4 se = make_float4(__shfl_sync(0xFFFFFFFFu, e.x, src), __shfl_sync(0xFFFFFFFFu, e.y, src),
-                                              __shfl_sync(0xFFFFFFFFu, e.z, src), __shfl_sync(0xFFFFFFFFu, e.w, src));
-                const int sbit = __shfl_sync(0xFFFFFFFFu, bit, src);
-                const uint32_t srid = __shfl_sync(0xFFFFFFFFu, rid, src);
-                const unsigned long long sp =
-                    __shfl_sync(0xFFFFFFFFu, (unsigned long long)reinterpret_cast<uintptr_t>(sink.P), src);
-                const float3 so = f3(__shfl_sync(0xFFFFFFFFu, sink.o.x, src), __shfl_sync(0xFFFFFFFFu, sink.o.y, src),
-                                     __shfl_sync(0xFFFFFFFFu, sink.o.z, src));
-                const float3 sd = f3(__shfl_sync(0xFFFFFFFFu, sink.d.x, src), __shfl_sync(0xFFFFFFFFu, sink.d.y, src),
-                                     __shfl_sync(0xFFFFFFFFu, sink.d.z, src));
-                const float sdist = __shfl_sync(0xFFFFFFFFu, sink.dist, src);
-                const float stol = __shfl_sync(0xFFFFFFFFu, c.tol, src);
-                if (isThief)
-                {
-                    rid = srid;
-                    sink.P = reinterpret_cast<const float4*>(uintptr_t(sp));
-                    sink.o = so; sink.d = sd; sink.dist = sdist; sink.uv = make_float2(0.0f, 0.0f);
-                    c.emin = make_float2(se.x, se.y);
-                    c.emax = make_float2(se.z, se.w);
-                    c.cutsideStack = sbit; c.sl = 0; c.it = 0; c.tol = stol;
-                    c.found = false; c.b64 = false; c.fresh = false; c.tposed = false;
-                    project_net(c.buf, sink.P, sink.o, sink.d);
-                    subpatchU(c.buf, se.x, se.z);
-                    subpatchV(c.buf, se.y, se.w);
-                    active = true; clipping = true; thief = true;
-                }
-            }
-        }
-        if (!active) continue;
 
-        bool finished = false;
-        // A lane without a search in progress walks its list -- object
-        // markers, patches culled by their leaf entry -- until it starts the
-        // next search or its chunk ends, so that the clip steps below run with
-        // as many lanes as possible.
-        while (!clipping && !finished)
+    // Takes ray r; false if it has nothing to search.
+    __device__ __forceinline__ bool take(const RaysSoA& rays, const Eng& E, int pass, uint32_t r)
+    {
+        const uint32_t st = E.status[r];
+        count = E.count[r];
+        if (count == 0 || st == kFinished) return false;
+        rid = r;
+        k = 0;
+        obj = -1;
+        sweep = false;
+        load_ray(rays, rid, o, d, tmax);
+        limit = kAny ? tmax : (pass == 0 ? tmax : E.limit[rid]);
+        list = E.list + size_t(rid) * kChunk;
+        return true;
+    }
+
+    // Walks the list -- object markers, patches culled by their leaf entry --
+    // to the next patch to search (true, with `sink` set up for it) or the end
+    // of the chunk (false).
+    __device__ __forceinline__ bool next(const DevScene& S, const Eng& E, HitsSoA& hits, HitSink& sink)
+    {
+        for (;;)
         {
             if (kAny && k >= count && E.originLast && !sweep)
             {
@@ -689,8 +598,7 @@ __global__ void __launch_bounds__(kResolveThreads, (!kG64 && !kSub) ? 4 : 3) k_r
                     E.limit[rid] = limit;
                     if (obj >= 0) { E.lt[rid] = lt; E.lu[rid] = lu; E.lv[rid] = lv; E.lpatch[rid] = lpatch; }
                 }
-                finished = true;
-                break;
+                return false;
             }
             const uint2 e = list[k++];
             if (e.x == kEnter || e.x == kCont)
@@ -727,56 +635,265 @@ __global__ void __launch_bounds__(kResolveThreads, (!kG64 && !kSub) ? 4 : 3) k_r
                     sink.P = S.patches + 16ull * (__ldg(S.patchBase + surface) + patch);
                     sink.dist = kAny ? lmax : lt;
                     sink.uv = kAny ? make_float2(0.0f, 0.0f) : make_float2(lu, lv);
-                    lc.candidates++;
-                    if (kSub) subdiv_begin(c, sink, q.tol);
-                    else if (!(kG64 && q.method != 0))
-                        clip_begin<kG64>(c, sink, q.tol, graze_sin(q.precision), ray64, &S.objects[obj], o, d);
-                    clipping = true;
+                    return true;
                 }
             }
         }
-        if (clipping)
+    }
+
+    // A closest-hit search of the patch ended with a closer root.
+    __device__ __forceinline__ void keep(const HitSink& sink)
+    {
+        lt = sink.dist; lu = sink.uv.x; lv = sink.uv.y; lpatch = int32_t(patch);
+    }
+};
+
+// The clipping searches.  A lane takes a ray, walks its list and searches its
+// patches; a search is made of the parts of clip_patch's loop.  The lanes of a
+// warp are in different parts most of the time, and a loop that ran every part
+// each time round for the lanes that are in it used 8 of 32 threads per
+// instruction (4.8 in the FP64 instance).  So each time round the warp runs
+// only the part that most of its lanes wait for (the projections and cuts in
+// FP64 count as parts of their own); the others wait until theirs gathers
+// more.  A lane's sequence of parts, and with it every result, does not depend on that.
+// 640,001 shadow rays of the 16,384-patch torus: 1.46 ms, 2.02 ms with all
+// parts each time round; 301,111 scattered rays 1.13 ms, before 1.29 ms.
+//
+// kG64: the search may take the FP64 grazing path (precision levels 3 and 5);
+// the other levels run an instance without that code.  The FP32 instances are
+// held to 128 registers, four 128-thread blocks per SM.
+enum : int { kPartWalk, kPartProject, kPartCut, kPartRoot, kPartProject64, kPartCut64, kPartNone };
+template<bool kAny, bool kG64>
+__global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene S, RaysSoA rays, uint32_t n0,
+                                                                         const uint32_t* nDev, Eng E, int pass, Query q,
+                                                                         HitsSoA hits, int32_t* occluded, Counters* cnt)
+{
+    const uint32_t n = nDev ? *nDev : n0;
+    LocalCounters lc;
+    float4 stack[kClipStack];
+    volatile double ray64[6];  // kG64: a near-grazing search's ray in double
+    ClipState c;
+    c.b64 = false;
+    c.sl = 0;
+    HitSink sink {nullptr, f3(0, 0, 0), f3(0, 0, 1), 0.0f, make_float2(0, 0)};
+    ListWalk<kAny> w;
+    int part = kPartWalk;
+    bool have = false;   // the lane has a ray
+    bool thief = false;  // any hit: the lane searches an interval taken from another lane's search
+    const float tol2 = below_sqrt(q.tol), tol2graze = kG64 ? below_sqrt(kGrazeTol) : 0.0f;
+    // pass 0 resolves every ray; a later pass the rays its traversal walked
+    const uint32_t m = pass == 0 ? n : E.ctl[4 * pass + 2];
+    const uint32_t* queue = E.queue[pass & 1];
+    for (;;)
+    {
+        // the part that most lanes wait for
+        int run = kPartNone;
+        int most = 0;
+#pragma unroll
+        for (int p = kPartWalk; p <= (kG64 ? kPartCut64 : kPartRoot); p++)
         {
-            bool found = false, more = false;
-            if (kG64 && q.method != 0)
+            const int lanes = __popc(__ballot_sync(0xFFFFFFFFu, part == p));
+            if (lanes > most) { most = lanes; run = p; }
+        }
+        if (run == kPartNone) break;
+        if constexpr (kAny && !kG64)
+        {
+            // The tail of an any-hit launch is a few long searches.  A lane
+            // left without rays takes the bottom (largest) pending interval of
+            // a search in its warp that holds one or more, and searches it as
+            // that search would after popping it: the same sub-net, derived
+            // from the projected net, and the same cut side.  The searched
+            // intervals are the same, so the roots found are; an any-hit
+            // answer needs one of them, and whichever lane finds it marks
+            // the ray occluded (writes of "occluded" never clear it).
+            const unsigned idleM = __ballot_sync(0xFFFFFFFFu, part == kPartNone);
+            if (idleM)
             {
-                // the precision form's subdivision searches run whole, one call each
-                found = subdiv_patch(sink, q.tol, lc);
+                const unsigned richM =
+                    __ballot_sync(0xFFFFFFFFu, part != kPartNone && part != kPartWalk && c.sl >= 1 && c.sl <= 30);
+                if (richM)
+                {
+                    const unsigned lane = lane_id(), below = (1u << lane) - 1u;
+                    const int pairs = min(__popc(idleM), __popc(richM));
+                    const int idleRank = __popc(idleM & below), richRank = __popc(richM & below);
+                    const bool isThief = ((idleM >> lane) & 1u) && idleRank < pairs;
+                    const bool isVictim = ((richM >> lane) & 1u) && richRank < pairs;
+                    const int src = isThief ? int(__fns(richM, 0, idleRank + 1)) : int(lane);
+                    float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    int bit = 0;
+                    if (isVictim)
+                    {
+                        // entry i's cut side is bit (sl - i) of the bit stack; the
+                        // bits above the bottom entry's are clear
+                        e = stack[0];
+                        bit = (c.cutsideStack >> c.sl) & 1;
+                        c.cutsideStack &= ~(1 << c.sl);
+                        for (int i = 1; i < c.sl; i++) stack[i - 1] = stack[i];
+                        c.sl--;
+                    }
+                    const float4 se =
+                        make_float4(__shfl_sync(0xFFFFFFFFu, e.x, src), __shfl_sync(0xFFFFFFFFu, e.y, src),
+                                    __shfl_sync(0xFFFFFFFFu, e.z, src), __shfl_sync(0xFFFFFFFFu, e.w, src));
+                    const int sbit = __shfl_sync(0xFFFFFFFFu, bit, src);
+                    const uint32_t srid = __shfl_sync(0xFFFFFFFFu, w.rid, src);
+                    const unsigned long long sp =
+                        __shfl_sync(0xFFFFFFFFu, (unsigned long long)reinterpret_cast<uintptr_t>(sink.P), src);
+                    const float3 so =
+                        f3(__shfl_sync(0xFFFFFFFFu, sink.o.x, src), __shfl_sync(0xFFFFFFFFu, sink.o.y, src),
+                           __shfl_sync(0xFFFFFFFFu, sink.o.z, src));
+                    const float3 sd =
+                        f3(__shfl_sync(0xFFFFFFFFu, sink.d.x, src), __shfl_sync(0xFFFFFFFFu, sink.d.y, src),
+                           __shfl_sync(0xFFFFFFFFu, sink.d.z, src));
+                    const float sdist = __shfl_sync(0xFFFFFFFFu, sink.dist, src);
+                    if (isThief)
+                    {
+                        w.rid = srid;
+                        sink.P = reinterpret_cast<const float4*>(uintptr_t(sp));
+                        sink.o = so; sink.d = sd; sink.dist = sdist; sink.uv = make_float2(0.0f, 0.0f);
+                        c.emin = make_float2(se.x, se.y);
+                        c.emax = make_float2(se.z, se.w);
+                        c.cutsideStack = sbit; c.sl = 0; c.it = 0; c.tol = q.tol;
+                        c.found = false; c.b64 = false; c.fresh = false; c.tposed = false;
+                        part = kPartProject;
+                        thief = true;
+                    }
+                }
             }
-            else if (!kSub)
+        }
+        if (run == kPartWalk)
+        {
+            const bool need = part == kPartWalk && !have;
+            const uint32_t idx = warp_fetch(E.ctl + 4 * pass + 1, need);
+            if (need)
             {
-                more = clip_step<kG64>(c, stack, sink, lc, ray64);
-                found = c.found;
-                if (kAny && found) more = false;  // an any-hit search ends at its first root
+                if (idx < m) have = w.take(rays, E, pass, pass == 0 ? idx : queue[idx]);
+                else part = kPartNone;
+            }
+            if (part == kPartWalk && have)
+            {
+                if (w.next(S, E, hits, sink))
+                {
+                    lc.candidates++;
+                    clip_begin<kG64>(c, sink, q.tol, graze_sin(q.precision), ray64, &S.objects[w.obj], w.o, w.d);
+                    part = kG64 && c.b64 ? kPartProject64 : kPartProject;
+                }
+                else
+                {
+                    have = false;
+                    E.count[w.rid] = 0;
+                }
+            }
+            continue;
+        }
+        if (part != run) continue;
+        ClipNext next;
+        if (run == kPartRoot) next = clip_root(c, stack, sink);
+        else
+        {
+            // c.b64 is uniform over the lanes of a part; naming it lets each part hold one kind of code
+            if (run == kPartProject || (kG64 && run == kPartProject64))
+            {
+                clip_project<kG64>(c, sink, ray64);
+                next = kClipCut;
             }
             else
+                next = clip_cut<kG64>(c, stack, lc);
+            if (next == kClipCut) next = clip_test<kG64>(c, kG64 && c.b64 ? tol2graze : tol2, lc);
+        }
+        if (kAny && c.found) next = kClipOver;  // an any-hit search ends at its first root
+        if (next != kClipOver)
+        {
+            const bool b64 = kG64 && c.b64;
+            part = next == kClipRoot ? kPartRoot
+                   : next == kClipCut ? (b64 ? kPartCut64 : kPartCut) : (b64 ? kPartProject64 : kPartProject);
+            continue;
+        }
+        part = kPartWalk;
+        if (!kAny)
+        {
+            if (c.found) w.keep(sink);
+            continue;
+        }
+        if (c.found)
+        {
+            occluded[w.rid] = 0;
+            E.status[w.rid] = kFinished;
+            E.count[w.rid] = 0;
+            have = false;
+        }
+        if (thief)
+        {
+            thief = false;
+            part = kPartNone;
+        }
+    }
+    flush_counters(cnt, lc, 0);
+}
+
+// The subdivision method's searches (at the precision form's levels too: it
+// has no FP64 bounds): a lane runs E.subdivLevels bisections a time round.
+template<bool kAny>
+__global__ void __launch_bounds__(kResolveThreads, 3) k_subdivide(DevScene S, RaysSoA rays, uint32_t n0,
+                                                                  const uint32_t* nDev, Eng E, int pass, Query q,
+                                                                  HitsSoA hits, int32_t* occluded, Counters* cnt)
+{
+    const uint32_t n = nDev ? *nDev : n0;
+    LocalCounters lc;
+    ClipState c;
+    HitSink sink {nullptr, f3(0, 0, 0), f3(0, 0, 1), 0.0f, make_float2(0, 0)};
+    ListWalk<kAny> w;
+    bool have = false, exhausted = false, searching = false;
+    const uint32_t m = pass == 0 ? n : E.ctl[4 * pass + 2];
+    const uint32_t* queue = E.queue[pass & 1];
+    for (;;)
+    {
+        const bool need = !have && !exhausted;
+        const uint32_t idx = warp_fetch(E.ctl + 4 * pass + 1, need);
+        if (need)
+        {
+            if (idx >= m) exhausted = true;
+            else
             {
-                more = subdiv_step(c, sink, lc, int(E.subdivLevels));
-                found = c.found;
-                if (kAny && found) more = false;
+                have = w.take(rays, E, pass, pass == 0 ? idx : queue[idx]);
+                searching = false;
             }
+        }
+        if (__ballot_sync(0xFFFFFFFFu, have || !exhausted) == 0) break;
+        if (!have) continue;
+        bool finished = false;
+        // A lane without a search in progress walks its list until it starts the
+        // next search or its chunk ends, so that the steps below run with as
+        // many lanes as possible.
+        if (!searching)
+        {
+            searching = w.next(S, E, hits, sink);
+            finished = !searching;
+            if (searching)
+            {
+                lc.candidates++;
+                subdiv_begin(c, sink, q.tol);
+            }
+        }
+        if (searching)
+        {
+            bool more = subdiv_step(c, sink, lc, int(E.subdivLevels));
+            if (kAny && c.found) more = false;  // an any-hit search ends at its first root
             if (!more)
             {
-                clipping = false;
-                if (kAny)
+                searching = false;
+                if (kAny && c.found)
                 {
-                    if (found) { occluded[rid] = 0; E.status[rid] = kFinished; finished = true; }
+                    occluded[w.rid] = 0;
+                    E.status[w.rid] = kFinished;
+                    finished = true;
                 }
-                else if (found)
-                {
-                    lt = sink.dist; lu = sink.uv.x; lv = sink.uv.y; lpatch = int32_t(patch);
-                }
+                if (!kAny && c.found) w.keep(sink);
             }
         }
         if (finished)
         {
-            active = false;
-            E.count[rid] = 0;
-        }
-        if (kAny && thief && !clipping)
-        {
-            thief = false;
-            active = false;
+            have = false;
+            E.count[w.rid] = 0;
         }
     }
     flush_counters(cnt, lc, 0);
@@ -923,13 +1040,19 @@ int resident(const void* fn, int threads)
 
 // Resident blocks per SM of kernel fn at `threads` per block (cached: the
 // values depend only on the kernel and the block size).
+template<bool kAny, bool kG64, bool kSub> auto* search_kernel()
+{
+    if constexpr (kSub) return k_subdivide<kAny>;
+    else return k_clip<kAny, kG64>;
+}
+
 template<bool kAny, bool kG64, bool kSub = false> int per_sm(bool collect, int threads, bool compressed = true)
 {
     static const int v[3][2] = {
         {resident((const void*)k_collect<kAny, false, true>, 128) / sms(),
          resident((const void*)k_collect<kAny, false, true>, 256) / sms()},
-        {resident((const void*)k_resolve<kAny, kG64, kSub>, 64) / sms(),
-         resident((const void*)k_resolve<kAny, kG64, kSub>, 128) / sms()},
+        {resident((const void*)search_kernel<kAny, kG64, kSub>(), 64) / sms(),
+         resident((const void*)search_kernel<kAny, kG64, kSub>(), 128) / sms()},
         {resident((const void*)k_collect<kAny, true, true>, 128) / sms(),
          resident((const void*)k_collect<kAny, true, true>, 256) / sms()}};
     return collect ? v[compressed ? 2 : 0][threads == 256] : v[1][threads == 128];
@@ -973,7 +1096,7 @@ void launch(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Q
                                                                                                         nDev, E, p);
             nl++;
         }
-        k_resolve<kAny, kG64, kSub><<<gr, rt, 0, stream>>>(S, rays, n, nDev, E, p, q, hits, occluded, cnt);
+        search_kernel<kAny, kG64, kSub>()<<<gr, rt, 0, stream>>>(S, rays, n, nDev, E, p, q, hits, occluded, cnt);
         nl += 2;
     }
     k_pending<<<gp, kPendingThreads, 0, stream>>>(E.status, n, nDev, E.queue[c.passes & 1], E.ctl + 4 * c.passes + 2);
@@ -1052,14 +1175,10 @@ cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_
     const int flat = sms() * 4;
     k_init<<<flat, 256, 0, stream>>>(rays, n, nDev, hits, any ? occluded : nullptr, E);
     int nl = 1;
-    // the FP64 grazing instance serves both methods at its level (its
-    // subdivision searches run whole); measured, it also runs the grazing
-    // clip 35% faster with that one-call search compiled in (6.35 against
-    // 4.72 Mrays/s on 2^20 grazing rays), a code-generation effect
     if (any) q.method != 0 ? launch<true, false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl)
                            : launch<true, false>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
-    else if (graze_sin(q.precision) > 0.0f) launch<false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
     else if (q.method != 0) launch<false, false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
+    else if (graze_sin(q.precision) > 0.0f) launch<false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
     else launch<false, false>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
     if (!any && polishes(q.precision))
     {
