@@ -265,7 +265,8 @@ __device__ __forceinline__ bool xAxisIntersection(float& lo, float& hi, float2 A
         float t = A.y / q;
         if (0.0f <= t && t <= 1.0f)
         {
-            float s = (1.0f - t) * A.x + t * B.x;
+            // t B.x is t at the walk's points with x = 1: written so, the sum contracts with the other product
+            float s = B.x == 1.0f ? (1.0f - t) * A.x + t : (1.0f - t) * A.x + t * B.x;
             lo = s; hi = s;
             return true;
         }
@@ -291,6 +292,73 @@ __device__ __forceinline__ bool triangleOriginIntersection(float2& coord, float2
     if (v < 0.0f || u + v > 1.0f) return false;
     coord = make_float2(u, v);
     return true;
+}
+
+// Point k of the walk around the distance patch's column extremes: the lower
+// chain's points 2 and 3, the upper chain back to the left, the start again.
+__device__ __forceinline__ float2 hull_point(const float* ybot, const float* ytop, int k)
+{
+    const float o1 = 1.0f / 3.0f, o2 = 2.0f / 3.0f;
+    return make_float2(k == 0 || k == 3 ? o2 : k == 1 || k == 2 ? 1.0f : k == 4 ? o1 : 0.0f,
+                       k == 0 ? ybot[2] : k == 1 ? ybot[3] : k == 2 ? ytop[3] : k == 3 ? ytop[2] : k == 4 ? ytop[1]
+                                                                                  : k == 5 ? ytop[0] : ybot[0]);
+}
+
+// The x range in which the walk's kept segments meet the x axis
+// (src/Spline_BezierClipping.cu:655-693): a convex-hull scan, xAxisIntersection
+// on every segment it keeps.
+//
+// A segment is only tested for whether it can meet the axis; the divisions are
+// done after the scan, for the first and the last that can (most nets have two
+// of the eight).  A segment is left out only where the test would reject it: both ends on
+// one side, neither so small that A.y - B.y rounds to the other, which puts
+// t = A.y / (A.y - B.y) below 0 or above 1, as rounded.  With the test inline,
+// each of the eight segments was a divergent division.  More than two that can
+// meet the axis: the scan again, testing each in turn.
+__device__ __forceinline__ void hull_scan(const float* ybot, const float* ytop, float& lower, float& upper)
+{
+    const float eps = 1.1920928955078125e-07f;  // FLT_EPSILON
+    float2 P1 = make_float2(0.0f, ybot[0]), P2 = make_float2(1.0f / 3.0f, ybot[1]);
+    float2 A0 = P1, B0 = P1, A1 = P1, B1 = P1;
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+    {
+        const float2 P3 = hull_point(ybot, ytop, k);
+        const float2 a = P2 - P1, b = P3 - P1;
+        const bool keep = k == 7 || a.x * b.y - a.y * b.x >= 0.0f;
+        const float q = P1.y - P2.y;
+        const bool meets = keep && ((__float_as_int(P1.y) ^ __float_as_int(P2.y)) < 0 || q == P1.y || q == -P2.y ||
+                                    fabsf(P1.y) <= eps);
+        A0 = meets && n == 0 ? P1 : A0;
+        B0 = meets && n == 0 ? P2 : B0;
+        A1 = meets ? P1 : A1;
+        B1 = meets ? P2 : B1;
+        n += meets ? 1 : 0;
+        P1 = keep ? P2 : P1;
+        P2 = P3;
+    }
+    float lo, hi;
+    if (n <= 2)
+    {
+        if (n > 0 && xAxisIntersection(lo, hi, A0, B0)) { lower = fminf(lower, lo); upper = fmaxf(upper, hi); }
+        if (n > 1 && xAxisIntersection(lo, hi, A1, B1)) { lower = fminf(lower, lo); upper = fmaxf(upper, hi); }
+        return;
+    }
+    P1 = make_float2(0.0f, ybot[0]);
+    P2 = make_float2(1.0f / 3.0f, ybot[1]);
+#pragma unroll 1
+    for (int k = 0; k < 8; k++)
+    {
+        const float2 P3 = hull_point(ybot, ytop, k);
+        const float2 a = P2 - P1, b = P3 - P1;
+        if (k == 7 || a.x * b.y - a.y * b.x >= 0.0f)
+        {
+            if (xAxisIntersection(lo, hi, P1, P2)) { lower = fminf(lower, lo); upper = fmaxf(upper, hi); }
+            P1 = P2;
+        }
+        P2 = P3;
+    }
 }
 
 // Fat-line clip range of a sub-net (src/Spline_BezierClipping.cu:610-701):
@@ -319,28 +387,7 @@ __device__ __forceinline__ void clip_range(const float2* p, int cutside, float& 
         ybot[i] = fminf(fminf(y0, y1), fminf(y2, y3));
         ytop[i] = fmaxf(fmaxf(y0, y1), fmaxf(y2, y3));
     }
-    const float o1 = 1.0f / 3.0f, o2 = 2.0f / 3.0f;
-    const float2 hull[7] = {make_float2(o2, ybot[2]), make_float2(1.0f, ybot[3]), make_float2(1.0f, ytop[3]),
-                            make_float2(o2, ytop[2]), make_float2(o1, ytop[1]), make_float2(0.0f, ytop[0]),
-                            make_float2(0.0f, ybot[0])};
-    float2 P1 = make_float2(0.0f, ybot[0]), P2 = make_float2(o1, ybot[1]);
-#pragma unroll
-    for (int k = 0; k < 7; k++)
-    {
-        float2 P3 = hull[k];
-        float2 a = P2 - P1, b = P3 - P1;
-        if (a.x * b.y - a.y * b.x >= 0.0f)
-        {
-            float lo, hi;
-            if (xAxisIntersection(lo, hi, P1, P2)) { lower = fminf(lower, lo); upper = fmaxf(upper, hi); }
-            P1 = P2;
-        }
-        P2 = P3;
-    }
-    {
-        float lo, hi;
-        if (xAxisIntersection(lo, hi, P1, P2)) { lower = fminf(lower, lo); upper = fmaxf(upper, hi); }
-    }
+    hull_scan(ybot, ytop, lower, upper);
     lower = lower * 0x0FFp-8f;
     upper = upper + (1.0f - upper) * 0x001p-8f;
 }
