@@ -471,17 +471,113 @@ __device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make
 __device__ __forceinline__ double2 operator*(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ double len2d(double2 a) { return sqrt(a.x * a.x + a.y * a.y); }
 
+// A scheduler's FP64 pipe takes a warp instruction for 64 cycles whatever its
+// active lanes (half a lane a cycle), so the number of FP64 instructions is
+// what FP64 searches cost first.  What they do besides arithmetic --
+// conversions, comparisons, selections -- is done on the numbers' bits, signs
+// that FP32 can tell are taken from FP32, and a popped net is not projected
+// again.  A near-grazing ray of 818 iterations, alone on the GPU: 6.7 ms, 10.8 ms
+// before; what is left is the latency of its chain, 2,300 instructions an
+// iteration.  65,537 grazing rays: 21.5 ms, before 31.0 ms.
+
+// double(f)
+__device__ __forceinline__ double widen(float f)
+{
+    const uint32_t b = __float_as_uint(f), a = b & 0x7FFFFFFFu;
+    if (a - 0x00800000u >= 0x7F000000u) return double(f);  // zero, denormal, not finite
+    return __hiloint2double(int((b & 0x80000000u) | ((a >> 3) + 0x38000000u)), int(b << 29));
+}
+// float(x), rounded to nearest
+__device__ __forceinline__ float narrow(double x)
+{
+    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+    if (((hi >> 20) & 0x7FFu) - 897u >= 254u) return float(x);  // not a normal float
+    uint32_t m = (((hi & 0x7FFFFFFFu) - 0x38000000u) << 3) | (lo >> 29);
+    m += ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (m & 1u)) >> 29;
+    return __uint_as_float((hi & 0x80000000u) | m);
+}
+// The order of finite doubles as that of signed integers, and back.
+__device__ __forceinline__ long long ordered(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll);
+}
+__device__ __forceinline__ double from_ordered(long long k)
+{
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7FFFFFFFFFFFFFFFll));
+}
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7FF00000) == 0x7FF00000; }
+// x >= 0
+__device__ __forceinline__ bool not_negative(double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    return b <= 0x7FF0000000000000ull || b == 0x8000000000000000ull;
+}
+
+__device__ __forceinline__ uint32_t exponent_bits(double x) { return (uint32_t(__double2hiint(x)) >> 20) & 0x7FFu; }
+// x 2^k, away from the ends of the exponent range
+__device__ __forceinline__ double scale2(double x, int k)
+{
+    return __hiloint2double(__double2hiint(x) + k * 0x100000, __double2loint(x));
+}
+
+// a / b, rounded to nearest: a reciprocal by Newton's iteration from FP32, then
+// the quotient corrected by its remainder (P. W. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34,
+// 1990).  Seven FP64 instructions; outside the exponents that this is safe for, the operator.
+__device__ __forceinline__ double quotient(double a, double b)
+{
+    if (exponent_bits(b) - 923u >= 200u || exponent_bits(a) - 523u >= 1000u) return a / b;
+    double y = widen(1.0f / narrow(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+// L divided by its length l = sqrt(|L|^2), each rounded to nearest (L itself
+// where l = 0): Goldschmidt's iteration for the root from FP32, its reciprocal
+// along with it, quotients as above.
+__device__ __forceinline__ double2 unit2d(double2 L)
+{
+    const double s = L.x * L.x + L.y * L.y;
+    if (exponent_bits(s) - 923u >= 200u || exponent_bits(L.x) - 523u >= 1000u || exponent_bits(L.y) - 523u >= 1000u)
+    {
+        const double l = sqrt(s);
+        return l != 0.0 ? make_double2(L.x / l, L.y / l) : L;
+    }
+    const double y0 = widen(rsqrtf(narrow(s)));
+    double g = s * y0, h = scale2(y0, -1);
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    const double l = fma(fma(-g, g, s), h, g);
+    double y = scale2(h, 1);
+    y = fma(y, fma(-l, y, 1.0), y);
+    const double qx = L.x * y, qy = L.y * y;
+    return make_double2(fma(fma(-l, qx, L.x), y, qx), fma(fma(-l, qy, L.y), y, qy));
+}
+
 // xAxisIntersection in double with DBL_EPSILON (src/Spline_BezierClipping.cu:127-156)
 __device__ __forceinline__ bool x_axis_d(double& lo, double& hi, double2 A, double2 B)
 {
-    const double eps = 2.220446049250313e-16;
+    constexpr unsigned long long kAbs = 0x7FFFFFFFFFFFFFFFull, kEps = 0x3CB0000000000000ull, kInf = 0x7FF0000000000000ull;
     const double q = A.y - B.y;
-    if (fabs(q) > eps)
+    const unsigned long long uq = (unsigned long long)__double_as_longlong(q) & kAbs;
+    if (uq > kEps && uq <= kInf)
     {
-        const double t = A.y / q;
-        if (0.0 <= t && t <= 1.0) { lo = hi = (1.0 - t) * A.x + t * B.x; return true; }
+        const double t = quotient(A.y, q);
+        const unsigned long long ut = (unsigned long long)__double_as_longlong(t);
+        if (ut <= 0x3FF0000000000000ull || ut == 0x8000000000000000ull)  // 0 <= t <= 1
+        {
+            lo = hi = B.x == 1.0 ? (1.0 - t) * A.x + t : (1.0 - t) * A.x + t * B.x;  // as xAxisIntersection
+            return true;
+        }
     }
-    else if (fabs(A.y) <= eps)
+    else if (((unsigned long long)__double_as_longlong(A.y) & kAbs) <= kEps)
     {
         lo = fmin(A.x, B.x); hi = fmax(A.x, B.x);
         return true;
@@ -489,52 +585,120 @@ __device__ __forceinline__ bool x_axis_d(double& lo, double& hi, double2 A, doub
     return false;
 }
 
-// clip_range in double (src/Spline_BezierClipping.cu:610-701)
-__device__ __forceinline__ void clip_range_d(const double2* p, int cutside, double& lower, double& upper)
+// Column extremes of four distances each: y[i][0..3].
+__device__ __forceinline__ void extremes_d(const double (*y)[4], double* ybot, double* ytop)
 {
-    lower = 1.0; upper = 0.0;
-    double2 L = p[15] - p[0];
-    const double2 D = p[12] - p[3];
-    L = cutside == 0 ? L + D : L - D;
-    {
-        const double l = len2d(L);
-        if (l != 0.0) L = make_double2(L.x / l, L.y / l);
-    }
-    const double2 N = make_double2(-L.y, L.x);
-    double ytop[4], ybot[4];
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) odd = odd || not_finite(y[i][k]);
 #pragma unroll
     for (int i = 0; i < 4; i++)
     {
-        double y[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++)
+        if (odd)
         {
-            const double2 q = cutside == 0 ? p[4 * k + i] : p[4 * i + k];
-            y[k] = N.x * q.x + N.y * q.y;
+            ybot[i] = fmin(fmin(y[i][0], y[i][1]), fmin(y[i][2], y[i][3]));
+            ytop[i] = fmax(fmax(y[i][0], y[i][1]), fmax(y[i][2], y[i][3]));
+            continue;
         }
-        ybot[i] = fmin(fmin(y[0], y[1]), fmin(y[2], y[3]));
-        ytop[i] = fmax(fmax(y[0], y[1]), fmax(y[2], y[3]));
+        const long long a = ordered(y[i][0]), b = ordered(y[i][1]), c = ordered(y[i][2]), d = ordered(y[i][3]);
+        ybot[i] = from_ordered(min(min(a, b), min(c, d)));
+        ytop[i] = from_ordered(max(max(a, b), max(c, d)));
     }
-    const double o1 = 1.0 / 3.0, o2 = 2.0 / 3.0;
-    const double2 hull[7] = {make_double2(o2, ybot[2]), make_double2(1.0, ybot[3]), make_double2(1.0, ytop[3]),
-                             make_double2(o2, ytop[2]), make_double2(o1, ytop[1]), make_double2(0.0, ytop[0]),
-                             make_double2(0.0, ybot[0])};
-    double2 P1 = make_double2(0.0, ybot[0]), P2 = make_double2(o1, ybot[1]);
+}
+
+// hull_scan in double with DBL_EPSILON.  The walk's x coordinates are 0, 1/3,
+// 2/3 and 1, so their differences are constants chosen by the kept point.
+__device__ __forceinline__ void hull_scan_d(const double* ybot, const double* ytop, double& lower, double& upper)
+{
+    const double X[4] = {0.0, 1.0 / 3.0, 2.0 / 3.0, 1.0};
+    const int at[8] = {2, 3, 3, 2, 1, 0, 0, 0};  // the x of point k
+    const double Y[8] = {ybot[2], ybot[3], ytop[3], ytop[2], ytop[1], ytop[0], ybot[0], 0.0};
+    auto pick = [&](int i, double a, double b, double c, double d) { return i == 0 ? a : i == 1 ? b : i == 2 ? c : d; };
+    auto minus = [&](int x, int i) { return pick(i, X[x] - X[0], X[x] - X[1], X[x] - X[2], X[x] - X[3]); };
+    auto pickf = [&](int i, float a, float b, float c, float d) { return i == 0 ? a : i == 1 ? b : i == 2 ? c : d; };
+    auto minusf = [&](int x, int i) {
+        return pickf(i, float(X[x] - X[0]), float(X[x] - X[1]), float(X[x] - X[2]), float(X[x] - X[3]));
+    };
+    int i1 = 0, i2 = 1;  // the x of P1 (kept) and P2
+    double y1 = ybot[0], y2 = ybot[1];
+    float f1 = narrow(y1), f2 = narrow(y2);
+    int a0 = 0, b0 = 0, a1 = 0, b1 = 0, n = 0;
+    double ya0 = 0.0, yb0 = 0.0, ya1 = 0.0, yb1 = 0.0;
 #pragma unroll
-    for (int k = 0; k < 7; k++)
+    for (int k = 0; k < 8; k++)
     {
-        const double2 P3 = hull[k];
-        const double2 a = P2 - P1, b = P3 - P1;
-        if (a.x * b.y - a.y * b.x >= 0.0)
+        bool keep = true;
+        const float f3 = narrow(Y[k]);
+        if (k < 7)
         {
-            double lo, hi;
+            // the turn's sign in FP32 where it is past the rounding of its inputs and terms, else in FP64
+            const float turn = minusf(i2, i1) * (f3 - f1) - (f2 - f1) * minusf(at[k], i1);
+            keep = turn > 0.0f;
+            if (!(fabsf(turn) > 0x1p-20f * (fabsf(f1) + fabsf(f2) + fabsf(f3))))
+                keep = not_negative(minus(i2, i1) * (Y[k] - y1) - (y2 - y1) * minus(at[k], i1));
+        }
+        // as in hull_scan; ends whose exponents differ by 50 or less do not round away in their difference
+        const long long u = __double_as_longlong(y1), v = __double_as_longlong(y2);
+        const bool meets = keep && ((u ^ v) < 0 || exponent_bits(y1) - exponent_bits(y2) + 50u > 100u ||
+                                    (u & 0x7FFFFFFFFFFFFFFFll) <= 0x3CB0000000000000ll);  // |P1.y| <= DBL_EPSILON
+        const bool first = meets && n == 0;
+        a0 = first ? i1 : a0; ya0 = first ? y1 : ya0; b0 = first ? i2 : b0; yb0 = first ? y2 : yb0;
+        a1 = meets ? i1 : a1; ya1 = meets ? y1 : ya1; b1 = meets ? i2 : b1; yb1 = meets ? y2 : yb1;
+        n += meets ? 1 : 0;
+        i1 = keep ? i2 : i1;
+        y1 = keep ? y2 : y1;
+        f1 = keep ? f2 : f1;
+        i2 = at[k];
+        y2 = Y[k];
+        f2 = f3;
+    }
+    auto point = [&](int i, double y) { return make_double2(pick(i, X[0], X[1], X[2], X[3]), y); };
+    double lo, hi;
+    if (n <= 2)
+    {
+        if (n > 0 && x_axis_d(lo, hi, point(a0, ya0), point(b0, yb0))) { lower = fmin(lower, lo); upper = fmax(upper, hi); }
+        if (n > 1 && x_axis_d(lo, hi, point(a1, ya1), point(b1, yb1))) { lower = fmin(lower, lo); upper = fmax(upper, hi); }
+        return;
+    }
+    double2 P1 = make_double2(0.0, ybot[0]), P2 = make_double2(X[1], ybot[1]);
+#pragma unroll 1
+    for (int k = 0; k < 8; k++)
+    {
+        const double2 P3 = make_double2(k == 0 || k == 3 ? X[2] : k == 1 || k == 2 ? 1.0 : k == 4 ? X[1] : 0.0,
+                                        k == 0 ? ybot[2] : k == 1 ? ybot[3] : k == 2 ? ytop[3] : k == 3 ? ytop[2]
+                                        : k == 4 ? ytop[1] : k == 5 ? ytop[0] : ybot[0]);
+        const double2 a = P2 - P1, b = P3 - P1;
+        if (k == 7 || a.x * b.y - a.y * b.x >= 0.0)
+        {
             if (x_axis_d(lo, hi, P1, P2)) { lower = fmin(lower, lo); upper = fmax(upper, hi); }
             P1 = P2;
         }
         P2 = P3;
     }
-    double lo, hi;
-    if (x_axis_d(lo, hi, P1, P2)) { lower = fmin(lower, lo); upper = fmax(upper, hi); }
+}
+
+// clip_range in double (src/Spline_BezierClipping.cu:610-701); p(i) is the
+// net's point i.
+template<class Net> __device__ __forceinline__ void clip_range_d(Net&& p, int cutside, double& lower, double& upper)
+{
+    lower = 1.0; upper = 0.0;
+    double2 L = p(15) - p(0);
+    const double2 D = p(12) - p(3);
+    L = unit2d(cutside == 0 ? L + D : L - D);
+    const double2 N = make_double2(-L.y, L.x);
+    double y[4][4], ytop[4], ybot[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+        {
+            const double2 q = cutside == 0 ? p(4 * k + i) : p(4 * i + k);
+            y[i][k] = N.x * q.x + N.y * q.y;
+        }
+    extremes_d(y, ybot, ytop);
+    hull_scan_d(ybot, ytop, lower, upper);
     lower = lower * 0x0FFp-8;
     upper = upper + (1.0 - upper) * 0x001p-8;
 }
@@ -542,11 +706,8 @@ __device__ __forceinline__ void clip_range_d(const double2* p, int cutside, doub
 // FP64 bounds of an FP32 sub-net, rounded outward.
 __device__ __forceinline__ void clip_range64(const float2* p, int cutside, float& lower, float& upper)
 {
-    double2 q[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) q[i] = make_double2(p[i].x, p[i].y);
     double lo, hi;
-    clip_range_d(q, cutside, lo, hi);
+    clip_range_d([&](int i) { return make_double2(widen(p[i].x), widen(p[i].y)); }, cutside, lo, hi);
     lower = __double2float_rd(lo);
     upper = __double2float_ru(hi);
 }
@@ -572,8 +733,8 @@ __device__ __forceinline__ void project_net64(float2* net, const float4* __restr
     for (int i = 0; i < 16; i++)
     {
         const float4 q = __ldg(P + i);
-        const double3 Q = make_double3(double(q.x) - o.x, double(q.y) - o.y, double(q.z) - o.z);
-        net[i] = make_float2(float(dot_d(a0, Q)), float(dot_d(a1, Q)));
+        const double3 Q = make_double3(widen(q.x) - o.x, widen(q.y) - o.y, widen(q.z) - o.z);
+        net[i] = make_float2(narrow(dot_d(a0, Q)), narrow(dot_d(a1, Q)));
     }
 }
 
@@ -665,27 +826,12 @@ struct ClipState
 // grazing get the FP64 bounds).  kG64 = false compiles the FP64 path out
 // (searches that never take it: a smaller loop body for the instruction
 // cache).
-// ob, wo, wd: the candidate's object and the world ray, from which a
-// near-grazing candidate's ray is recomputed in double (to_local64); a null
-// ob projects it from the FP32 ray in the sink.  ray64: where that ray
-// (origin, direction) is kept for the search's projections, a six-double
-// array in local memory (read only where a projection starts, it would
-// otherwise hold twelve registers through the whole search).
+// A near-grazing search (c.b64) also needs clip_begin64.
 template<bool kG64 = true>
-__device__ __forceinline__ void clip_begin(ClipState& c, const HitSink& sink, float tol, float grazeSin,
-                                           volatile double* ray64, const DevObject* ob = nullptr, float3 wo = {},
-                                           float3 wd = {})
+__device__ __forceinline__ void clip_begin(ClipState& c, const HitSink& sink, float tol, float grazeSin)
 {
     c.b64 = kG64 && grazeSin > 0.0f && near_grazing(sink.P, sink.d, grazeSin);
     c.tol = c.b64 ? kGrazeTol : tol;
-    if (kG64 && c.b64)
-    {
-        Ray64 r;
-        if (ob) r = to_local64(*ob, wo, wd);
-        else r = Ray64 {make_double3(sink.o.x, sink.o.y, sink.o.z), make_double3(sink.d.x, sink.d.y, sink.d.z)};
-        ray64[0] = r.o.x; ray64[1] = r.o.y; ray64[2] = r.o.z;
-        ray64[3] = r.d.x; ray64[4] = r.d.y; ray64[5] = r.d.z;
-    }
     c.fresh = true;
     c.tposed = false;
     c.emin = make_float2(0.0f, 0.0f);
@@ -694,6 +840,22 @@ __device__ __forceinline__ void clip_begin(ClipState& c, const HitSink& sink, fl
     c.sl = 0;
     c.it = 0;
     c.found = false;
+}
+
+// The start of a near-grazing search: projects the net from the ray in double,
+// recomputed from the world ray and the candidate's object (to_local64), or the
+// FP32 ray in the sink where ob is null.  net0 keeps the projected net in local
+// memory for the search's pops, which would have to project it again: 144 FP64 instructions.
+__device__ __forceinline__ void clip_begin64(ClipState& c, const HitSink& sink, volatile float* net0, const DevObject* ob,
+                                             float3 wo, float3 wd)
+{
+    Ray64 r;
+    if (ob) r = to_local64(*ob, wo, wd);
+    else r = Ray64 {make_double3(sink.o.x, sink.o.y, sink.o.z), make_double3(sink.d.x, sink.d.y, sink.d.z)};
+    project_net64(c.buf, sink.P, r.o, r.d);
+#pragma unroll
+    for (int i = 0; i < 16; i++) { net0[2 * i] = c.buf[i].x; net0[2 * i + 1] = c.buf[i].y; }
+    c.fresh = false;
 }
 
 // Transposes the 4x4 net in registers where t holds.  A cut along v
@@ -753,14 +915,16 @@ __device__ __forceinline__ ClipNext clip_pop(ClipState& c, const float4* st)
     return kClipProject;
 }
 
-// Projects the patch; after a pop also derives the popped interval's sub-net
-// (in the natural orientation).
+// Projects the patch (a near-grazing search's projection is in net0); after a
+// pop also derives the popped interval's sub-net (in the natural orientation).
 template<bool kG64> __device__ __forceinline__ void clip_project(ClipState& c, const HitSink& sink,
-                                                                 const volatile double* ray64)
+                                                                 const volatile float* net0)
 {
     if (kG64 && c.b64)
-        project_net64(c.buf, sink.P, make_double3(ray64[0], ray64[1], ray64[2]),
-                      make_double3(ray64[3], ray64[4], ray64[5]));
+    {
+#pragma unroll
+        for (int i = 0; i < 16; i++) c.buf[i] = make_float2(net0[2 * i], net0[2 * i + 1]);
+    }
     else project_net(c.buf, sink.P, sink.o, sink.d);
     c.tposed = false;
     if (!c.fresh)
@@ -829,17 +993,22 @@ static __device__ __noinline__ bool clip_patch(HitSink& sink, float tol, float g
 {
     float4 st[kClipStack];
     ClipState c;
-    volatile double ray64[6];
-    clip_begin(c, sink, tol, grazeSin, ray64, ob, wo, wd);
+    volatile float net0[32];
+    clip_begin(c, sink, tol, grazeSin);
     const float tol2 = below_sqrt(c.tol);
     ClipNext next = kClipProject;
+    if (c.b64)
+    {
+        clip_begin64(c, sink, net0, ob, wo, wd);
+        next = clip_test<true>(c, tol2, lc);
+    }
     while (next != kClipOver && !(anyHit && c.found))
     {
         if (next == kClipRoot) next = clip_root(c, st, sink);
         else
         {
             if (next == kClipCut) next = clip_cut<true>(c, st, lc);
-            if (next == kClipProject) { clip_project<true>(c, sink, ray64); next = kClipCut; }
+            if (next == kClipProject) { clip_project<true>(c, sink, net0); next = kClipCut; }
             if (next == kClipCut) next = clip_test<true>(c, tol2, lc);
         }
     }

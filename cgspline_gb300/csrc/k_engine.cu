@@ -662,7 +662,7 @@ template<bool kAny> struct ListWalk
 // kG64: the search may take the FP64 grazing path (precision levels 3 and 5);
 // the other levels run an instance without that code.  The FP32 instances are
 // held to 128 registers, four 128-thread blocks per SM.
-enum : int { kPartWalk, kPartProject, kPartCut, kPartRoot, kPartProject64, kPartCut64, kPartNone };
+enum : int { kPartWalk, kPartProject, kPartCut, kPartRoot, kPartBegin64, kPartCut64, kPartNone };
 template<bool kAny, bool kG64>
 __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene S, RaysSoA rays, uint32_t n0,
                                                                          const uint32_t* nDev, Eng E, int pass, Query q,
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
     const uint32_t n = nDev ? *nDev : n0;
     LocalCounters lc;
     float4 stack[kClipStack];
-    volatile double ray64[6];  // kG64: a near-grazing search's ray in double
+    volatile float net0[32];  // kG64: a near-grazing search's projected net
     ClipState c;
     c.b64 = false;
     c.sl = 0;
@@ -774,8 +774,8 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
                 if (w.next(S, E, hits, sink))
                 {
                     lc.candidates++;
-                    clip_begin<kG64>(c, sink, q.tol, graze_sin(q.precision), ray64, &S.objects[w.obj], w.o, w.d);
-                    part = kG64 && c.b64 ? kPartProject64 : kPartProject;
+                    clip_begin<kG64>(c, sink, q.tol, graze_sin(q.precision));
+                    part = kG64 && c.b64 ? kPartBegin64 : kPartProject;
                 }
                 else
                 {
@@ -790,10 +790,14 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
         if (run == kPartRoot) next = clip_root(c, stack, sink);
         else
         {
-            // c.b64 is uniform over the lanes of a part; naming it lets each part hold one kind of code
-            if (run == kPartProject || (kG64 && run == kPartProject64))
+            if (kG64 && run == kPartBegin64)
             {
-                clip_project<kG64>(c, sink, ray64);
+                clip_begin64(c, sink, net0, &S.objects[w.obj], w.o, w.d);
+                next = kClipCut;
+            }
+            else if (run == kPartProject)
+            {
+                clip_project<kG64>(c, sink, net0);
                 next = kClipCut;
             }
             else
@@ -803,9 +807,8 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
         if (kAny && c.found) next = kClipOver;  // an any-hit search ends at its first root
         if (next != kClipOver)
         {
-            const bool b64 = kG64 && c.b64;
             part = next == kClipRoot ? kPartRoot
-                   : next == kClipCut ? (b64 ? kPartCut64 : kPartCut) : (b64 ? kPartProject64 : kPartProject);
+                   : next == kClipProject ? kPartProject : kG64 && c.b64 ? kPartCut64 : kPartCut;
             continue;
         }
         part = kPartWalk;

@@ -158,7 +158,7 @@ __device__ __noinline__ bool clip64(Sink64& sink, double tol, LocalCounters& lc)
         else
         {
             double lower, upper;
-            clip_range_d(buf, cutside, lower, upper);
+            clip_range_d([&](int i) { return buf[i]; }, cutside, lower, upper);
             const double delta = upper - lower;
             if (delta > 0.8)
             {
