@@ -816,8 +816,7 @@ struct ClipState
     bool found, b64;  // b64: FP64 projection and fat-line bounds (near-grazing)
     bool fresh;       // the next projection is the search's first
     bool tposed;      // buf holds the transposed net (left so by a cut along v)
-    // The resumable subdivision search (subdiv_step) keeps its walk in the
-    // same state: the bit trail in cutsideStack, the level in sl, the
+    // The resumable subdivision search keeps its walk in the same state: the bit trail in cutsideStack, the level in sl, the
     // sub-domain's integer coordinates in the bits of emin (which it does not
     // use otherwise), and `fresh` as its reload flag.
 };
@@ -1021,72 +1020,88 @@ static __device__ __noinline__ bool clip_patch(HitSink& sink, float tol, float g
 // backtrack, accept a leaf whose bounding box strictly contains the origin
 // once both diagonals are below tol (or after 31 halvings).  The sub-domain
 // follows the buffer: after k halvings su = 2^-ceil(k/2), sv = 2^-floor(k/2).
-// subdiv_patch as a resumable search for the query engine: subdiv_begin
-// projects the net; each subdiv_step runs up to `levels` iterations of the
-// same loop and returns false when the search is over (c.found: a root was
-// kept), so lanes of a warp interleave their searches and refill from the
-// queue one search at a time.  The iterations are subdiv_patch's, in the same
-// order, so the results are the same bit for bit.
-__device__ __forceinline__ void subdiv_begin(ClipState& c, const HitSink& sink, float tol)
+//
+// For the query engine the search comes in resumable parts, as the clipping
+// search does: subdiv_begin, subdiv_project (the net, after a backtrack with the
+// sub-domain's slices), subdiv_cut (one iteration of subdiv_patch's loop up to a
+// leaf) and subdiv_root (a leaf's roots).  The iterations are subdiv_patch's, in the
+// same order, so the results are the same bit for bit.
+__device__ __forceinline__ void subdiv_begin(ClipState& c)
 {
-    project_net(c.buf, sink.P, sink.o, sink.d);
     c.cutsideStack = 0; c.sl = 0; c.it = 0;
     c.emin = make_float2(__uint_as_float(0u), __uint_as_float(0u));  // tu, tv
-    c.fresh = false; c.found = false; c.tol = tol;
+    c.fresh = false; c.found = false;
 }
-__device__ __forceinline__ bool subdiv_step(ClipState& c, HitSink& sink, LocalCounters& lc, int levels)
+__device__ __forceinline__ void subdiv_domain(const ClipState& c, float2& emin, float2& emax)
+{
+    const int k = c.sl;
+    const float su = ldexpf(1.0f, -((k + 1) >> 1)), sv = ldexpf(1.0f, -(k >> 1));
+    emin = make_float2(float(__float_as_uint(c.emin.x)) * su, float(__float_as_uint(c.emin.y)) * sv);
+    emax = make_float2(emin.x + su, emin.y + sv);
+}
+__device__ __forceinline__ void subdiv_project(ClipState& c, const HitSink& sink)
+{
+    project_net(c.buf, sink.P, sink.o, sink.d);
+    c.tposed = false;
+    if (!c.fresh) return;
+    float2 emin, emax;
+    subdiv_domain(c, emin, emax);
+    subpatchU(c.buf, emin.x, emax.x);
+    subpatchV(c.buf, emin.y, emax.y);
+}
+// To the sibling postponed last, or the search's end.
+__device__ __forceinline__ ClipNext subdiv_back(ClipState& c)
 {
     uint32_t trail = uint32_t(c.cutsideStack), tu = __float_as_uint(c.emin.x), tv = __float_as_uint(c.emin.y);
     int k = c.sl;
-    bool more = true;
-    for (int s = 0; s < levels; s++)
-    {
-        if (c.it >= 4 * kMaxClipIterations) { lc.errors |= kErrClipIterations; more = false; break; }
-        c.it++;
-        lc.iterations++;
-        const float su = ldexpf(1.0f, -((k + 1) >> 1)), sv = ldexpf(1.0f, -(k >> 1));
-        const float2 emin = make_float2(float(tu) * su, float(tv) * sv);
-        const float2 emax = make_float2(emin.x + su, emin.y + sv);
-        if (c.fresh)
-        {
-            project_net(c.buf, sink.P, sink.o, sink.d);
-            subpatchU(c.buf, emin.x, emax.x);
-            subpatchV(c.buf, emin.y, emax.y);
-        }
-        float2 bmin = c.buf[0], bmax = c.buf[0];
-#pragma unroll
-        for (int i = 1; i < 16; i++)
-        {
-            bmin = make_float2(fminf(bmin.x, c.buf[i].x), fminf(bmin.y, c.buf[i].y));
-            bmax = make_float2(fmaxf(bmax.x, c.buf[i].x), fmaxf(bmax.y, c.buf[i].y));
-        }
-        if (bmin.x < 0.0f && bmin.y < 0.0f && bmax.x > 0.0f && bmax.y > 0.0f)
-        {
-            if ((len2(c.buf[3] - c.buf[12]) < c.tol && len2(c.buf[15] - c.buf[0]) < c.tol) || k >= 31)
-                c.found |= approximateIntersection(sink, c.buf, emin, emax);
-            else
-            {
-                c.fresh = false;
-                if ((k & 1) == 0) { subpatchU(c.buf, 0.0f, 0.5f); tu <<= 1; }
-                else { subpatchV(c.buf, 0.0f, 0.5f); tv <<= 1; }
-                trail <<= 1;
-                ++k;
-                continue;
-            }
-        }
-        const int ones = __clz(__brev(~trail));
-        if (ones >= k) { more = false; break; }
-        const int hi = k - 1, lo = k - ones;
-        const int evens = (hi / 2) - ((lo + 1) / 2) + 1;
-        tu >>= evens;
-        tv >>= (ones - evens);
-        k -= ones;
-        trail = (trail >> ones) | 1u;
-        if (((k - 1) & 1) == 0) tu |= 1u; else tv |= 1u;
-        c.fresh = true;
-    }
+    const int ones = __clz(__brev(~trail));
+    if (ones >= k) return kClipOver;
+    // levels k-1 .. k-ones are undone: even levels were u cuts
+    const int hi = k - 1, lo = k - ones;
+    const int evens = (hi / 2) - ((lo + 1) / 2) + 1;
+    tu >>= evens;
+    tv >>= (ones - evens);
+    k -= ones;
+    trail = (trail >> ones) | 1u;
+    if (((k - 1) & 1) == 0) tu |= 1u; else tv |= 1u;
     c.cutsideStack = int(trail); c.emin = make_float2(__uint_as_float(tu), __uint_as_float(tv)); c.sl = k;
-    return more;
+    c.fresh = true;
+    return kClipProject;
+}
+// A level's cut along v is one along u of the transposed net, as in the
+// clipping search, so a warp's lanes cut together whatever their levels.
+__device__ __forceinline__ ClipNext subdiv_cut(ClipState& c, float tol2, LocalCounters& lc)
+{
+    if (c.it >= 4 * kMaxClipIterations) { lc.errors |= kErrClipIterations; return kClipOver; }
+    c.it++;
+    lc.iterations++;
+    float2 bmin = c.buf[0], bmax = c.buf[0];
+#pragma unroll
+    for (int i = 1; i < 16; i++)
+    {
+        bmin = make_float2(fminf(bmin.x, c.buf[i].x), fminf(bmin.y, c.buf[i].y));
+        bmax = make_float2(fmaxf(bmax.x, c.buf[i].x), fmaxf(bmax.y, c.buf[i].y));
+    }
+    if (!(bmin.x < 0.0f && bmin.y < 0.0f && bmax.x > 0.0f && bmax.y > 0.0f)) return subdiv_back(c);
+    const float2 e = c.buf[3] - c.buf[12], f = c.buf[15] - c.buf[0];
+    if ((dot2(e, e) <= tol2 && dot2(f, f) <= tol2) || c.sl >= 31) return kClipRoot;
+    const bool tr = (c.sl & 1) != 0;
+    transpose_if(c.buf, tr != c.tposed);
+    c.tposed = tr;
+    subpatchU(c.buf, 0.0f, 0.5f);
+    const uint32_t tu = __float_as_uint(c.emin.x), tv = __float_as_uint(c.emin.y);
+    c.emin = make_float2(__uint_as_float(tr ? tu : tu << 1), __uint_as_float(tr ? tv << 1 : tv));
+    c.cutsideStack = int(uint32_t(c.cutsideStack) << 1);
+    c.sl++;
+    return kClipCut;
+}
+__device__ __forceinline__ ClipNext subdiv_root(ClipState& c, HitSink& sink)
+{
+    float2 emin, emax;
+    subdiv_domain(c, emin, emax);
+    const float2 p3 = c.tposed ? c.buf[12] : c.buf[3], p12 = c.tposed ? c.buf[3] : c.buf[12];
+    c.found |= approximateIntersection(sink, c.buf[0], p3, p12, c.buf[15], emin, emax);
+    return subdiv_back(c);
 }
 
 static __device__ __noinline__ bool subdiv_patch(HitSink& sink, float tol, LocalCounters& lc)
