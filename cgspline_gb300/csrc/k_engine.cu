@@ -153,6 +153,32 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t* fetch, bool need, uint3
     return need ? base + __popc(m & lt) : EMPTY;
 }
 
+// Where a kernel's warps take their rays.  A pass of the whole query: pass 0
+// takes every ray, a later pass the queue of rays that parked; which: 0 the
+// traversal's counter, 1 the searches'.  (Everything but m is recomputed from the
+// kernel's arguments, so that it holds no registers.)
+template<int which> struct PassSource
+{
+    const Eng& E;
+    int pass;
+    uint32_t m;
+    __device__ __forceinline__ PassSource(const Eng& E, int pass, uint32_t n0, const uint32_t* nDev)
+        : E(E), pass(pass), m(pass == 0 ? (nDev ? *nDev : n0) : E.ctl[4 * pass + 2])
+    {
+    }
+    __device__ __forceinline__ uint32_t* fetch() const { return E.ctl + 4 * pass + which; }
+    __device__ __forceinline__ uint32_t ray(uint32_t k) const { return pass == 0 ? k : E.queue[pass & 1][k]; }
+};
+// One warp's own rays: m of them from a queue, or from `base` on.
+struct WarpSource
+{
+    uint32_t* next;
+    uint32_t m, base;
+    const uint32_t* queue;
+    __device__ __forceinline__ uint32_t* fetch() const { return next; }
+    __device__ __forceinline__ uint32_t ray(uint32_t k) const { return queue ? queue[k] : base + k; }
+};
+
 __device__ __forceinline__ void load_ray(const RaysSoA& r, uint32_t i, float3& o, float3& d, float& tmax)
 {
     o = f3(r.ox[i], r.oy[i], r.oz[i]);
@@ -180,17 +206,13 @@ __device__ __forceinline__ void load_ray(const RaysSoA& r, uint32_t i, float3& o
 //
 // kWalk: some surface has a walk tree; stores without any run an instance
 // without that code.
-template<bool kAny, bool kQ, bool kWalk>
-__global__ void __launch_bounds__(kCollectThreads, 4) k_collect(DevScene S, RaysSoA rays, uint32_t n0,
-                                                                const uint32_t* nDev, Eng E, int pass, int cache,
-                                                                Counters* cnt)
+template<bool kAny, bool kQ, bool kWalk, class Source>
+__device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, int pass, int cache,
+                                             const Source& src, uint32_t* ring, LocalCounters& lc, uint32_t& nrays)
 {
     // entry s of this lane's ring at ring[s * blockDim.x + threadIdx.x]; the
     // ring's state packs its top slot (bits 0-2) with `rvalid` (bits 3-6)
-    __shared__ uint32_t ring[kRing * kCollectThreads];
     uint32_t rstate = 0;
-    const uint32_t n = nDev ? *nDev : n0;
-    LocalCounters lc;
     bool active = false, exhausted = false, jumped = false;
     uint32_t rid = 0, ncand = 0;
     // o, inv, limit: the world ray and its culling bound; co, ci, clim: those
@@ -204,19 +226,16 @@ __global__ void __launch_bounds__(kCollectThreads, 4) k_collect(DevScene S, Rays
     bool walk = true;     // false: the object in hand is walked on the reference tree
     uint32_t topIdx = 0;  // the ray's object-level BVH (its group's)
     BvhRef B {};  // the BVH walked now; its hash parameters are read at a table lookup
-    uint32_t nrays = 0;
     uint2* list = nullptr;
-    // pass 0 walks every ray; a later pass only the queue of rays that parked
-    const uint32_t m = pass == 0 ? n : E.ctl[4 * pass + 2];
-    const uint32_t* queue = E.queue[pass & 1];
+    const uint32_t m = src.m;
     for (;;)
     {
         const bool need = !active && !exhausted;
         // a lane the packet rule holds back gets EMPTY (ray counts stay below 2^31)
-        const uint32_t idx = warp_fetch(E.ctl + 4 * pass, need, E.packetWidth, active);
+        const uint32_t idx = warp_fetch(src.fetch(), need, E.packetWidth, active);
         if (need && idx != EMPTY)
         {
-            const uint32_t r = idx < m ? (pass == 0 ? idx : queue[idx]) : 0u;
+            const uint32_t r = idx < m ? src.ray(idx) : 0u;
             if (idx >= m)
                 exhausted = true;
             else if (pass == 0 && rays.group && __ldg(rays.group + r) >= S.ngroups)
@@ -474,6 +493,17 @@ __global__ void __launch_bounds__(kCollectThreads, 4) k_collect(DevScene S, Rays
             active = false;
         }
     }
+}
+
+template<bool kAny, bool kQ, bool kWalk>
+__global__ void __launch_bounds__(kCollectThreads, 4) k_collect(DevScene S, RaysSoA rays, uint32_t n0,
+                                                                const uint32_t* nDev, Eng E, int pass, int cache,
+                                                                Counters* cnt)
+{
+    __shared__ uint32_t ring[kRing * kCollectThreads];
+    LocalCounters lc;
+    uint32_t nrays = 0;
+    collect_rays<kAny, kQ, kWalk>(S, rays, E, pass, cache, PassSource<0>(E, pass, n0, nDev), ring, lc, nrays);
     flush_counters(cnt, lc, nrays);
 }
 
@@ -503,14 +533,13 @@ __device__ __forceinline__ bool visits_first(const DevScene& S, const DevBVH& H,
 // sort of each object's patches (two or three on most rays, in nearly that
 // order already).  What was collected on the reference tree is in order and stays.
 constexpr int kOrderThreads = 128;
-__global__ void __launch_bounds__(kOrderThreads) k_order(DevScene S, RaysSoA rays, uint32_t n0, const uint32_t* nDev,
-                                                         Eng E, int pass)
+template<class Source>
+__device__ __forceinline__ void order_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, const Source& src,
+                                           uint32_t first, uint32_t stride)
 {
-    const uint32_t m = pass == 0 ? (nDev ? *nDev : n0) : E.ctl[4 * pass + 2];
-    const uint32_t* queue = E.queue[pass & 1];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+    for (uint32_t i = first; i < src.m; i += stride)
     {
-        const uint32_t rid = pass == 0 ? i : queue[i];
+        const uint32_t rid = src.ray(i);
         const uint32_t count = E.count[rid];
         uint2* list = E.list + size_t(rid) * kChunk;
         for (uint32_t k = 0; k + 2 < count; k++)
@@ -544,6 +573,12 @@ __global__ void __launch_bounds__(kOrderThreads) k_order(DevScene S, RaysSoA ray
             k = j - 1;
         }
     }
+}
+__global__ void __launch_bounds__(kOrderThreads) k_order(DevScene S, RaysSoA rays, uint32_t n0, const uint32_t* nDev,
+                                                         Eng E, int pass)
+{
+    order_rays(S, rays, E, PassSource<0>(E, pass, n0, nDev), blockIdx.x * blockDim.x + threadIdx.x,
+               gridDim.x * blockDim.x);
 }
 
 // ------------------------------------------------------------ resolve --
@@ -760,13 +795,11 @@ template<bool kAny> __device__ __forceinline__ void lend_settle(Lend& L, int& pa
     __syncwarp();
 }
 
-template<bool kAny, bool kG64>
-__global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene S, RaysSoA rays, uint32_t n0,
-                                                                         const uint32_t* nDev, Eng E, int pass, Query q,
-                                                                         HitsSoA hits, int32_t* occluded, Counters* cnt)
+template<bool kAny, bool kG64, class Source>
+__device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, int pass, const Query& q,
+                                          HitsSoA& hits, int32_t* occluded, const Source& src, Lend& L,
+                                          LocalCounters& lc)
 {
-    const uint32_t n = nDev ? *nDev : n0;
-    LocalCounters lc;
     float4 stack[kClipStack];
     volatile float net0[32];  // kG64: a near-grazing search's projected net
     ClipState c;
@@ -778,12 +811,8 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
     bool have = false;   // the lane has a ray
     bool thief = false;  // the lane searches an interval borrowed from another lane's search
     bool lent = false;   // closest hit: the lane's search has lent intervals
-    __shared__ Lend lend[kAny || kG64 ? 1 : kResolveThreads / 32];
-    Lend& L = lend[kAny || kG64 ? 0 : threadIdx.x / 32];
     const float tol2 = below_sqrt(q.tol), tol2graze = kG64 ? below_sqrt(kGrazeTol) : 0.0f;
-    // pass 0 resolves every ray; a later pass the rays its traversal walked
-    const uint32_t m = pass == 0 ? n : E.ctl[4 * pass + 2];
-    const uint32_t* queue = E.queue[pass & 1];
+    const uint32_t m = src.m;
     for (;;)
     {
         if constexpr (!kG64)
@@ -858,10 +887,10 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
         if (run == kPartWalk)
         {
             const bool need = part == kPartWalk && !have;
-            const uint32_t idx = warp_fetch(E.ctl + 4 * pass + 1, need);
+            const uint32_t idx = warp_fetch(src.fetch(), need);
             if (need)
             {
-                if (idx < m) have = w.take(rays, E, pass, pass == 0 ? idx : queue[idx]);
+                if (idx < m) have = w.take(rays, E, pass, src.ray(idx));
                 else part = kPartNone;
             }
             if (part == kPartWalk && have)
@@ -926,6 +955,17 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
             part = kPartNone;
         }
     }
+}
+
+template<bool kAny, bool kG64>
+__global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene S, RaysSoA rays, uint32_t n0,
+                                                                         const uint32_t* nDev, Eng E, int pass, Query q,
+                                                                         HitsSoA hits, int32_t* occluded, Counters* cnt)
+{
+    __shared__ Lend lend[kAny || kG64 ? 1 : kResolveThreads / 32];
+    LocalCounters lc;
+    clip_rays<kAny, kG64>(S, rays, E, pass, q, hits, occluded, PassSource<1>(E, pass, n0, nDev),
+                          lend[kAny || kG64 ? 0 : threadIdx.x / 32], lc);
     flush_counters(cnt, lc, 0);
 }
 
@@ -936,25 +976,20 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
 // has not reached; the first (largest) one is at the trail's first 0 bit.
 // 131,101 rays on a 2,048-patch torus, the longest of 3,429 bisections: 0.91 ms
 // a query, 1.81 ms with every part each time round and no lending.
-template<bool kAny>
-__global__ void __launch_bounds__(kResolveThreads, 4) k_subdivide(DevScene S, RaysSoA rays, uint32_t n0,
-                                                                  const uint32_t* nDev, Eng E, int pass, Query q,
-                                                                  HitsSoA hits, int32_t* occluded, Counters* cnt)
+template<bool kAny, class Source>
+__device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, int pass,
+                                               const Query& q, HitsSoA& hits, int32_t* occluded, const Source& src,
+                                               Lend& L, LocalCounters& lc)
 {
-    const uint32_t n = nDev ? *nDev : n0;
-    LocalCounters lc;
     ClipState c;
     HitSink sink {nullptr, f3(0, 0, 0), f3(0, 0, 1), 0.0f, make_float2(0, 0)};
     ListWalk<kAny> w;
     int part = kPartWalk;
     bool have = false, thief = false, lent = false;
-    __shared__ Lend lend[kAny ? 1 : kResolveThreads / 32];
-    Lend& L = lend[kAny ? 0 : threadIdx.x / 32];
     const float tol2 = below_sqrt(q.tol);
     c.sl = 0;
     c.found = false;
-    const uint32_t m = pass == 0 ? n : E.ctl[4 * pass + 2];
-    const uint32_t* queue = E.queue[pass & 1];
+    const uint32_t m = src.m;
     for (;;)
     {
         if (!kAny && __ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
@@ -1024,10 +1059,10 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_subdivide(DevScene S, Ra
         if (run == kPartWalk)
         {
             const bool need = part == kPartWalk && !have;
-            const uint32_t idx = warp_fetch(E.ctl + 4 * pass + 1, need);
+            const uint32_t idx = warp_fetch(src.fetch(), need);
             if (need)
             {
-                if (idx < m) have = w.take(rays, E, pass, pass == 0 ? idx : queue[idx]);
+                if (idx < m) have = w.take(rays, E, pass, src.ray(idx));
                 else part = kPartNone;
             }
             if (part == kPartWalk && have)
@@ -1081,10 +1116,41 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_subdivide(DevScene S, Ra
             part = kPartNone;
         }
     }
+}
+
+template<bool kAny>
+__global__ void __launch_bounds__(kResolveThreads, 4) k_subdivide(DevScene S, RaysSoA rays, uint32_t n0,
+                                                                  const uint32_t* nDev, Eng E, int pass, Query q,
+                                                                  HitsSoA hits, int32_t* occluded, Counters* cnt)
+{
+    __shared__ Lend lend[kAny ? 1 : kResolveThreads / 32];
+    LocalCounters lc;
+    subdivide_rays<kAny>(S, rays, E, pass, q, hits, occluded, PassSource<1>(E, pass, n0, nDev),
+                         lend[kAny ? 0 : threadIdx.x / 32], lc);
     flush_counters(cnt, lc, 0);
 }
 
-// Rays unfinished after the last pass: the inline search from the start.
+// A ray unfinished after the last pass: the inline search from the start.
+template<bool kAny>
+__device__ __forceinline__ void rest_ray(const DevScene& S, const RaysSoA& rays, const Query& q, HitsSoA& hits,
+                                         int32_t* occluded, uint32_t rid, LocalCounters& lc)
+{
+    float3 o, d; float tmax;
+    load_ray(rays, rid, o, d, tmax);
+    Query q32 = q;
+    q32.precision = search_only(q.precision);  // the polish runs afterwards
+    const uint32_t g = rays.group ? rays.group[rid] : 0u;
+    if (g >= S.ngroups) return;
+    if (kAny)
+        occluded[rid] = scene_any(S, g, o, d, tmax, q32, lc) ? 0 : -1;
+    else
+    {
+        HitRecord h {tmax, 0.0f, 0.0f, -1, -1};
+        int ob = scene_closest(S, g, o, d, tmax, q32, h, lc);
+        hits.t[rid] = ob >= 0 ? h.t : tmax; hits.u[rid] = h.u; hits.v[rid] = h.v;
+        hits.patch[rid] = ob >= 0 ? h.patch : -1; hits.object[rid] = ob;
+    }
+}
 template<bool kAny>
 __global__ void __launch_bounds__(128) k_rest(DevScene S, RaysSoA rays, Eng E, int passes, Query q, HitsSoA hits,
                                               int32_t* occluded, Counters* cnt)
@@ -1097,22 +1163,7 @@ __global__ void __launch_bounds__(128) k_rest(DevScene S, RaysSoA rays, Eng E, i
     for (uint32_t i = tid; i < m; i += nt)
     {
         const uint32_t rid = queue[i];
-        if (E.status[rid] != kPending) continue;
-        float3 o, d; float tmax;
-        load_ray(rays, rid, o, d, tmax);
-        Query q32 = q;
-        q32.precision = search_only(q.precision);  // the polish kernel runs afterwards
-        const uint32_t g = rays.group ? rays.group[rid] : 0u;
-        if (g >= S.ngroups) continue;
-        if (kAny)
-            occluded[rid] = scene_any(S, g, o, d, tmax, q32, lc) ? 0 : -1;
-        else
-        {
-            HitRecord h {tmax, 0.0f, 0.0f, -1, -1};
-            int ob = scene_closest(S, g, o, d, tmax, q32, h, lc);
-            hits.t[rid] = ob >= 0 ? h.t : tmax; hits.u[rid] = h.u; hits.v[rid] = h.v;
-            hits.patch[rid] = ob >= 0 ? h.patch : -1; hits.object[rid] = ob;
-        }
+        if (E.status[rid] == kPending) rest_ray<kAny>(S, rays, q, hits, occluded, rid, lc);
     }
     flush_counters(cnt, lc, 0);
 }
@@ -1152,16 +1203,18 @@ __global__ void __launch_bounds__(kPendingThreads) k_pending(const uint32_t* __r
     }
 }
 
+__device__ __forceinline__ void init_ray(const RaysSoA& rays, HitsSoA& hits, int32_t* occluded, const Eng& E, uint32_t i)
+{
+    E.count[i] = 0;
+    if (occluded) { occluded[i] = -1; return; }
+    hits.t[i] = rays.tmax ? rays.tmax[i] : INFINITY;
+    hits.u[i] = 0.0f; hits.v[i] = 0.0f; hits.patch[i] = -1; hits.object[i] = -1;
+}
 __global__ void k_init(RaysSoA rays, uint32_t n0, const uint32_t* nDev, HitsSoA hits, int32_t* occluded, Eng E)
 {
     const uint32_t n = nDev ? *nDev : n0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        E.count[i] = 0;
-        if (occluded) { occluded[i] = -1; continue; }
-        hits.t[i] = rays.tmax ? rays.tmax[i] : INFINITY;
-        hits.u[i] = 0.0f; hits.v[i] = 0.0f; hits.patch[i] = -1; hits.object[i] = -1;
-    }
+        init_ray(rays, hits, occluded, E, i);
 }
 
 // One polish per hit.  A warp gathers the hits of the rays it sweeps into a
@@ -1203,6 +1256,71 @@ __global__ void __launch_bounds__(kPolishThreads) k_polish(DevScene S, RaysSoA r
         }
     }
     if (lane < cnt) polish_ray(S, rays, hits, my[lane]);
+}
+
+// ------------------------------------------------------ small queries --
+// A whole query in one launch, for ray counts that leave no work to balance: a
+// warp takes an even share of the rays through every step -- the passes'
+// traversal, order and searches on counters and queues of its own, the inline
+// fallback, the polish -- so nothing is shared between warps.  A launch costs the
+// host about 6 us, and a query of separate kernels is 11 of them and two
+// memsets.  Each ray goes through the same steps, with the same results.
+template<bool kAny, bool kG64, bool kSub>
+__global__ void __launch_bounds__(32, 8) k_small(DevScene S, RaysSoA rays, uint32_t n0, const uint32_t* nDev,
+                                                              Eng E, int passes, int cache, Query q, HitsSoA hits,
+                                                              int32_t* occluded, Counters* cnt)
+{
+    __shared__ uint32_t ring[kRing * 32], fetch;
+    __shared__ Lend lend;
+    const uint32_t n = nDev ? *nDev : n0, lane = threadIdx.x;
+    const uint32_t share = (n + gridDim.x - 1) / gridDim.x, base = blockIdx.x * share;
+    if (base >= n) return;
+    const uint32_t mine = min(share, n - base);
+    LocalCounters lc;
+    uint32_t nrays = 0;
+    for (uint32_t i = lane; i < mine; i += 32) init_ray(rays, hits, kAny ? occluded : nullptr, E, base + i);
+    WarpSource src {&fetch, mine, base, nullptr};
+    for (int p = 0;; p++)
+    {
+        if (p > 0)
+        {
+            // the rays still parked, in ray order
+            uint32_t* queue = E.queue[p & 1] + base;
+            uint32_t m = 0;
+            for (uint32_t i0 = 0; i0 < mine; i0 += 32)
+            {
+                const uint32_t r = base + i0 + lane;
+                const bool parked = i0 + lane < mine && E.status[r] == kPending;
+                const unsigned b = __ballot_sync(0xFFFFFFFFu, parked);
+                if (parked) queue[m + __popc(b & ((1u << lane) - 1u))] = r;
+                m += __popc(b);
+            }
+            src.m = m;
+            src.queue = queue;
+            if (m == 0) break;
+        }
+        __syncwarp();
+        if (p == passes)
+        {
+            for (uint32_t i = lane; i < src.m; i += 32) rest_ray<kAny>(S, rays, q, hits, occluded, src.ray(i), lc);
+            break;
+        }
+        if (lane == 0) fetch = 0;
+        __syncwarp();
+        collect_rays<kAny, false, true>(S, rays, E, p, cache, src, ring, lc, nrays);
+        __syncwarp();
+        if (!kAny && S.leafKeys) order_rays(S, rays, E, src, lane, 32);
+        if (lane == 0) fetch = 0;
+        __syncwarp();
+        if constexpr (kSub) subdivide_rays<kAny>(S, rays, E, p, q, hits, occluded, src, lend, lc);
+        else clip_rays<kAny, kG64>(S, rays, E, p, q, hits, occluded, src, lend, lc);
+        __syncwarp();
+    }
+    __syncwarp();
+    if (!kAny && polishes(q.precision))
+        for (uint32_t i = lane; i < mine; i += 32)
+            if (hits.object[base + i] >= 0) polish_ray(S, rays, hits, base + i);
+    flush_counters(cnt, lc, nrays);
 }
 
 int sms()
@@ -1252,11 +1370,31 @@ void launch_collect(int grid, int threads, cudaStream_t stream, const DevScene& 
     k<<<grid, threads, 0, stream>>>(S, rays, n, nDev, E, pass, c.backtrackCache, cnt);
 }
 
+// Up to this many rays a query is one launch of k_small.  Closest hits, us a
+// query in one launch / in separate kernels: camera rays of a 16,384-patch torus
+// 92 / 229 at 32, 178 / 320 at 2,000, 273 / 365 at 16,000, 306 / 410 at 32,000,
+// 528 / 598 at 64,000, 721 / 689 at 120,000; scattered rays of a 60,000-patch
+// store 613 / 618 at 64,000; subdivision 552 / 658 at 32,000, 861 / 779 at 64,000.
+constexpr uint32_t kSmallRays = 65536, kSmallSubdivRays = 32768;
+
 template<bool kAny, bool kG64, bool kSub = false>
 void launch(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Query q, HitsSoA hits,
             int32_t* occluded, Eng E, Counters* cnt, cudaStream_t stream, int& nl)
 {
     const EngineConfig c = engine_config();
+    // a render's shadow queue is sized for a ray per sample and light and holds the ones that face it
+    const uint32_t small = (kSub ? kSmallSubdivRays : kSmallRays) * (kAny && nDev ? 2 : 1);
+    if (n <= small && !c.compressedNodes)
+    {
+        static const int warps = resident((const void*)k_small<kAny, kG64, kSub>, 32);
+        k_small<kAny, kG64, kSub><<<int(std::min<uint32_t>(n, uint32_t(warps))), 32, 0, stream>>>(
+            S, rays, n, nDev, E, c.passes, c.backtrackCache, q, hits, occluded, cnt);
+        nl++;
+        return;
+    }
+    cudaMemsetAsync(E.ctl, 0, sizeof(uint32_t) * 4 * (kMaxPasses + 1), stream);
+    k_init<<<sms() * 4, 256, 0, stream>>>(rays, n, nDev, hits, kAny ? occluded : nullptr, E);
+    nl++;
     const int ct = c.collectThreads, rt = c.resolveThreads;
     const int pc = per_sm<kAny, kG64, kSub>(true, ct, c.compressedNodes != 0);
     const int pr = per_sm<kAny, kG64, kSub>(false, rt);
@@ -1287,6 +1425,11 @@ void launch(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Q
     k_pending<<<gp, kPendingThreads, 0, stream>>>(E.status, n, nDev, E.queue[c.passes & 1], E.ctl + 4 * c.passes + 2);
     k_rest<kAny><<<sms() * 4, 128, 0, stream>>>(S, rays, E, c.passes, q, hits, occluded, cnt);
     nl += 2;
+    if (!kAny && polishes(q.precision))
+    {
+        k_polish<<<sms() * 8, kPolishThreads, 0, stream>>>(S, rays, n, nDev, hits);
+        nl++;
+    }
 }
 
 }  // namespace
@@ -1356,20 +1499,12 @@ cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_
         E.originLast = uint32_t(ec.originLast);
         E.subdivLevels = uint32_t(ec.subdivLevels);
     }
-    cudaMemsetAsync(E.ctl, 0, sizeof(uint32_t) * 4 * (kMaxPasses + 1), stream);
-    const int flat = sms() * 4;
-    k_init<<<flat, 256, 0, stream>>>(rays, n, nDev, hits, any ? occluded : nullptr, E);
-    int nl = 1;
+    int nl = 0;
     if (any) q.method != 0 ? launch<true, false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl)
                            : launch<true, false>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
     else if (q.method != 0) launch<false, false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
     else if (graze_sin(q.precision) > 0.0f) launch<false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
     else launch<false, false>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
-    if (!any && polishes(q.precision))
-    {
-        k_polish<<<flat * 2, kPolishThreads, 0, stream>>>(S, rays, n, nDev, hits);
-        nl++;
-    }
     if (launches) *launches += nl;
     return cudaGetLastError();
 }
