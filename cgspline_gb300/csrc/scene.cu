@@ -5,6 +5,7 @@
 #include <bit>
 #include <thread>
 #include <cmath>
+#include <memory>
 #include <numeric>
 #include <random>
 
@@ -148,50 +149,39 @@ void build_surface_bvh(const Surface& s, HostBVH& out)
     out.build(el);
 }
 
-// Scene::buildBVH (src/rt/Scene.cu:218-232) for one group: object bounds of
-// the transformed points (BezierSurface::bounds(M), src/rt/Primitive.cu:172-179),
-// centroid = box centre, element index = the global object id.
-void build_group_bvh(const cgs_scene* sc, const Group& g, HostBVH& out)
+// BezierSurface::bounds(M) (src/rt/Primitive.cu:172-179): the bounds of an
+// object's transformed points.
+Box object_bounds(const cgs_scene* sc, const Object& ob)
+{
+    const Surface& s = sc->surfaces[ob.surface];
+    const float* M = ob.l2w;
+    Box b;
+    for (uint32_t idx : s.indices)
+    {
+        const float* w = &s.points[4ull * idx];
+        float x = ((w[0] * M[0] + w[1] * M[4]) + w[2] * M[8]) + w[3] * M[12];
+        float y = ((w[0] * M[1] + w[1] * M[5]) + w[2] * M[9]) + w[3] * M[13];
+        float z = ((w[0] * M[2] + w[1] * M[6]) + w[2] * M[10]) + w[3] * M[14];
+        float ww = ((w[0] * M[3] + w[1] * M[7]) + w[2] * M[11]) + w[3] * M[15];
+        float p[3] = {x / ww, y / ww, z / ww};
+        b.inflate(p);
+    }
+    return b;
+}
+
+// Scene::buildBVH (src/rt/Scene.cu:218-232) for one group: centroid = box
+// centre, element index = the global object id; bounds: one box per object.
+void build_group_bvh(const Group& g, const std::vector<Box>& bounds, HostBVH& out)
 {
     std::vector<Element> el(g.objects.size());
     for (uint32_t i = 0; i < el.size(); i++)
     {
-        const Object& ob = sc->objects[g.objects[i]];
-        const Surface& s = sc->surfaces[ob.surface];
-        const float* M = ob.l2w;
-        Box b;
-        for (uint32_t idx : s.indices)
-        {
-            const float* w = &s.points[4ull * idx];
-            float x = ((w[0] * M[0] + w[1] * M[4]) + w[2] * M[8]) + w[3] * M[12];
-            float y = ((w[0] * M[1] + w[1] * M[5]) + w[2] * M[9]) + w[3] * M[13];
-            float z = ((w[0] * M[2] + w[1] * M[6]) + w[2] * M[10]) + w[3] * M[14];
-            float ww = ((w[0] * M[3] + w[1] * M[7]) + w[2] * M[11]) + w[3] * M[15];
-            float p[3] = {x / ww, y / ww, z / ww};
-            b.inflate(p);
-        }
+        const Box& b = bounds[g.objects[i]];
         el[i].index = g.objects[i];
         el[i].bounds = b;
         for (int k = 0; k < 3; k++) el[i].centroid[k] = 0.5f * (b.lo[k] + b.hi[k]);
     }
     out.build(el);
-}
-
-void pack_nodes(const HostBVH& b, std::vector<float4>& out)
-{
-    for (const Node& n : b.nodes)
-    {
-        const Box &L = n.leftBox, &R = n.rightBox;
-        float4 q0 = make_float4(L.lo[0], L.lo[1], L.lo[2], L.hi[0]);
-        float4 q1 = make_float4(L.hi[1], L.hi[2], R.lo[0], R.lo[1]);
-        float4 q2 = make_float4(R.lo[2], R.hi[0], R.hi[1], R.hi[2]);
-        float4 q3;
-        uint32_t l = n.left, r = n.right;
-        std::memcpy(&q3.x, &l, 4);
-        std::memcpy(&q3.y, &r, 4);
-        q3.z = 0.0f; q3.w = 0.0f;
-        out.push_back(q0); out.push_back(q1); out.push_back(q2); out.push_back(q3);
-    }
 }
 
 // ------------------------------------------------- compressed node mirror --
@@ -219,85 +209,118 @@ void pack_nodes(const HostBVH& b, std::vector<float4>& out)
 // coordinate, an extent no grid of 2^-126..2^127 covers, or a left child
 // that does not follow its parent, as a loaded blob may have) is read from
 // the exact records only.
-namespace {
-
 constexpr uint32_t kQLeaf = 1u;
 
-float round_down_float(double x)
+__device__ float round_down_float(double x)
 {
     float f = float(x);
-    if (double(f) > x) f = std::nextafter(f, -INFINITY);
+    if (double(f) > x) f = nextafterf(f, -INFINITY);
     return f;
 }
 
 // Grid of one axis of a node covering [lo, hi] with a two-step margin below
 // lo and at least two steps above hi inside 255 steps.  False if none.
-bool axis_grid(double lo, double hi, float& P, int& e)
+__device__ bool axis_grid(double lo, double hi, float& P, int& e)
 {
-    if (!std::isfinite(lo) || !std::isfinite(hi) || hi < lo) return false;
+    if (!isfinite(lo) || !isfinite(hi) || hi < lo) return false;
     // the smallest e with 250 s >= extent, from the binary exponent of
     // extent / 250 (then checked upward)
     const double extent = hi - lo;
-    int e0 = extent > 0.0 ? std::max(1, std::ilogb(extent / 250.0) + 127) : 1;
-    while (e0 < 254 && std::ldexp(250.0, e0 - 127) < extent) e0++;
+    int e0 = extent > 0.0 ? max(1, ilogb(extent / 250.0) + 127) : 1;
+    while (e0 < 254 && ldexp(250.0, e0 - 127) < extent) e0++;
     for (e = e0; e <= 254; e++)
     {
-        const double s = std::ldexp(1.0, e - 127);
+        const double s = ldexp(1.0, e - 127);
         P = round_down_float(lo - 2.0 * s);
-        if (!std::isfinite(P)) return false;
+        if (!isfinite(P)) return false;
         if ((hi - double(P)) / s <= 253.0) return true;
     }
     return false;
 }
 
-}  // namespace
+// One tree's nodes among a store's: [first, first + count), its records in the
+// compressed mirror from qbase on (EMPTY: it has none there), the BVH that they belong to.
+struct PackJob { uint32_t first, count, qbase, bvh; };
 
-// Appends the BVH's compressed records (two uint4 per node); false, with
-// zero records written for the failing node on, if a node has none.
-bool pack_qnodes(const HostBVH& b, std::vector<uint4>& out)
+// The node records of a store from the host trees' nodes: a thread per node,
+// all trees in one launch (their jobs in ascending order).  failed[bvh] is set
+// where a node has no compressed record.  Bound by the upload of its input;
+// packing on the host, one thread over 120,000 nodes, was most of the 8.4 ms that
+// the upload and hash build of a 30,000-patch store took (2.0 ms now).
+__global__ void k_pack_nodes(const Node* __restrict__ raw, const PackJob* __restrict__ jobs, uint32_t njobs, uint32_t total,
+                             float4* nodes, uint4* qnodes, uint32_t* failed)
 {
-    bool all = true;
-    for (size_t i = 0; i < b.nodes.size(); i++)
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
     {
-        const Node& n = b.nodes[i];
+        const Node n = raw[g];
+        const Box &L = n.leftBox, &R = n.rightBox;
+        float4* q = nodes + 4ull * g;
+        q[0] = make_float4(L.lo[0], L.lo[1], L.lo[2], L.hi[0]);
+        q[1] = make_float4(L.hi[1], L.hi[2], R.lo[0], R.lo[1]);
+        q[2] = make_float4(R.lo[2], R.hi[0], R.hi[1], R.hi[2]);
+        q[3] = make_float4(__uint_as_float(n.left), __uint_as_float(n.right), 0.0f, 0.0f);
+        uint32_t lo = 0, hi = njobs;
+        while (hi - lo > 1)
+        {
+            const uint32_t mid = (lo + hi) / 2;
+            if (jobs[mid].first <= g) lo = mid; else hi = mid;
+        }
+        const PackJob J = jobs[lo];
+        if (J.qbase == EMPTY) continue;
+        const uint32_t i = g - J.first;
         const bool leaf = n.left == EMPTY;
-        uint32_t w[8] = {};
         // the compressed record names only the right child: the left one must follow
         bool ok = leaf || n.left == i + 1;
-        uint32_t bytes[3] = {}, ex[3] = {};
+        uint32_t P[3] = {}, bytes[3] = {}, ex[3] = {};
         for (int a = 0; a < 3 && ok; a++)
         {
-            const Box& L = n.leftBox;
-            const Box& R = n.rightBox;
-            const double lo = leaf ? double(L.lo[a]) : std::min(double(L.lo[a]), double(R.lo[a]));
-            const double hi = leaf ? double(L.hi[a]) : std::max(double(L.hi[a]), double(R.hi[a]));
-            float P = 0;
+            const double blo = leaf ? double(L.lo[a]) : fmin(double(L.lo[a]), double(R.lo[a]));
+            const double bhi = leaf ? double(L.hi[a]) : fmax(double(L.hi[a]), double(R.hi[a]));
+            float p = 0;
             int e = 0;
-            if (!axis_grid(lo, hi, P, e)) { ok = false; break; }
-            const double s = std::ldexp(1.0, e - 127);
-            auto qlo = [&](double c) { return std::ceil((c - double(P)) / s) - 2.0; };
-            auto qhi = [&](double c) { return std::floor((c - double(P)) / s) + 2.0; };
-            const double q[4] = {qlo(L.lo[a]), qhi(L.hi[a]), leaf ? 0.0 : qlo(R.lo[a]), leaf ? 0.0 : qhi(R.hi[a])};
-            for (double v : q) if (!(v >= 0.0 && v <= 255.0)) ok = false;
-            if (!ok) break;
-            std::memcpy(&w[a], &P, 4);
+            if (!axis_grid(blo, bhi, p, e)) { ok = false; break; }
+            const double s = ldexp(1.0, e - 127), pd = double(p);
+            const double v[4] = {ceil((double(L.lo[a]) - pd) / s) - 2.0, floor((double(L.hi[a]) - pd) / s) + 2.0,
+                                 leaf ? 0.0 : ceil((double(R.lo[a]) - pd) / s) - 2.0,
+                                 leaf ? 0.0 : floor((double(R.hi[a]) - pd) / s) + 2.0};
+            for (int k = 0; k < 4; k++)
+            {
+                if (!(v[k] >= 0.0 && v[k] <= 255.0)) ok = false;
+                else bytes[a] |= uint32_t(v[k]) << (8 * k);
+            }
+            P[a] = __float_as_uint(p);
             ex[a] = uint32_t(e);
-            bytes[a] = uint32_t(q[0]) | (uint32_t(q[1]) << 8) | (uint32_t(q[2]) << 16) | (uint32_t(q[3]) << 24);
         }
         if (!ok)
         {
-            all = false;
-            w[0] = w[1] = w[2] = 0;
-            ex[0] = ex[1] = ex[2] = 127;
-            bytes[0] = bytes[1] = bytes[2] = 0;
+            failed[J.bvh] = 1u;
+            for (int a = 0; a < 3; a++) { P[a] = 0; ex[a] = 127; bytes[a] = 0; }
         }
-        w[3] = ex[0] | (ex[1] << 8) | (ex[2] << 16) | ((leaf ? kQLeaf : 0u) << 24);
-        w[4] = bytes[0]; w[5] = bytes[1]; w[6] = bytes[2];
-        w[7] = n.right;
-        out.push_back(make_uint4(w[0], w[1], w[2], w[3]));
-        out.push_back(make_uint4(w[4], w[5], w[6], w[7]));
+        uint4* w = qnodes + 2ull * (J.qbase + i);
+        w[0] = make_uint4(P[0], P[1], P[2], ex[0] | (ex[1] << 8) | (ex[2] << 16) | ((leaf ? kQLeaf : 0u) << 24));
+        w[1] = make_uint4(bytes[0], bytes[1], bytes[2], n.right);
     }
-    return all;
+}
+
+// De-indexed patches: 16 points each.
+__global__ void k_gather_patches(const float4* __restrict__ points, const uint32_t* __restrict__ index, size_t n,
+                                 float4* patches)
+{
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+        patches[i] = points[index[i]];
+}
+
+// Runs fn(0) .. fn(n - 1) on the host's cores, in any order; on this thread
+// alone where there is little to do.
+template<class F> void on_host_cores(size_t n, bool parallel, F&& fn)
+{
+    std::atomic<size_t> next {0};
+    auto worker = [&]() { for (size_t w; (w = next.fetch_add(1)) < n;) fn(w); };
+    const size_t nt = parallel ? std::min<size_t>(n, std::max(1u, std::min(64u, std::thread::hardware_concurrency()))) : 1;
+    std::vector<std::thread> pool;
+    for (size_t t = 1; t < nt; t++) pool.emplace_back(worker);
+    worker();
+    for (auto& th : pool) th.join();
 }
 
 // Lights of all groups, concatenated; groupLights[g] = (first, count);
@@ -382,37 +405,31 @@ void cgs::check_walk_bvh(Surface& s)
 // Device copy of the store's host state (everything but the hash tables).
 int cgs::upload_store(cgs_scene* sc)
 {
-    const uint32_t nb = sc->nbvh();
-    std::vector<float4> hp, hn;
-    std::vector<uint4> hq;
-    std::vector<uint32_t> hi, pbase, pmat, gtop, lkeys;
+    const uint32_t nb = sc->nbvh(), ns = uint32_t(sc->surfaces.size());
+    std::vector<uint32_t> pbase, pmat, gtop;
     std::vector<DevMaterial> hm;
     std::vector<DevObject> ho;
+    std::vector<PackJob> jobs;
     sc->hbvh.assign(nb, DevBVH {});
-    sc->walkTrees = false;
     sc->tableCap.assign(nb, 0);
-    uint32_t patchCursor = 0, tableCursor = 0, dispCursor = 0;
+    sc->walkTrees = false;
+    uint32_t tableCursor = 0, dispCursor = 0, nodeCursor = 0, indexCursor = 0, qCursor = 0;
     for (uint32_t k = 0; k < nb; k++)
     {
         const HostBVH& b = sc->bvh(k);
         DevBVH& d = sc->hbvh[k];
-        d.nodeBase = uint32_t(hn.size() / 4);
-        d.indexBase = uint32_t(hi.size());
-        d.qnodeBase = uint32_t(hq.size() / 2);
-        d.walkBase = EMPTY;
-        pack_nodes(b, hn);
-        if (k < sc->surfaces.size() && !sc->surfaces[k].walk.nodes.empty())
-        {
-            const HostBVH& w = sc->surfaces[k].walk;
-            d.walkBase = uint32_t(hn.size() / 4);
-            pack_nodes(w, hn);
-            d.compressed = pack_qnodes(w, hq) ? 1u : 0u;
-            sc->walkTrees = true;
-        }
-        else
-            d.compressed = pack_qnodes(b, hq) ? 1u : 0u;
-        hi.insert(hi.end(), b.indices.begin(), b.indices.end());
-        uint32_t n = uint32_t(b.keys.size());
+        const uint32_t n = uint32_t(b.nodes.size());
+        const bool walk = k < ns && !sc->surfaces[k].walk.nodes.empty();
+        d.nodeBase = nodeCursor;
+        d.indexBase = indexCursor;
+        d.qnodeBase = qCursor;
+        d.walkBase = walk ? nodeCursor + n : EMPTY;
+        jobs.push_back({nodeCursor, n, walk ? EMPTY : qCursor, k});
+        if (walk) jobs.push_back({nodeCursor + n, n, qCursor, k});
+        nodeCursor += walk ? 2 * n : n;
+        qCursor += n;
+        indexCursor += uint32_t(b.indices.size());
+        sc->walkTrees = sc->walkTrees || walk;
         d.tableBase = tableCursor;
         d.dispBase = dispCursor;
         sc->tableCap[k] = table_capacity(n);
@@ -422,26 +439,18 @@ int cgs::upload_store(cgs_scene* sc)
         d.N = n; d.A = 31; d.B = 19;
         d.Nmagic = fastmod_magic(std::max<uint32_t>(n, 1));
     }
-    for (uint32_t g = 0; g < sc->groups.size(); g++) gtop.push_back(uint32_t(sc->surfaces.size()) + g);
+    for (uint32_t g = 0; g < sc->groups.size(); g++) gtop.push_back(ns + g);
+    std::vector<size_t> pointBase;
+    size_t points = 0;
+    uint32_t patches = 0;
     for (const Surface& s : sc->surfaces)
     {
-        pbase.push_back(patchCursor);
-        for (uint32_t p = 0; p < s.patchCount(); p++)
-            for (int j = 0; j < 16; j++)
-            {
-                const float* w = &s.points[4ull * s.indices[16ull * p + j]];
-                hp.push_back(make_float4(w[0], w[1], w[2], w[3]));
-            }
-        if (sc->walkTrees)
-        {
-            lkeys.resize(size_t(patchCursor) + s.patchCount(), 0);
-            if (!s.walk.nodes.empty())
-                for (size_t i = 0; i < s.bvh.nodes.size(); i++)
-                    if (s.bvh.nodes[i].left == EMPTY)
-                        lkeys[patchCursor + s.bvh.indices[s.bvh.nodes[i].right]] = s.bvh.keys[i];
-        }
-        patchCursor += s.patchCount();
+        pbase.push_back(patches);
+        pointBase.push_back(points);
+        patches += s.patchCount();
+        points += s.points.size() / 4;
     }
+    if (points > 0xFFFFFFFFull) return CGS_ERR_INVALID_ARGUMENT;
     for (const Object& ob : sc->objects)
     {
         DevObject d {};
@@ -460,10 +469,46 @@ int cgs::upload_store(cgs_scene* sc)
             d.patchMaterialBase = -1;
         ho.push_back(d);
     }
-    CGS_TRY(sc->patches.reserve(hp.size()));
-    CGS_TRY(sc->nodes.reserve(hn.size()));
-    CGS_TRY(sc->qnodes.reserve(hq.size()));
-    CGS_TRY(sc->indices.reserve(hi.size()));
+    // The host trees and control points as they are, in one staging area: nodes,
+    // points, point indices, leaf lists, leaf keys.  Each surface and group is
+    // copied into its places by one of the host's cores; the device makes its
+    // records from them (k_pack_nodes, k_gather_patches).
+    auto place = [cursor = size_t(0)](size_t bytes) mutable {
+        const size_t at = cursor;
+        cursor = (cursor + bytes + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t oPoints = place(points * sizeof(float4)), oIndex = place(size_t(patches) * 64),
+                 oNodes = place(size_t(nodeCursor) * sizeof(Node)), oJobs = place(jobs.size() * sizeof(PackJob)),
+                 oFailed = place(nb * sizeof(uint32_t)), raw = place(0), oList = place(size_t(indexCursor) * 4),
+                 oKeys = place(sc->walkTrees ? size_t(patches) * 4 : 0), total = place(0);
+    std::unique_ptr<uint8_t[]> stage(new (std::nothrow) uint8_t[std::max<size_t>(total, 1)]);
+    if (!stage) return CGS_ERR_OUT_OF_MEMORY;
+    uint8_t* h = stage.get();
+    std::memcpy(h + oJobs, jobs.data(), jobs.size() * sizeof(PackJob));
+    std::memset(h + oFailed, 0, nb * sizeof(uint32_t));
+    on_host_cores(nb, total > (1u << 20), [&](size_t k) {
+        const HostBVH& b = sc->bvh(uint32_t(k));
+        const DevBVH& d = sc->hbvh[k];
+        Node* nodes = reinterpret_cast<Node*>(h + oNodes);
+        std::copy(b.nodes.begin(), b.nodes.end(), nodes + d.nodeBase);
+        std::copy(b.indices.begin(), b.indices.end(), reinterpret_cast<uint32_t*>(h + oList) + d.indexBase);
+        if (k >= ns) return;
+        const Surface& s = sc->surfaces[k];
+        std::memcpy(h + oPoints + pointBase[k] * sizeof(float4), s.points.data(), s.points.size() * sizeof(float));
+        uint32_t* index = reinterpret_cast<uint32_t*>(h + oIndex) + size_t(pbase[k]) * 16;
+        for (size_t i = 0; i < s.indices.size(); i++) index[i] = uint32_t(pointBase[k]) + s.indices[i];
+        if (!sc->walkTrees) return;
+        uint32_t* keys = reinterpret_cast<uint32_t*>(h + oKeys) + pbase[k];
+        if (d.walkBase == EMPTY) { std::fill(keys, keys + s.patchCount(), 0u); return; }
+        std::copy(s.walk.nodes.begin(), s.walk.nodes.end(), nodes + d.walkBase);
+        for (size_t i = 0; i < b.nodes.size(); i++)
+            if (b.nodes[i].left == EMPTY) keys[b.indices[b.nodes[i].right]] = b.keys[i];
+    });
+    CGS_TRY(sc->patches.reserve(size_t(patches) * 16));
+    CGS_TRY(sc->nodes.reserve(4ull * nodeCursor));
+    CGS_TRY(sc->qnodes.reserve(2ull * qCursor));
+    CGS_TRY(sc->indices.reserve(indexCursor));
     CGS_TRY(sc->tables.reserve(tableCursor));
     CGS_TRY(sc->disps.reserve(dispCursor));
     CGS_TRY(sc->patchBase.reserve(pbase.size()));
@@ -473,21 +518,33 @@ int cgs::upload_store(cgs_scene* sc)
     CGS_TRY(sc->dobjects.reserve(ho.size()));
     CGS_TRY(sc->materials.reserve(hm.size()));
     CGS_TRY(sc->counters.reserve(1));
-    if (sc->walkTrees)
+    if (sc->walkTrees) CGS_TRY(sc->leafKeys.reserve(patches));
+    struct Temp
     {
-        CGS_TRY(sc->leafKeys.reserve(lkeys.size()));
-        CGS_TRY(cudaMemcpy(sc->leafKeys.p, lkeys.data(), lkeys.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    }
-    CGS_TRY(cudaMemcpy(sc->patches.p, hp.data(), hp.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    CGS_TRY(cudaMemcpy(sc->nodes.p, hn.data(), hn.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    CGS_TRY(cudaMemcpy(sc->qnodes.p, hq.data(), hq.size() * sizeof(uint4), cudaMemcpyHostToDevice));
-    CGS_TRY(cudaMemcpy(sc->indices.p, hi.data(), hi.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+        DBuf<uint8_t> b;
+        ~Temp() { b.release(); }
+    } temp;
+    CGS_TRY(temp.b.reserve(raw));
+    uint8_t* dv = temp.b.p;
+    CGS_TRY(cudaMemcpy(dv, h, raw, cudaMemcpyHostToDevice));
+    const uint32_t blocks = 1216;
+    k_gather_patches<<<blocks, 256>>>(reinterpret_cast<const float4*>(dv + oPoints),
+                                      reinterpret_cast<const uint32_t*>(dv + oIndex), size_t(patches) * 16, sc->patches.p);
+    k_pack_nodes<<<blocks, 128>>>(reinterpret_cast<const Node*>(dv + oNodes), reinterpret_cast<const PackJob*>(dv + oJobs),
+                                  uint32_t(jobs.size()), nodeCursor, sc->nodes.p, sc->qnodes.p,
+                                  reinterpret_cast<uint32_t*>(dv + oFailed));
+    CGS_TRY(cudaGetLastError());
+    CGS_TRY(cudaMemcpy(sc->indices.p, h + oList, size_t(indexCursor) * 4, cudaMemcpyHostToDevice));
+    if (sc->walkTrees) CGS_TRY(cudaMemcpy(sc->leafKeys.p, h + oKeys, size_t(patches) * 4, cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->patchBase.p, pbase.data(), pbase.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     if (!pmat.empty())
         CGS_TRY(cudaMemcpy(sc->patchMaterial.p, pmat.data(), pmat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->dobjects.p, ho.data(), ho.size() * sizeof(DevObject), cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->materials.p, hm.data(), hm.size() * sizeof(DevMaterial), cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->groupTop.p, gtop.data(), gtop.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    std::vector<uint32_t> failed(nb);
+    CGS_TRY(cudaMemcpy(failed.data(), dv + oFailed, nb * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    for (uint32_t k = 0; k < nb; k++) sc->hbvh[k].compressed = failed[k] ? 0u : 1u;
     CGS_TRY(cudaMemcpy(sc->bvhs.p, sc->hbvh.data(), nb * sizeof(DevBVH), cudaMemcpyHostToDevice));
     int r = upload_lights(sc);
     if (r) return r;
@@ -632,7 +689,12 @@ int mirror_export(const cgs_scene* s, uint32_t k, HostBVH& ref, std::vector<uint
     const size_t ns = s->surfaces.size();
     ref.split_mode = CGS_SPLIT_REFERENCE;
     if (k < ns) build_surface_bvh(s->surfaces[k], ref);
-    else build_group_bvh(s, s->groups[k - ns], ref);
+    else
+    {
+        std::vector<Box> bounds(s->objects.size());
+        for (uint32_t o : s->groups[k - ns].objects) bounds[o] = object_bounds(s, s->objects[o]);
+        build_group_bvh(s->groups[k - ns], bounds, ref);
+    }
     if (ref.emptyLeaf) return CGS_ERR_EMPTY_LEAF;
     params[0] = params[1] = params[2] = params[3] = 0;
     table.clear();
@@ -859,50 +921,41 @@ int cgs_bvh_build(cgs_scene* s)
     if (s->objects.empty()) return CGS_ERR_INVALID_ARGUMENT;
     for (const Group& gr : s->groups)
         if (gr.objects.empty()) return CGS_ERR_EMPTY_LEAF;
-    // the surfaces' and groups' BVHs are independent: built on all host
-    // cores, largest first, each by one thread (the same result as in order)
-    const size_t ns = s->surfaces.size(), ng = s->groups.size();
-    std::vector<std::pair<uint64_t, size_t>> work;
+    // the surfaces' BVHs and walk trees and the objects' bounds are independent:
+    // built on all host cores, largest first, each by one thread (the same
+    // result as in order); then the groups' BVHs over the bounds
+    const size_t ns = s->surfaces.size(), no = s->objects.size(), ng = s->groups.size();
     const bool walk = s->splitMode == CGS_SPLIT_REFERENCE;
+    // a mirrored store traverses the longest-axis build
+    const int mode = s->splitMode == CGS_SPLIT_MIRROR ? CGS_SPLIT_LONGEST : s->splitMode;
+    std::vector<std::pair<uint64_t, size_t>> work;
+    uint64_t all = 0;
     for (size_t i = 0; i < ns; i++)
     {
-        work.push_back({s->surfaces[i].patchCount(), i});
-        if (walk) work.push_back({s->surfaces[i].patchCount(), ns + ng + i});
+        const uint64_t cost = 4ull * s->surfaces[i].patchCount();
+        work.push_back({cost, i});
+        if (walk) work.push_back({cost, ns + i});
         s->surfaces[i].walk = HostBVH {};
+        all += cost;
     }
-    for (size_t g = 0; g < ng; g++)
-    {
-        uint64_t cost = 0;
-        for (uint32_t o : s->groups[g].objects) cost += s->surfaces[s->objects[o].surface].indices.size() / 16;
-        work.push_back({cost, ns + g});
-    }
+    for (size_t o = 0; o < no; o++)
+        work.push_back({s->surfaces[s->objects[o].surface].patchCount(), 2 * ns + o});
     std::sort(work.begin(), work.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-    std::atomic<size_t> next {0};
-    auto worker = [&]() {
-        for (size_t w; (w = next.fetch_add(1)) < work.size();)
+    std::vector<Box> bounds(no);
+    on_host_cores(work.size(), all > 1000, [&](size_t w) {
+        const size_t i = work[w].second;
+        if (i < ns)
         {
-            const size_t i = work[w].second;
-            // a mirrored store traverses the longest-axis build
-            const int mode = s->splitMode == CGS_SPLIT_MIRROR ? CGS_SPLIT_LONGEST : s->splitMode;
-            if (i < ns)
-            {
-                s->surfaces[i].bvh.split_mode = mode;
-                build_surface_bvh(s->surfaces[i], s->surfaces[i].bvh);
-            }
-            else if (i >= ns + ng)
-                build_walk_bvh(s->surfaces[i - ns - ng], s->surfaces[i - ns - ng].walk);
-            else
-            {
-                s->groups[i - ns].top.split_mode = mode;
-                build_group_bvh(s, s->groups[i - ns], s->groups[i - ns].top);
-            }
+            s->surfaces[i].bvh.split_mode = mode;
+            build_surface_bvh(s->surfaces[i], s->surfaces[i].bvh);
         }
-    };
-    const size_t nt = std::min<size_t>(work.size(), std::max(1u, std::min(64u, std::thread::hardware_concurrency())));
-    std::vector<std::thread> pool;
-    for (size_t t = 1; t < nt; t++) pool.emplace_back(worker);
-    worker();
-    for (auto& th : pool) th.join();
+        else if (i < 2 * ns) build_walk_bvh(s->surfaces[i - ns], s->surfaces[i - ns].walk);
+        else bounds[i - 2 * ns] = object_bounds(s, s->objects[i - 2 * ns]);
+    });
+    on_host_cores(ng, ng > 64, [&](size_t g) {
+        s->groups[g].top.split_mode = mode;
+        build_group_bvh(s->groups[g], bounds, s->groups[g].top);
+    });
     for (auto& sf : s->surfaces)
         if (sf.bvh.emptyLeaf) return CGS_ERR_EMPTY_LEAF;
     for (auto& gr : s->groups)
