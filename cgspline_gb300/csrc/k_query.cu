@@ -1,7 +1,6 @@
-// k_query.cu -- per-thread query kernels: spline::doBezierClipping /
-// doSubdivision on explicit (ray, patch) pairs (src/Spline.h:488-508), the
-// plain one-thread-per-ray scene query, and the gather / scatter of the ray
-// arrays of several query requests into one batch.
+// k_query.cu -- per-thread query kernels: the plain one-thread-per-ray scene
+// query, the surface normals, and the gather / scatter of the ray arrays of
+// several query requests into one batch.
 #include <algorithm>
 
 #include "kernels.h"
@@ -9,32 +8,6 @@
 namespace cgs {
 
 namespace {
-
-constexpr int kPairThreads = 128;
-
-__global__ void __launch_bounds__(kPairThreads) k_patch_pairs(DevScene S, uint32_t surface, uint32_t patches,
-                                                              RaysSoA rays, const uint32_t* __restrict__ pids,
-                                                              uint32_t n, Query q, HitsSoA hits, Counters* cnt)
-{
-    LocalCounters lc;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && __ldg(pids + i) >= patches)
-    {
-        hits.patch[i] = 0;
-        lc.errors |= kErrPatchId;
-    }
-    else if (i < n)
-    {
-        const float3 o = f3(__ldg(rays.ox + i), __ldg(rays.oy + i), __ldg(rays.oz + i));
-        const float3 d = f3(__ldg(rays.dx + i), __ldg(rays.dy + i), __ldg(rays.dz + i));
-        const float4* P = S.patches + 16ull * (__ldg(S.patchBase + surface) + __ldg(pids + i));
-        HitSink sink {P, o, d, hits.t[i], make_float2(0.0f, 0.0f)};
-        const bool b = search_patch(sink, q, lc);
-        if (b) { hits.t[i] = sink.dist; hits.u[i] = sink.uv.x; hits.v[i] = sink.uv.y; }
-        hits.patch[i] = b ? 1 : 0;
-    }
-    flush_counters(cnt, lc, i < n ? 1u : 0u);
-}
 
 // One thread per ray, the whole search inline (the reference's per-ray
 // kernel shape, src/rt/RayTracer.cu:171-274): the plain query path.
@@ -139,16 +112,6 @@ cudaError_t launch_scatter_hits(const QueryChunk* table, const uint32_t* hdr, ui
     if (cap == 0) return cudaSuccess;
     const uint32_t blocks = std::min<uint32_t>((cap + 255) / 256, 4096u);
     k_scatter_hits<<<blocks, 256, 0, stream>>>(table, hdr, hits, any);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_patch_pairs(const DevScene& S, uint32_t surface, uint32_t patches, RaysSoA rays,
-                               const uint32_t* patch_ids, uint32_t n, Query q, HitsSoA hits, Counters* counters,
-                               cudaStream_t stream)
-{
-    if (n == 0) return cudaSuccess;
-    k_patch_pairs<<<(n + kPairThreads - 1) / kPairThreads, kPairThreads, 0, stream>>>(S, surface, patches, rays,
-                                                                                      patch_ids, n, q, hits, counters);
     return cudaGetLastError();
 }
 

@@ -14,7 +14,8 @@ struct RaysSoA { const float *ox, *oy, *oz, *dx, *dy, *dz, *tmax; const uint32_t
 struct HitsSoA { float *t, *u, *v; int32_t *patch, *object; };
 
 // ---------------------------------------------------------- ray queries --
-// spline::doBezierClipping on explicit (ray, patch) pairs, one thread per pair;
+// spline::doBezierClipping / doSubdivision on explicit (ray, patch) pairs
+// (src/Spline.h:488-508, k_engine.cu);
 // a patch id at or past `patches` (the surface's count) is a miss and raises
 // error bit kErrPatchId.
 cudaError_t launch_patch_pairs(const DevScene& S, uint32_t surface, uint32_t patches, RaysSoA rays,
