@@ -1208,9 +1208,10 @@ __device__ __forceinline__ void surface_d(const float4* __restrict__ P, double U
 #pragma unroll
         for (int i = 0; i < 4; i++)
         {
-            const float4 q = __ldg(P + 4 * j + i);
-            r[0] += wu[i] * q.x; r[1] += wu[i] * q.y; r[2] += wu[i] * q.z; r[3] += wu[i] * q.w;
-            ru[0] += du[i] * q.x; ru[1] += du[i] * q.y; ru[2] += du[i] * q.z; ru[3] += du[i] * q.w;
+            const float4 f = __ldg(P + 4 * j + i);
+            const double q[4] = {widen(f.x), widen(f.y), widen(f.z), widen(f.w)};
+#pragma unroll
+            for (int k = 0; k < 4; k++) { r[k] += wu[i] * q[k]; ru[k] += du[i] * q[k]; }
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) { H[k] += wv[j] * r[k]; Hu[k] += wv[j] * ru[k]; Hv[k] += dv[j] * r[k]; }
@@ -1221,86 +1222,116 @@ __device__ __forceinline__ void surface_d(const float4* __restrict__ P, double U
     Sv = make_double3((Hv[0] - Hv[3] * Sp.x) * iw, (Hv[1] - Hv[3] * Sp.y) * iw, (Hv[2] - Hv[3] * Sp.z) * iw);
 }
 
-static __device__ __noinline__ bool newton_polish64(const float4* __restrict__ P, double3 o, double3 d, double& t,
-                                                    double& u, double& v)
+// A polish in parts, so that a warp can interleave those of its lanes: the
+// start, mixed-precision steps and, for the few that they leave, full FP64 steps.
+struct Polish
 {
-    double U = u, V = v, T = t;
-    const float3 df = f3(float(d.x), float(d.y), float(d.z));
-    bool converged = false;
-    for (int it = 0; it < kPolishSteps; it++)
-    {
-        double wu[4], wv[4];
-        basis_d(U, wu);
-        basis_d(V, wv);
-        double S[4] = {0, 0, 0, 0};
+    const float4* P;
+    double3 o, d;       // the ray in the object's space
+    double U, V, T;
+    double u, v, t;     // the start
+    int it;
+    bool affine;        // all of the net's weights are 1
+};
+enum PolishNext : int { kPolishStep, kPolishStep64, kPolishDone, kPolishFailed };
+
+__device__ __forceinline__ void polish_begin(Polish& p, const float4* __restrict__ P, double3 o, double3 d, double t,
+                                             double u, double v)
+{
+    p.P = P; p.o = o; p.d = d;
+    p.U = p.u = u; p.V = p.v = v; p.T = p.t = t;
+    p.it = 0;
+    p.affine = true;
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-        {
-            double r[4] = {0, 0, 0, 0};
+    for (int i = 0; i < 16; i++) p.affine = p.affine && __ldg(P + i).w == 1.0f;
+}
+
+__device__ __forceinline__ PolishNext polish_step(Polish& p)
+{
+    const float4* __restrict__ P = p.P;
+    double wu[4], wv[4];
+    basis_d(p.U, wu);
+    basis_d(p.V, wv);
+    double S[4] = {0, 0, 0, 0};
+    double w1 = 0.0;  // a row's weight where all of the net's are 1: the same sum for every row
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-            {
-                const float4 q = __ldg(P + 4 * j + i);
-                r[0] += wu[i] * q.x; r[1] += wu[i] * q.y; r[2] += wu[i] * q.z; r[3] += wu[i] * q.w;
-            }
-            S[0] += wv[j] * r[0]; S[1] += wv[j] * r[1]; S[2] += wv[j] * r[2]; S[3] += wv[j] * r[3];
-        }
-        const double iw = 1.0 / S[3];
-        const double px = S[0] * iw, py = S[1] * iw, pz = S[2] * iw;
-        const float fx = float(px - (o.x + T * d.x)), fy = float(py - (o.y + T * d.y)), fz = float(pz - (o.z + T * d.z));
-        // FP32 Jacobian of the projected surface at (U, V)
-        const float uf = float(U), vf = float(V);
-        const float4 Hu = tensor_eval(P, dbasis(uf), basis(vf));
-        const float4 Hv = tensor_eval(P, basis(uf), dbasis(vf));
-        const float4 H = tensor_eval(P, basis(uf), basis(vf));
-        const float ih = 1.0f / H.w;
-        const float3 Pf = f3(H.x * ih, H.y * ih, H.z * ih);
-        const float3 Su = (xyz(Hu) - Hu.w * Pf) * ih, Sv = (xyz(Hv) - Hv.w * Pf) * ih;
-        const float3 c = -df;
-        const float3 svxc = cross(Sv, c);
-        const float det = dot(Su, svxc);
-        if (!(fabsf(det) > 1e-30f)) break;
-        const float3 mF = f3(-fx, -fy, -fz);
-        const float idet = 1.0f / det;
-        const double dU = double(dot(mF, svxc) * idet);
-        const double dV = double(dot(Su, cross(mF, c)) * idet);
-        const double dT = double(dot(Su, cross(Sv, mF)) * idet);
-        U += dU; V += dV; T += dT;
-        if (!isfinite(U + V + T)) { U = u; V = v; T = t; break; }
-        // the last step bounds the error of the previous iterate and contracts
-        // by ~1e-7 x the Jacobian's condition: below 1e-9 the result is FP32-exact
-        if (fabs(dT) <= 1e-9 * fabs(T) && fabs(dU) + fabs(dV) <= 1e-9) { converged = true; break; }
-        // a small step on a well-conditioned system: the next would only confirm it
-        if (fabs(dT) <= kPolishAccept * fabs(T) && fabs(dU) + fabs(dV) <= kPolishAccept &&
-            fabsf(det) >= kPolishMinSin * len(Su) * len(Sv))
-        {
-            converged = true;
-            break;
-        }
-    }
-    if (!converged)
+    for (int i = 0; i < 4; i++) w1 += wu[i];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
     {
-        // the oracle's polish: FP64 Jacobian and solve
-        const double3 c = make_double3(-d.x, -d.y, -d.z);
-        for (int it = 0; it < kPolishSteps64; it++)
+        double r[4] = {0, 0, 0, w1};
+        if (!p.affine) r[3] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
         {
-            double3 Sp, Su, Sv;
-            surface_d(P, U, V, Sp, Su, Sv);
-            const double3 mF = make_double3(o.x + T * d.x - Sp.x, o.y + T * d.y - Sp.y, o.z + T * d.z - Sp.z);
-            const double3 svxc = cross_d(Sv, c);
-            const double det = dot_d(Su, svxc);
-            if (!(fabs(det) > 1e-300)) return false;
-            const double dU = dot_d(mF, svxc) / det;
-            const double dV = dot_d(Su, cross_d(mF, c)) / det;
-            const double dT = dot_d(Su, cross_d(Sv, mF)) / det;
-            U += dU; V += dV; T += dT;
-            if (!isfinite(U + V + T)) return false;
-            if (fabs(dU) + fabs(dV) < 1e-15 && fabs(dT) < 1e-15 * fabs(T)) { converged = true; break; }
+            const float4 q = __ldg(P + 4 * j + i);
+            r[0] += wu[i] * widen(q.x); r[1] += wu[i] * widen(q.y); r[2] += wu[i] * widen(q.z);
+            if (!p.affine) r[3] += wu[i] * widen(q.w);
         }
+        S[0] += wv[j] * r[0]; S[1] += wv[j] * r[1]; S[2] += wv[j] * r[2]; S[3] += wv[j] * r[3];
     }
-    if (U < -1e-6 || U > 1.0 + 1e-6 || V < -1e-6 || V > 1.0 + 1e-6 || T <= 0.0) return false;
-    t = T; u = U; v = V;
-    return true;
+    const double iw = quotient(1.0, S[3]);
+    const double px = S[0] * iw, py = S[1] * iw, pz = S[2] * iw;
+    const float fx = narrow(px - (p.o.x + p.T * p.d.x)), fy = narrow(py - (p.o.y + p.T * p.d.y)),
+                fz = narrow(pz - (p.o.z + p.T * p.d.z));
+    // FP32 Jacobian of the projected surface at (U, V)
+    const float uf = narrow(p.U), vf = narrow(p.V);
+    const float4 Hu = tensor_eval(P, dbasis(uf), basis(vf));
+    const float4 Hv = tensor_eval(P, basis(uf), dbasis(vf));
+    const float4 H = tensor_eval(P, basis(uf), basis(vf));
+    const float ih = 1.0f / H.w;
+    const float3 Pf = f3(H.x * ih, H.y * ih, H.z * ih);
+    const float3 Su = (xyz(Hu) - Hu.w * Pf) * ih, Sv = (xyz(Hv) - Hv.w * Pf) * ih;
+    const float3 c = -f3(narrow(p.d.x), narrow(p.d.y), narrow(p.d.z));
+    const float3 svxc = cross(Sv, c);
+    const float det = dot(Su, svxc);
+    const bool last = ++p.it >= kPolishSteps;
+    if (!(fabsf(det) > 1e-30f)) { p.it = 0; return kPolishStep64; }
+    const float3 mF = f3(-fx, -fy, -fz);
+    const float idet = 1.0f / det;
+    const double dU = widen(dot(mF, svxc) * idet);
+    const double dV = widen(dot(Su, cross(mF, c)) * idet);
+    const double dT = widen(dot(Su, cross(Sv, mF)) * idet);
+    p.U += dU; p.V += dV; p.T += dT;
+    if (!isfinite(p.U + p.V + p.T))
+    {
+        p.U = p.u; p.V = p.v; p.T = p.t;
+        p.it = 0;
+        return kPolishStep64;
+    }
+    // the last step bounds the error of the previous iterate and contracts
+    // by ~1e-7 x the Jacobian's condition: below 1e-9 the result is FP32-exact
+    if (fabs(dT) <= 1e-9 * fabs(p.T) && fabs(dU) + fabs(dV) <= 1e-9) return kPolishDone;
+    // a small step on a well-conditioned system: the next would only confirm it
+    if (fabs(dT) <= kPolishAccept * fabs(p.T) && fabs(dU) + fabs(dV) <= kPolishAccept &&
+        fabsf(det) >= kPolishMinSin * len(Su) * len(Sv))
+        return kPolishDone;
+    if (last) p.it = 0;
+    return last ? kPolishStep64 : kPolishStep;
+}
+
+// the oracle's polish: FP64 Jacobian and solve
+__device__ __forceinline__ PolishNext polish_step64(Polish& p)
+{
+    const double3 c = make_double3(-p.d.x, -p.d.y, -p.d.z);
+    double3 Sp, Su, Sv;
+    surface_d(p.P, p.U, p.V, Sp, Su, Sv);
+    const double3 mF = make_double3(p.o.x + p.T * p.d.x - Sp.x, p.o.y + p.T * p.d.y - Sp.y, p.o.z + p.T * p.d.z - Sp.z);
+    const double3 svxc = cross_d(Sv, c);
+    const double det = dot_d(Su, svxc);
+    if (!(fabs(det) > 1e-300)) return kPolishFailed;
+    const double dU = dot_d(mF, svxc) / det;
+    const double dV = dot_d(Su, cross_d(mF, c)) / det;
+    const double dT = dot_d(Su, cross_d(Sv, mF)) / det;
+    p.U += dU; p.V += dV; p.T += dT;
+    if (!isfinite(p.U + p.V + p.T)) return kPolishFailed;
+    if (fabs(dU) + fabs(dV) < 1e-15 && fabs(dT) < 1e-15 * fabs(p.T)) return kPolishDone;
+    return ++p.it >= kPolishSteps64 ? kPolishDone : kPolishStep64;
+}
+
+__device__ __forceinline__ bool polish_accepted(const Polish& p)
+{
+    return !(p.U < -1e-6 || p.U > 1.0 + 1e-6 || p.V < -1e-6 || p.V > 1.0 + 1e-6 || p.T <= 0.0);
 }
 
 // ----------------------------------------------------------- traversal --
@@ -1479,26 +1510,44 @@ __device__ __forceinline__ bool search_patch(HitSink& sink, const Query& q, Loca
 }
 
 // FP64 Newton polish of a world-space hit, done in the object's space.
-__device__ __forceinline__ void polish_hit(const DevScene& S, float3 o, float3 d, HitRecord& hit)
+// isc: 1 / the object-space length of the world direction.
+__device__ __forceinline__ void polish_start(const DevScene& S, float3 o, float3 d, const HitRecord& hit, Polish& p,
+                                             double& isc)
 {
     const DevObject& ob = S.objects[hit.object];
     const float4* P = S.patches + 16ull * (__ldg(S.patchBase + ob.surface) + uint32_t(hit.patch));
-    const float* m = ob.w2l;
-    double ox = o.x, oy = o.y, oz = o.z, dx = d.x, dy = d.y, dz = d.z;
+    const float* f = ob.w2l;
+    double m[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) m[k] = widen(f[k]);
+    const double ox = widen(o.x), oy = widen(o.y), oz = widen(o.z), dx = widen(d.x), dy = widen(d.y), dz = widen(d.z);
     double3 lo = make_double3(ox * m[0] + oy * m[4] + oz * m[8] + m[12], ox * m[1] + oy * m[5] + oz * m[9] + m[13],
                               ox * m[2] + oy * m[6] + oz * m[10] + m[14]);
     // an affine world-to-object matrix (the usual case) has w = 1: no division
-    if (!(m[3] == 0.0f && m[7] == 0.0f && m[11] == 0.0f && m[15] == 1.0f))
+    if (!(f[3] == 0.0f && f[7] == 0.0f && f[11] == 0.0f && f[15] == 1.0f))
     {
         const double lw = ox * m[3] + oy * m[7] + oz * m[11] + m[15];
         lo = make_double3(lo.x / lw, lo.y / lw, lo.z / lw);
     }
     double3 ld = make_double3(dx * m[0] + dy * m[4] + dz * m[8], dx * m[1] + dy * m[5] + dz * m[9],
                               dx * m[2] + dy * m[6] + dz * m[10]);
-    const double sc = sqrt(ld.x * ld.x + ld.y * ld.y + ld.z * ld.z), isc = 1.0 / sc;
+    const double sc = sqrt(ld.x * ld.x + ld.y * ld.y + ld.z * ld.z);
+    isc = quotient(1.0, sc);
     ld = make_double3(ld.x * isc, ld.y * isc, ld.z * isc);
-    double t = double(hit.t) * sc, u = hit.u, v = hit.v;
-    if (newton_polish64(P, lo, ld, t, u, v)) { hit.t = float(t * isc); hit.u = float(u); hit.v = float(v); }
+    polish_begin(p, P, lo, ld, widen(hit.t) * sc, widen(hit.u), widen(hit.v));
+}
+static __device__ __noinline__ void polish_hit(const DevScene& S, float3 o, float3 d, HitRecord& hit)
+{
+    Polish p;
+    double isc;
+    polish_start(S, o, d, hit, p, isc);
+    PolishNext next = kPolishStep;
+    while (next == kPolishStep) next = polish_step(p);
+    while (next == kPolishStep64) next = polish_step64(p);
+    if (next == kPolishDone && polish_accepted(p))
+    {
+        hit.t = narrow(p.T * isc); hit.u = narrow(p.U); hit.v = narrow(p.V);
+    }
 }
 
 // Closest hit over the object-level BVH and each object's patch BVH
