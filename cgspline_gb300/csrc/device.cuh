@@ -105,6 +105,7 @@ __device__ __forceinline__ float3 group_ambient(const DevScene& S, uint32_t g)
 struct Counters
 {
     unsigned long long nodes, hashLookups, candidates, iterations, rays, errors, tableReads;
+    unsigned long long longLists;  // long candidate lists taken (the query engine's allocator)
 };
 
 struct LocalCounters

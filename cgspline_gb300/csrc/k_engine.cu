@@ -77,6 +77,9 @@ constexpr int kMaxPasses = 8;
 
 // list entry word 0: a patch index, or one of these markers (word 1 = object)
 constexpr uint32_t kLeave = 0xFFFFFFFFu, kEnter = 0xFFFFFFFEu, kCont = 0xFFFFFFFDu;
+// or, in place of the first entry: the list is long list word 1
+constexpr uint32_t kLong = 0xFFFFFFFCu;
+constexpr uint32_t kLongList = 256;  // entries of a long list
 // ray status
 enum : uint32_t { kPending = 0, kTraversed = 1, kFinished = 2 };
 
@@ -97,9 +100,22 @@ struct Eng  // per-ray engine state, SoA over the query's capacity
     uint32_t packetWidth;  // idle lanes a warp gathers before the traversal refills it
     uint32_t originLast;   // any hit: search candidates whose leaf box holds the ray's origin last
     uint32_t subdivLevels; // subdivision searches: bisection levels a lane runs per resolve round
+    // Long lists, for the few rays whose candidates on a walk tree outgrow their
+    // chunk: kLongList entries each, taken by *longNext, nlong of them (none left:
+    // the ray goes back to the reference tree).
+    uint2* longs;
+    uint32_t nlong;
+    unsigned long long* longNext;
+    __device__ __forceinline__ uint2* list_of(uint32_t rid) const
+    {
+        uint2* l = list + size_t(rid) * kChunk;
+        const uint2 first = l[0];
+        return first.x == kLong ? longs + size_t(first.y) * kLongList : l;
+    }
 };
 
 constexpr size_t kWordsPerRay = 2 + 2 * kChunk + 18;
+constexpr uint32_t long_lists(uint32_t cap) { return cap / 48 + 32; }
 
 Eng carve(uint32_t* base, uint32_t cap)
 {
@@ -116,6 +132,10 @@ Eng carve(uint32_t* base, uint32_t cap)
     e.lv = reinterpret_cast<float*>(take(cap));
     e.queue[0] = take(cap); e.queue[1] = take(cap);
     e.ctl = take(4 * (kMaxPasses + 1));
+    if (size_t(p - base) % 2) p++;
+    e.nlong = long_lists(cap);
+    e.longs = reinterpret_cast<uint2*>(take(2ull * e.nlong * kLongList));
+    e.longNext = nullptr;
     return e;
 }
 
@@ -227,6 +247,7 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
     uint32_t topIdx = 0;  // the ray's object-level BVH (its group's)
     BvhRef B {};  // the BVH walked now; its hash parameters are read at a table lookup
     uint2* list = nullptr;
+    uint32_t cap = 0;  // entries that the list in hand holds
     const uint32_t m = src.m;
     for (;;)
     {
@@ -254,6 +275,7 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                 load_ray(rays, rid, o, d, tmax);
                 inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
                 list = E.list + size_t(rid) * kChunk;
+                cap = min(kChunk, E.chunk << pass);
                 ncand = 0;
                 rstate = 0;
                 topIdx = __ldg(S.groupTop + g);
@@ -291,10 +313,26 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
         if (__ballot_sync(0xFFFFFFFFu, active || !exhausted) == 0) break;
         if (!active) continue;
 
-        if (ncand + kMaxAppendsPerStep > min(kChunk, E.chunk << pass))
+        if (ncand + kMaxAppendsPerStep > cap)
         {
             if (kWalk && obj >= 0 && B.indexBase == EMPTY)
             {
+                // a full chunk goes on in a long list: a search of all of an
+                // object's candidates in the reference order keeps the same
+                // hit as one chunk by chunk, which would cull some of them first
+                if (cap == kChunk && E.nlong)
+                {
+                    const unsigned long long at = atomicAdd(E.longNext, 1ull);
+                    if (at < E.nlong)
+                    {
+                        uint2* l = E.longs + size_t(at) * kLongList;
+                        for (uint32_t k = 0; k < ncand; k++) l[k] = list[k];
+                        list[0] = make_uint2(kLong, uint32_t(at));
+                        list = l;
+                        cap = kLongList;
+                        continue;
+                    }
+                }
                 // the object's patches do not fit: collect it again on the
                 // reference tree, whose order decides which of them do
                 do ncand--; while (list[ncand].x != kEnter);
@@ -508,6 +546,39 @@ __global__ void __launch_bounds__(kCollectThreads, 4) k_collect(DevScene S, Rays
 }
 
 // -------------------------------------------------------------- order --
+// The lists of a closest-hit pass whose objects were collected on walk trees,
+// into the reference traversal's order: one thread per ray, a segment (an
+// object's patches) at a time.  What was collected on the reference tree is in
+// order and stays.
+//
+// An insertion sort in place: segments are short (8.6 patches on a ray of the
+// 1920x1080 torus frame that hits) and the walk meets them in nearly that order.
+// Bound by the latency of the comparisons' loads (hash, node) and the lists'
+// scattered lines: 300 us for 2,073,600 rays, held to 64 registers.  (Testing only
+// the m - 1 nodes where neighbouring heap keys part and sorting by keys with those
+// bits flipped has a third of the tests and took 372 us, its arrays in local memory.)
+//
+// A long segment is sorted by its warp instead: each patch gets a code with a
+// bit per level of the reference tree, 1 where its path takes the child visited
+// last, which orders as the traversal does.
+constexpr int kOrderThreads = 128;
+constexpr uint32_t kLongSegment = 24;
+
+// Whether the reference traversal by the ray (ro, ri) visits the left child of
+// the node with heap key `key` first.
+__device__ __forceinline__ bool left_first(const DevScene& S, const DevBVH& H, uint32_t key, float3 ro, float3 ri)
+{
+    const uint32_t node = __ldg(S.tables + H.tableBase + hash_slot(S, H, key));
+    const float4* q = S.nodes + 4ull * (H.nodeBase + node);
+    float4 q0, q1, q2, q3;
+    ldg256(q, q0, q1);
+    ldg256(q + 2, q2, q3);
+    float L0, R0;
+    slab(L0, f3(q0.x, q0.y, q0.z), f3(q0.w, q1.x, q1.y), ro, ri);
+    slab(R0, f3(q1.z, q1.w, q2.x), f3(q2.y, q2.z, q2.w), ro, ri);
+    return L0 < R0;
+}
+
 // Whether leaf a (heap key) comes before leaf b in the reference traversal of
 // BVH H by the ray (ro, ri), both of them met: at their lowest common
 // ancestor the nearer child goes first, the right one on equal distances.
@@ -517,68 +588,165 @@ __device__ __forceinline__ bool visits_first(const DevScene& S, const DevBVH& H,
     const int da = __clz(a), db = __clz(b);  // the deeper key has fewer leading zeros
     if (da < db) a >>= db - da; else b >>= da - db;
     const int up = 32 - __clz(a ^ b);
-    const uint32_t node = __ldg(S.tables + H.tableBase + hash_slot(S, H, a >> up));
-    const float4* q = S.nodes + 4ull * (H.nodeBase + node);
-    float4 q0, q1, q2, q3;
-    ldg256(q, q0, q1);
-    ldg256(q + 2, q2, q3);
-    float L0, R0;
-    slab(L0, f3(q0.x, q0.y, q0.z), f3(q0.w, q1.x, q1.y), ro, ri);
-    slab(R0, f3(q1.z, q1.w, q2.x), f3(q2.y, q2.z, q2.w), ro, ri);
-    return (L0 < R0) == (((a >> (up - 1)) & 1u) == 0u);
+    return left_first(S, H, a >> up, ro, ri) == (((a >> (up - 1)) & 1u) == 0u);
 }
 
-// The lists of a closest-hit pass whose objects were collected on walk trees,
-// into the reference traversal's order: one thread per ray, an insertion
-// sort of each object's patches (two or three on most rays, in nearly that
-// order already).  What was collected on the reference tree is in order and stays.
-constexpr int kOrderThreads = 128;
-template<class Source>
-__device__ __forceinline__ void order_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, const Source& src,
-                                           uint32_t first, uint32_t stride)
+// The ray, BVH and keys of an entered object that has a walk tree.
+struct OrderSegment
 {
-    for (uint32_t i = first; i < src.m; i += stride)
+    float3 ro, ri;
+    DevBVH H;
+    const uint32_t* keys;
+    __device__ __forceinline__ bool open(const DevScene& S, const RaysSoA& rays, uint32_t rid, uint32_t obj)
     {
-        const uint32_t rid = src.ray(i);
-        const uint32_t count = E.count[rid];
-        uint2* list = E.list + size_t(rid) * kChunk;
-        for (uint32_t k = 0; k + 2 < count; k++)
-        {
-            if (list[k].x != kEnter) continue;
-            // patches are list[k + 1 .. end); end is the object's leave marker or the list's end
-            if (list[k + 1].x >= kCont || list[k + 2].x >= kCont) continue;
-            const DevObject& O = S.objects[list[k].y];
-            const DevBVH H = S.bvhs[O.surface];
-            if (H.walkBase == EMPTY) continue;
-            float3 o, d, ro, ld;
-            float tmax, lmax, sinv;
-            load_ray(rays, rid, o, d, tmax);
-            to_local(O, o, d, tmax, ro, ld, lmax, sinv);
-            const float3 ri = f3(1.0f / ld.x, 1.0f / ld.y, 1.0f / ld.z);
-            const uint32_t* keys = S.leafKeys + __ldg(S.patchBase + O.surface);
-            uint32_t j = k + 2;
-            for (; j < count && list[j].x < kCont; j++)
-            {
-                const uint2 e = list[j];
-                const uint32_t ke = __ldg(keys + e.x);
-                uint32_t at = j;
-                for (; at > k + 1; at--)
-                {
-                    const uint2 p = list[at - 1];
-                    if (visits_first(S, H, __ldg(keys + p.x), ke, ro, ri)) break;
-                    list[at] = p;
-                }
-                if (at != j) list[at] = e;
-            }
-            k = j - 1;
-        }
+        const DevObject& O = S.objects[obj];
+        H = S.bvhs[O.surface];
+        if (H.walkBase == EMPTY) return false;
+        float3 o, d, ld;
+        float tmax, lmax, sinv;
+        load_ray(rays, rid, o, d, tmax);
+        to_local(O, o, d, tmax, ro, ld, lmax, sinv);
+        ri = f3(1.0f / ld.x, 1.0f / ld.y, 1.0f / ld.z);
+        keys = S.leafKeys + __ldg(S.patchBase + O.surface);
+        return true;
     }
+};
+
+// The long segments of one ray's list, by a whole warp.
+__device__ __forceinline__ void order_long(const DevScene& S, const RaysSoA& rays, uint2* list, uint32_t rid,
+                                               uint32_t n)
+{
+    const uint32_t lane = lane_id();
+    for (uint32_t k = 0; k + kLongSegment < n; k++)
+    {
+        if (list[k].x != kEnter) continue;
+        uint32_t end = k + 1;
+        while (end < n && list[end].x < kCont) end++;
+        OrderSegment G;
+        const uint32_t size = end - (k + 1);
+        if (size > kLongSegment && G.open(S, rays, rid, list[k].y))
+        {
+            // ranks by counting smaller codes; up to kLongList entries, 8 a lane
+            uint2 e[kLongList / 32];
+            uint32_t code[kLongList / 32], rank[kLongList / 32];
+#pragma unroll
+            for (uint32_t c = 0; c < kLongList / 32; c++)
+            {
+                const uint32_t at = c * 32 + lane;
+                rank[c] = 0;
+                code[c] = 0xFFFFFFFFu;
+                if (at >= size) continue;
+                e[c] = list[k + 1 + at];
+                const uint32_t key = __ldg(G.keys + e[c].x);
+                const int depth = 31 - __clz(key);
+                code[c] = 0;
+                for (int l = 0; l < depth; l++)
+                {
+                    const uint32_t child = key >> (depth - 1 - l);
+                    if (left_first(S, G.H, child >> 1, G.ro, G.ri) != ((child & 1u) == 0u)) code[c] |= 0x80000000u >> l;
+                }
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < kLongList / 32; c++)
+            {
+                if (c * 32 >= size) break;
+                const uint32_t there = min(32u, size - c * 32);
+                for (uint32_t l = 0; l < there; l++)
+                {
+                    const uint32_t other = __shfl_sync(0xFFFFFFFFu, code[c], int(l));
+#pragma unroll
+                    for (uint32_t x = 0; x < kLongList / 32; x++) rank[x] += other < code[x] ? 1u : 0u;
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (uint32_t c = 0; c < kLongList / 32; c++)
+                if (c * 32 + lane < size) list[k + 1 + rank[c]] = e[c];
+            __syncwarp();
+        }
+        k = end - 1;
+    }
+}
+
+// Orders one ray's segments; true if it has a long one, which is left.
+__device__ __forceinline__ bool order_ray(const DevScene& S, const RaysSoA& rays, const Eng& E, uint32_t rid, uint32_t count)
+{
+    bool longer = false;
+    if (count <= 3) return false;
+    uint2* list = E.list_of(rid);
+    for (uint32_t k = 0; k + 2 < count; k++)
+    {
+        if (list[k].x != kEnter) continue;
+        // the segment is list[k + 1 .. end): to the object's leave marker or the list's end
+        if (list[k + 1].x >= kCont || list[k + 2].x >= kCont) continue;
+        OrderSegment G;
+        if (!G.open(S, rays, rid, list[k].y)) continue;
+        uint32_t j = k + 2;
+        for (; j < count && list[j].x < kCont; j++)
+        {
+            if (j > k + kLongSegment) { longer = true; break; }
+            const uint2 e = list[j];
+            const uint32_t ke = __ldg(G.keys + e.x);
+            uint32_t at = j;
+            for (; at > k + 1; at--)
+            {
+                const uint2 p = list[at - 1];
+                if (visits_first(S, G.H, __ldg(G.keys + p.x), ke, G.ro, G.ri)) break;
+                list[at] = p;
+            }
+            if (at != j) list[at] = e;
+        }
+        k = j - 1;
+    }
+    return longer;
 }
 __global__ void __launch_bounds__(kOrderThreads) k_order(DevScene S, RaysSoA rays, uint32_t n0, const uint32_t* nDev,
                                                          Eng E, int pass)
 {
-    order_rays(S, rays, E, PassSource<0>(E, pass, n0, nDev), blockIdx.x * blockDim.x + threadIdx.x,
-               gridDim.x * blockDim.x);
+    const PassSource<0> src(E, pass, n0, nDev);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < src.m; i += gridDim.x * blockDim.x)
+    {
+        const uint32_t rid = src.ray(i);
+        // the rays left to k_order_long: in the queue that the next k_pending fills
+        if (order_ray(S, rays, E, rid, E.count[rid])) E.queue[(pass + 1) & 1][atomicAdd(E.ctl + 4 * pass + 3, 1u)] = rid;
+    }
+}
+// Orders a source's rays 32 at a time, all of their segments, by one warp of several (warp w of nw).
+template<class Source>
+__device__ __forceinline__ void order_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, const Source& src,
+                                           uint32_t w, uint32_t nw)
+{
+    const uint32_t lane = lane_id();
+    for (uint32_t i0 = 32 * w; i0 < src.m; i0 += 32 * nw)
+    {
+        const uint32_t rid = i0 + lane < src.m ? src.ray(i0 + lane) : 0u;
+        const uint32_t count = i0 + lane < src.m ? E.count[rid] : 0u;
+        const bool longer = order_ray(S, rays, E, rid, count);
+        for (unsigned b = __ballot_sync(0xFFFFFFFFu, longer); b; b &= b - 1)
+        {
+            const int owner = __ffs(b) - 1;
+            const uint32_t r = __shfl_sync(0xFFFFFFFFu, rid, owner), n = __shfl_sync(0xFFFFFFFFu, count, owner);
+            __syncwarp();
+            order_long(S, rays, E.list_of(r), r, n);
+        }
+    }
+}
+// A later pass's rays: few, so in one launch.
+__global__ void __launch_bounds__(kOrderThreads) k_order_queue(DevScene S, RaysSoA rays, Eng E, int pass)
+{
+    order_rays(S, rays, E, PassSource<0>(E, pass, 0, nullptr), (blockIdx.x * blockDim.x + threadIdx.x) / 32,
+               gridDim.x * blockDim.x / 32);
+}
+// The first pass's rays with long segments, a warp each: a kernel of its own, so
+// that its registers are not k_order's.
+__global__ void __launch_bounds__(kOrderThreads) k_order_long(DevScene S, RaysSoA rays, Eng E, int pass)
+{
+    const uint32_t m = E.ctl[4 * pass + 3], nw = gridDim.x * blockDim.x / 32;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < m; i += nw)
+    {
+        const uint32_t rid = E.queue[(pass + 1) & 1][i];
+        order_long(S, rays, E.list_of(rid), rid, E.count[rid]);
+    }
 }
 
 // ------------------------------------------------------------ resolve --
@@ -607,7 +775,7 @@ template<bool kAny> struct ListWalk
         sweep = false;
         load_ray(rays, rid, o, d, tmax);
         limit = kAny ? tmax : (pass == 0 ? tmax : E.limit[rid]);
-        list = E.list + size_t(rid) * kChunk;
+        list = E.list_of(rid);
         return true;
     }
 
@@ -1346,7 +1514,9 @@ __global__ void __launch_bounds__(kPolishThreads) k_polish(DevScene S, RaysSoA r
 // host about 6 us, and a query of separate kernels is 11 of them and two
 // memsets.  Each ray goes through the same steps, with the same results.
 template<bool kAny, bool kG64, bool kSub>
-__global__ void __launch_bounds__(32, 8) k_small(DevScene S, RaysSoA rays, uint32_t n0, const uint32_t* nDev,
+__global__ void __launch_bounds__(32, 8) k_small(DevScene S,
+                                                              RaysSoA rays, uint32_t n0,
+                                                              const uint32_t* nDev,
                                                               Eng E, int passes, int cache, Query q, HitsSoA hits,
                                                               int32_t* occluded, Counters* cnt)
 {
@@ -1390,7 +1560,8 @@ __global__ void __launch_bounds__(32, 8) k_small(DevScene S, RaysSoA rays, uint3
         __syncwarp();
         collect_rays<kAny, false, true>(S, rays, E, p, cache, src, ring, lc, nrays);
         __syncwarp();
-        if (!kAny && S.leafKeys) order_rays(S, rays, E, src, lane, 32);
+        if (!kAny && S.leafKeys)
+            order_rays(S, rays, E, src, 0, 1);
         if (lane == 0) fetch = 0;
         __syncwarp();
         if constexpr (kSub) subdivide_rays<kAny>(S, rays, E, p, q, hits, occluded, src, lend, lc, ListWalk<kAny> {});
@@ -1520,9 +1691,14 @@ void launch(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Q
         launch_collect<kAny>(gc, ct, stream, S, rays, n, nDev, E, p, c, cnt);
         if (!kAny && S.leafKeys)
         {
-            const uint32_t blocks = (n + kOrderThreads - 1) / kOrderThreads;
-            k_order<<<int(std::min<uint32_t>(blocks, uint32_t(sms() * 16))), kOrderThreads, 0, stream>>>(S, rays, n,
-                                                                                                        nDev, E, p);
+            const int blocks = int(std::min<uint32_t>((n + kOrderThreads - 1) / kOrderThreads, uint32_t(sms() * 16)));
+            if (p == 0)
+            {
+                k_order<<<blocks, kOrderThreads, 0, stream>>>(S, rays, n, nDev, E, p);
+                k_order_long<<<sms(), kOrderThreads, 0, stream>>>(S, rays, E, p);
+                nl++;
+            }
+            else k_order_queue<<<blocks, kOrderThreads, 0, stream>>>(S, rays, E, p);
             nl++;
         }
         search_kernel<kAny, kG64, kSub>()<<<gr, rt, 0, stream>>>(S, rays, n, nDev, E, p, q, hits, occluded, cnt);
@@ -1580,7 +1756,7 @@ bool set_engine_config(const EngineConfig& c)
 
 size_t engine_words(uint32_t capacity, int)
 {
-    return size_t(capacity) * kWordsPerRay + 4 * (kMaxPasses + 1) + 64;
+    return size_t(capacity) * kWordsPerRay + 4 * (kMaxPasses + 1) + 64 + 2ull * kLongList * long_lists(capacity);
 }
 
 cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Query q, bool any,
@@ -1605,6 +1781,8 @@ cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_
         E.originLast = uint32_t(ec.originLast);
         E.subdivLevels = uint32_t(ec.subdivLevels);
     }
+    E.longNext = &cnt->longLists;
+    if (!cnt) E.nlong = 0;
     int nl = 0;
     if (any) q.method != 0 ? launch<true, false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl)
                            : launch<true, false>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);
@@ -1641,6 +1819,7 @@ cudaError_t run_traverse(const DevScene& S, RaysSoA rays, uint32_t n, bool any, 
         E.originLast = uint32_t(ec.originLast);
         E.subdivLevels = uint32_t(ec.subdivLevels);
     }
+    E.nlong = 0;  // a list as long as a chunk is the entry point's contract
     cudaMemsetAsync(E.ctl, 0, sizeof(uint32_t) * 4 * (kMaxPasses + 1), stream);
     const EngineConfig c = engine_config();
     const int ct = c.collectThreads;

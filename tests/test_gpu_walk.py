@@ -81,6 +81,33 @@ def test_ties_and_full_lists_match_the_reference_order(copies, objects, engine, 
     assert np.array_equal(free, ~occluded)
 
 
+@pytest.mark.parametrize("copies,objects", [(31, 1), (32, 1), (90, 1), (120, 1), (130, 1), (150, 2), (15, 7)])
+@pytest.mark.parametrize("n", [37, 70001])
+def test_long_lists_match_the_reference(copies, objects, n, oracle_mod):
+    """A few rays whose candidates outgrow their chunk, alone and among 70,000 rays that miss: they go on in long lists
+    (one of 256 entries each), which are sorted by a warp; past that, on the reference tree."""
+    torch = pytest.importorskip("torch")
+    from cgspline_gb300 import _capi, rt
+    sc = stacked(copies, objects=objects)
+    rays = np.ascontiguousarray(field_rays(2)[:, :: 173])  # 37 rays
+    ref = oracle_mod.OracleScene(sc).intersect(rays, method=oracle_mod.CLIP_DEVICE)
+    assert rays.shape[1] <= 37 and (ref["patch"] >= 0).mean() > 0.4
+    at = np.linspace(0, n - 1, rays.shape[1]).astype(np.int64)
+    many = np.zeros((7, n), np.float32)
+    many[2], many[5], many[6] = 50.0, 1.0, np.inf
+    many[:, at] = rays
+    g = rt.GpuScene(sc, lib_path=_capi.LIB_NOFMA_PATH)
+    dev = torch.from_numpy(many).cuda()
+    got = {k: v.cpu().numpy() for k, v in g.intersect(dev).items()}
+    free = g.intersect(dev, any_hit=True)["patch"].cpu().numpy() < 0
+    assert g.counters()["device_errors"] == 0
+    g.close()
+    for k in ("t", "u", "v", "patch", "object"):
+        assert np.array_equal(got[k][at], ref[k]), (k, int((got[k][at] != ref[k]).sum()))
+    assert (np.delete(got["patch"], at) < 0).all()
+    assert np.array_equal(free[at], ref["patch"] < 0)
+
+
 def test_loaded_store_walks_its_own_trees(tmp_path):
     """A store read back gives the built one's hits; one whose file hides the root's left half behind an empty box is
     walked as the file says."""
