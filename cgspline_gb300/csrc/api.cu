@@ -355,6 +355,16 @@ void query_end(cgs_scene* s, cudaStream_t st, bool captured)
     }
 }
 
+// How many of the rows of n words from rows[0] on lie one after another in
+// memory: those go in one copy (a copy of a few rays costs about 6 us of calls,
+// and a query took twelve: 33 rays 162 us, 130 us with three).
+template<class T> int adjacent_rows(const T* const* rows, int count, uint32_t n)
+{
+    int run = 1;
+    while (rows[0] && run < count && rows[run] == rows[run - 1] + n) run++;
+    return run;
+}
+
 }  // namespace cgs
 
 extern "C" {
@@ -436,10 +446,14 @@ int cgs_intersect_host(cgs_scene* s, const cgs_rays* rays, uint32_t n, int metho
         CGS_TRY(s->hitF.reserve(3ull * n));
         CGS_TRY(s->hitI.reserve(2ull * n));
         const float* src[7] = {rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax};
-        for (int k = 0; k < 7; k++)
+        for (int k = 0; k < 6; k++)
+            if (!src[k]) return CGS_ERR_INVALID_ARGUMENT;
+        for (int k = 0, run; k < 7; k += run)
         {
-            if (!src[k]) { if (k == 6) continue; return CGS_ERR_INVALID_ARGUMENT; }
-            CGS_TRY(cudaMemcpyAsync(s->rayStage.p + size_t(k) * n, src[k], n * sizeof(float), cudaMemcpyHostToDevice, st));
+            run = adjacent_rows(src + k, 7 - k, n);
+            if (src[k])
+                CGS_TRY(cudaMemcpyAsync(s->rayStage.p + size_t(k) * n, src[k], size_t(run) * n * sizeof(float),
+                                        cudaMemcpyHostToDevice, st));
         }
         float* R = s->rayStage.p;
         dr = cgs_rays {R, R + n, R + 2ull * n, R + 3ull * n, R + 4ull * n, R + 5ull * n,
@@ -454,13 +468,21 @@ int cgs_intersect_host(cgs_scene* s, const cgs_rays* rays, uint32_t n, int metho
     }
     int r = cgs_intersect(s, &dr, n, method, precision, tol, any_hit, &dh, stream);
     if (r) return r;
-    if (hits->patch) CGS_TRY(cudaMemcpyAsync(hits->patch, dh.patch, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    if (!any_hit)
+    const int32_t* whole[2] = {hits->patch, any_hit ? nullptr : hits->object};
+    for (int k = 0, run; k < 2; k += run)
     {
-        if (hits->t) CGS_TRY(cudaMemcpyAsync(hits->t, dh.t, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-        if (hits->u) CGS_TRY(cudaMemcpyAsync(hits->u, dh.u, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-        if (hits->v) CGS_TRY(cudaMemcpyAsync(hits->v, dh.v, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-        if (hits->object) CGS_TRY(cudaMemcpyAsync(hits->object, dh.object, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        run = adjacent_rows(whole + k, 2 - k, n);
+        if (whole[k])
+            CGS_TRY(cudaMemcpyAsync(const_cast<int32_t*>(whole[k]), s->hitI.p + size_t(k) * n,
+                                    size_t(run) * n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    }
+    const float* real[3] = {hits->t, hits->u, hits->v};
+    for (int k = 0, run; !any_hit && k < 3; k += run)
+    {
+        run = adjacent_rows(real + k, 3 - k, n);
+        if (real[k])
+            CGS_TRY(cudaMemcpyAsync(const_cast<float*>(real[k]), s->hitF.p + size_t(k) * n,
+                                    size_t(run) * n * sizeof(float), cudaMemcpyDeviceToHost, st));
     }
     CGS_TRY(cudaStreamSynchronize(st));
     return CGS_OK;
