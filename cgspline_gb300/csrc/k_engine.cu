@@ -105,6 +105,7 @@ struct Eng  // per-ray engine state, SoA over the query's capacity
     // the ray goes back to the reference tree).
     uint2* longs;
     uint32_t nlong;
+    uint32_t allMarkers;  // lists keep the markers of objects that the ray meets no patch of (cgs_traverse)
     unsigned long long* longNext;
     __device__ __forceinline__ uint2* list_of(uint32_t rid) const
     {
@@ -136,6 +137,7 @@ Eng carve(uint32_t* base, uint32_t cap)
     e.nlong = long_lists(cap);
     e.longs = reinterpret_cast<uint2*>(take(2ull * e.nlong * kLongList));
     e.longNext = nullptr;
+    e.allMarkers = 0;
     return e;
 }
 
@@ -244,6 +246,7 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
     float leafEntry = -INFINITY;
     int32_t obj = -1;
     bool walk = true;     // false: the object in hand is walked on the reference tree
+    bool hollow = false;  // the list ends with the marker that entered the object in hand
     uint32_t topIdx = 0;  // the ray's object-level BVH (its group's)
     BvhRef B {};  // the BVH walked now; its hash parameters are read at a table lookup
     uint2* list = nullptr;
@@ -306,6 +309,7 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                         clim = kAny ? lmax : E.lt[rid];
                         B = bvh_ref<kQ, kWalk>(S, O.surface, walk);
                         list[ncand++] = make_uint2(kCont, uint32_t(obj));
+                        hollow = false;
                     }
                 }
             }
@@ -337,6 +341,7 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                 // reference tree, whose order decides which of them do
                 do ncand--; while (list[ncand].x != kEnter);
                 ncand++;
+                hollow = true;
                 walk = false;
                 node = 0; key = 1; post = 0; leaf = EMPTY; jumped = false;
                 leafEntry = -INFINITY;
@@ -375,9 +380,13 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                     node = 0; key = 1; post = 0; leaf = EMPTY; jumped = false;
                     leafEntry = -INFINITY;
                     list[ncand++] = make_uint2(kEnter, e);
+                    hollow = true;
                 }
                 else
+                {
                     list[ncand++] = make_uint2(e, __float_as_uint(leafEntry));
+                    hollow = false;
+                }
             }
             else
             {
@@ -448,10 +457,12 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                     node = 0; key = 1; post = 0; leaf = EMPTY; jumped = false;
                     leafEntry = -INFINITY;
                     list[ncand++] = make_uint2(kEnter, e0);
+                    hollow = true;
                 }
                 else
                 {
                     list[ncand++] = make_uint2(e0, __float_as_uint(leafEntry));
+                    hollow = false;
                     if (e1 == EMPTY)
                     {
                         leaf = EMPTY;
@@ -493,7 +504,11 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                     done = true;
                 else
                 {
-                    list[ncand++] = make_uint2(kLeave, uint32_t(obj));
+                    // an object without candidates leaves nothing in the list: the search
+                    // kernel enters no object in vain and skips rays that miss (2,073,600
+                    // primary rays 2.56 -> 2.49 ms)
+                    if (hollow && !E.allMarkers) ncand--;
+                    else list[ncand++] = make_uint2(kLeave, uint32_t(obj));
                     obj = -1;
                     walk = true;
                     co = o; ci = inv; clim = limit;
@@ -1819,7 +1834,8 @@ cudaError_t run_traverse(const DevScene& S, RaysSoA rays, uint32_t n, bool any, 
         E.originLast = uint32_t(ec.originLast);
         E.subdivLevels = uint32_t(ec.subdivLevels);
     }
-    E.nlong = 0;  // a list as long as a chunk is the entry point's contract
+    E.nlong = 0;  // a list of patches and markers as long as a chunk is the entry point's contract
+    E.allMarkers = 1;
     cudaMemsetAsync(E.ctl, 0, sizeof(uint32_t) * 4 * (kMaxPasses + 1), stream);
     const EngineConfig c = engine_config();
     const int ct = c.collectThreads;
