@@ -263,7 +263,7 @@ int device_sms()
 
 // ------------------------------------------ one CTA or cluster per BVH --
 // The same build for one BVH run entirely on the device by one CTA (kShared:
-// up to kHashBlockMaxKeys keys) or one cluster of kHashCluster CTAs (up to
+// up to kHashBlockMaxKeys keys) or one cluster of 16 CTAs (up to
 // kHashGlobalBlockMaxKeys): the bid and commit phases of a round are separated
 // by a CTA or cluster barrier instead of kernel launches, and a whole store's
 // BVHs are built by one launch of each kind, with no host round trip between
@@ -274,16 +274,15 @@ int device_sms()
 // and its read-back, up to 128 rounds per trial.  So a thread keeps its buckets
 // (at most kItems of the class in hand, in rank order) in registers and a
 // round touches only the slots' owner tags, which are in the CTA's shared
-// memory or spread over the cluster's, slot s in CTA s % kHashCluster; a slot's
+// memory or spread over the cluster's, slot s in CTA s % C; a slot's
 // tag is (round, rank) in 16 + 16 bits (rounds < 2^11, ranks < 2^16), lower
 // for later rounds, and 0 once a bucket is placed there.  A trial ends at the
 // first class that does not place all of its buckets: it has failed then.
-// 39,199 keys (15 trials): 1.60 ms; 15.8 ms as one CTA that swept all buckets
+// 39,199 keys (15 trials): 1.33 ms, 1.60 ms by 8 CTAs, 15.8 ms as one CTA that swept all buckets
 // of a global scratch area in every round and ran failed trials to their end.
 // The 25 BVHs of a 30,000-patch store, largest 4,800 keys: 0.257 ms, before 0.707 ms.
 // The cluster's rounds are bound by their scattered reads of other CTAs' memory
-// (about 3.3 us a round at 39,199 keys).
-constexpr int kHashCluster = 8;
+// (about 2.8 us a round at 39,199 keys).
 
 __device__ __forceinline__ uint4 warp_incl_scan4(uint4 v)
 {
@@ -302,13 +301,15 @@ __device__ __forceinline__ uint4 warp_incl_scan4(uint4 v)
 // Words of the bucket arrays: bkeys [4 nb], bsize, ord, dcur [nb] each.
 __host__ __device__ inline uint64_t bucket_words(uint32_t nb) { return 7ull * nb; }
 
-template<bool kShared>
+// kCluster: 1 (everything in one CTA's shared memory), else the CTAs of a cluster.
+template<int kCluster>
 __global__ void __launch_bounds__(kBlockThreads) k_hash_block(const uint32_t* __restrict__ keys,
                                                               const HashJob* __restrict__ jobs, uint32_t* disps,
                                                               uint32_t* tables, uint32_t* out, uint32_t* gscratch)
 {
-    constexpr uint32_t C = kShared ? 1u : uint32_t(kHashCluster);
-    constexpr int kItems = kShared ? 2 : 4;  // nb <= kItems * C * bd below
+    constexpr bool kShared = kCluster == 1;
+    constexpr uint32_t C = kCluster;
+    constexpr int kItems = kCluster == 8 ? 4 : 2;  // nb <= kItems * C * bd below
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint32_t sErr, sCount[4], sPlaced[64];  // sPlaced: the first CTA's is the cluster's
     __shared__ uint4 sWarp[kBlockThreads / 32];
@@ -658,24 +659,37 @@ cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_
     if (maxKeys > kHashGlobalBlockMaxKeys || (maxKeys > kHashBlockMaxKeys && !gscratch)) return cudaErrorInvalidValue;
     uint32_t nb = 0, nmax = 0;
     block_sizes(maxKeys, nb, nmax);
-    const bool shared = maxKeys <= kHashBlockMaxKeys;
-    const size_t smem = sizeof(uint32_t) *
-                        (shared ? size_t(bucket_words(nb)) + nmax : size_t(nmax + kHashCluster - 1) / kHashCluster);
-    auto* k = shared ? k_hash_block<true> : k_hash_block<false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(shared ? njobs : njobs * kHashCluster);
-    cfg.blockDim = dim3(kBlockThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = shared ? 1 : kHashCluster;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, keys, jobs, disps, tables, out, gscratch);
+    auto launch = [&](auto* k, uint32_t cluster, bool probe) {
+        const size_t smem =
+            sizeof(uint32_t) * (cluster == 1 ? size_t(bucket_words(nb)) + nmax : size_t(nmax + cluster - 1) / cluster);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e == cudaSuccess && cluster > 8)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg {};
+        cfg.gridDim = dim3(njobs * cluster);
+        cfg.blockDim = dim3(kBlockThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute at {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = cluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        if (probe)
+        {
+            int fits = 0;
+            e = cudaOccupancyMaxActiveClusters(&fits, k, &cfg);
+            return e != cudaSuccess ? e : fits > 0 ? cudaSuccess : cudaErrorInvalidConfiguration;
+        }
+        return cudaLaunchKernelEx(&cfg, k, keys, jobs, disps, tables, out, gscratch);
+    };
+    if (maxKeys <= kHashBlockMaxKeys) return launch(k_hash_block<1>, 1u, false);
+    // clusters of 16 are outside the portable size: where none fits on the device, 8
+    if (launch(k_hash_block<16>, 16u, true) == cudaSuccess) return launch(k_hash_block<16>, 16u, false);
+    cudaGetLastError();
+    return launch(k_hash_block<8>, 8u, false);
 }
 
 }  // namespace cgs
