@@ -301,15 +301,15 @@ __device__ __forceinline__ uint4 warp_incl_scan4(uint4 v)
 // Words of the bucket arrays: bkeys [4 nb], bsize, ord, dcur [nb] each.
 __host__ __device__ inline uint64_t bucket_words(uint32_t nb) { return 7ull * nb; }
 
-// kCluster: 1 (everything in one CTA's shared memory), else the CTAs of a cluster.
-template<int kCluster>
+// kCluster: 1 (everything in one CTA's shared memory), else the CTAs of a cluster;
+// nb <= kItems * kCluster * bd below.
+template<int kCluster, int kItems = 2>
 __global__ void __launch_bounds__(kBlockThreads) k_hash_block(const uint32_t* __restrict__ keys,
                                                               const HashJob* __restrict__ jobs, uint32_t* disps,
                                                               uint32_t* tables, uint32_t* out, uint32_t* gscratch)
 {
     constexpr bool kShared = kCluster == 1;
     constexpr uint32_t C = kCluster;
-    constexpr int kItems = kCluster == 8 ? 4 : 2;  // nb <= kItems * C * bd below
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint32_t sErr, sCount[4], sPlaced[64];  // sPlaced: the first CTA's is the cluster's
     __shared__ uint4 sWarp[kBlockThreads / 32];
@@ -644,6 +644,13 @@ void block_sizes(uint32_t n, uint32_t& nb, uint32_t& nmax)
 
 }  // namespace
 
+uint32_t hash_block_buckets(uint32_t n)
+{
+    uint32_t nb = 0, nmax = 0;
+    block_sizes(n, nb, nmax);
+    return nb;
+}
+
 uint64_t hash_block_scratch_words(uint32_t n)
 {
     uint32_t nb = 0, nmax = 0;
@@ -653,7 +660,7 @@ uint64_t hash_block_scratch_words(uint32_t n)
 
 cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_t njobs, uint32_t maxKeys,
                               uint32_t* disps, uint32_t* tables, uint32_t* out, cudaStream_t stream,
-                              uint32_t* gscratch)
+                              uint32_t* gscratch, uint32_t batch)
 {
     if (njobs == 0) return cudaSuccess;
     if (maxKeys > kHashGlobalBlockMaxKeys || (maxKeys > kHashBlockMaxKeys && !gscratch)) return cudaErrorInvalidValue;
@@ -686,10 +693,23 @@ cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_
         return cudaLaunchKernelEx(&cfg, k, keys, jobs, disps, tables, out, gscratch);
     };
     if (maxKeys <= kHashBlockMaxKeys) return launch(k_hash_block<1>, 1u, false);
+    // The CTAs a BVH's buckets need (2 a thread), or more where the batch leaves SMs idle:
+    // 144 CTAs at once (9 clusters of 16).  A store of 1,129 BVHs, 387 of them for
+    // clusters, builds in 12.2 ms; with clusters of 16 for all 23.7 ms, with one CTA a
+    // BVH 20.8 ms.  One such BVH alone is fastest with 16 (39,199 keys: 1.8 ms, 16.1 ms
+    // with one CTA).
+    const uint32_t room = 144u / std::max(batch, njobs);
+    switch (std::max(nb / 2048u, std::min(bit_floor_u32(std::max(room, 1u)), 16u)))
+    {
+    case 0: case 1: case 2: return launch(k_hash_block<2>, 2u, false);
+    case 4: return launch(k_hash_block<4>, 4u, false);
+    case 8: return launch(k_hash_block<8>, 8u, false);
+    default: break;
+    }
     // clusters of 16 are outside the portable size: where none fits on the device, 8
     if (launch(k_hash_block<16>, 16u, true) == cudaSuccess) return launch(k_hash_block<16>, 16u, false);
     cudaGetLastError();
-    return launch(k_hash_block<8>, 8u, false);
+    return launch(k_hash_block<8, 4>, 8u, false);
 }
 
 }  // namespace cgs

@@ -202,14 +202,17 @@ constexpr uint32_t kHashBlockMaxKeys = 8192;          // one CTA, everything in 
 constexpr uint32_t kHashGlobalBlockMaxKeys = 131072;  // a cluster of CTAs, buckets in global memory
 // Global scratch words of a BVH of n keys (above kHashBlockMaxKeys).
 uint64_t hash_block_scratch_words(uint32_t n);
+// Its hash buckets, a power of two: what a launch of hash_build_blocks sizes its clusters by.
+uint32_t hash_block_buckets(uint32_t n);
 // Builds every job's table, one CTA or cluster each, in one launch (asynchronous):
 // all jobs at most kHashBlockMaxKeys keys, or all in
 // (kHashBlockMaxKeys, kHashGlobalBlockMaxKeys] with gscratch.  out[8 j ..]:
 // status (0 ok, 3 no trial found a table, 4 bucket overflow, 5 duplicate
 // slot), A, B, N, mask, trial -- the values hash_build_device returns.
+// batch: the jobs of all launches of this batch, where there are several.
 cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_t njobs, uint32_t maxKeys,
                               uint32_t* disps, uint32_t* tables, uint32_t* out, cudaStream_t stream,
-                              uint32_t* gscratch = nullptr);
+                              uint32_t* gscratch = nullptr, uint32_t batch = 0);
 
 // Deterministic perfect hash of keys[0..n).  A[], B[] are the 16 trials'
 // coefficients, drawn on the host.  Writes disp[displSize] and

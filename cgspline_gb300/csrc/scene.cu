@@ -567,7 +567,7 @@ int hash_all(cgs_scene* sc, cudaStream_t stream)
 {
     const uint32_t nb = sc->nbvh();
     std::vector<uint32_t> small, mid, large;
-    uint32_t maxSmall = 1, maxMid = 1, maxLarge = 1;
+    uint32_t maxSmall = 1, maxLarge = 1;
     size_t blockKeys = 0;
     uint64_t midScratch = 0;
     for (uint32_t k = 0; k < nb; k++)
@@ -577,13 +577,14 @@ int hash_all(cgs_scene* sc, cudaStream_t stream)
         else if (n <= kHashGlobalBlockMaxKeys)
         {
             mid.push_back(k);
-            maxMid = std::max(maxMid, n);
             blockKeys += n;
             midScratch += hash_block_scratch_words(n) + 1;
         }
         else { large.push_back(k); maxLarge = std::max(maxLarge, n); }
     }
     CGS_TRY(sc->keys.reserve(std::max<size_t>({blockKeys, size_t(maxLarge), 1})));
+    std::stable_sort(mid.begin(), mid.end(),
+                     [&](uint32_t a, uint32_t b) { return sc->bvh(a).keys.size() > sc->bvh(b).keys.size(); });
     if (!small.empty() || !mid.empty())
     {
         std::vector<uint32_t> hk;
@@ -627,10 +628,15 @@ int hash_all(cgs_scene* sc, cudaStream_t stream)
                                       dOut, stream));
             sc->launches += 1;
         }
-        if (!mid.empty())
+        // the mid BVHs' launches: one for each number of buckets, the largest first
+        for (size_t i = 0, e = 0; i < mid.size(); i = e)
         {
-            CGS_TRY(hash_build_blocks(sc->keys.p, dj + small.size(), uint32_t(mid.size()), maxMid, sc->disps.p,
-                                      sc->tables.p, dOut + 8 * small.size(), stream, sc->scratch32.p));
+            const uint32_t maxKeys = uint32_t(sc->bvh(mid[i]).keys.size());
+            for (e = i; e < mid.size(); e++)
+                if (hash_block_buckets(uint32_t(sc->bvh(mid[e]).keys.size())) != hash_block_buckets(maxKeys)) break;
+            CGS_TRY(hash_build_blocks(sc->keys.p, dj + small.size() + i, uint32_t(e - i), maxKeys, sc->disps.p,
+                                      sc->tables.p, dOut + 8 * (small.size() + i), stream, sc->scratch32.p,
+                                      uint32_t(mid.size())));
             sc->launches += 1;
         }
         std::vector<uint32_t> res(8 * jobs.size());

@@ -1,6 +1,6 @@
 """The perfect-hash build at the edges of its three forms (one thread block,
-one cluster, many launches), on keys in a shuffled order, against the oracle:
-key sets that need several trials, key sets that no trial places, and a bucket
+one cluster, many launches), on keys in a shuffled order, and in stores of many
+BVHs that share the device, against the oracle: key sets that need several trials, key sets that no trial places, and a bucket
 that overflows."""
 import numpy as np
 import pytest
@@ -41,3 +41,24 @@ def test_bucket_overflow_is_reported(n):
     keys = np.arange(1, n + 1, dtype=np.uint32)
     keys[:5] = np.uint32(1 << 20) * np.arange(1, 6, dtype=np.uint32) + np.uint32(7)  # five keys of one bucket
     assert build(keys)[1] == 5  # CGS_ERR_HASH_BUCKET_OVERFLOW
+
+
+# 77 BVHs of 9,247 to 69,937 keys: clusters of 2, 4, 8 and 16; 12 of them: 8 or 16 for all.
+@pytest.mark.parametrize("sides", [[68] * 74 + [187, 92, 137], [68] * 9 + [92, 187, 137]])
+def test_stores_of_many_bvhs_match_the_oracle(sides, oracle_mod):
+    from cgspline_gb300 import rt
+    fields = {n: S.heightfield(n, n=n) for n in sorted(set(sides))}
+    l2w, w2l = S.IDENTITY16.copy(), S.IDENTITY16.copy()
+    sc = S.Scene([fields[n] for n in sides], [S.Object(k, l2w, w2l) for k in range(len(sides))], S.scene_c1().lights,
+                 name="fields")
+    g = rt.GpuScene(sc)
+    want = {}
+    for k, n in enumerate(sides):
+        b = g.bvh(k)
+        if n not in want:
+            want[n] = oracle_mod.hash_build(b["keys"])
+            assert want[n]["status"] == 0
+        o = want[n]
+        assert (b["A"], b["B"], b["N"], b["mask"]) == (o["A"], o["B"], o["N"], o["mask"])
+        assert np.array_equal(b["disp"], o["disp"]) and np.array_equal(b["table"][:o["N"]], o["table"][:o["N"]])
+    g.close()
