@@ -55,8 +55,7 @@ __device__ __forceinline__ void subV_d(double2* p, double a, double b)
 }
 
 // triangleOriginIntersection with the FP64 restatement's determinant floor
-// 2^-200 (xAxisIntersection and the fat-line bounds in double are shared
-// with the FP32 search's near-grazing variant).
+// 2^-200.
 __device__ __forceinline__ bool tri_origin_d(double2& coord, double2 P, double2 A, double2 B)
 {
     const double2 p = A - P, q = B - P;
@@ -80,7 +79,7 @@ __device__ __forceinline__ bool polish_full(const float4* P, double3 o, double3 
     for (int it = 0; it < 12; it++)
     {
         double3 Sp, Su, Sv;
-        surface_d(P, U, V, Sp, Su, Sv);
+        surface_full(P, U, V, Sp, Su, Sv);
         const double3 mF = make_double3(o.x + T * d.x - Sp.x, o.y + T * d.y - Sp.y, o.z + T * d.z - Sp.z);
         const double3 svxc = cross_d(Sv, c);
         const double det = dot_d(Su, svxc);
@@ -107,7 +106,7 @@ struct Sink64
     __device__ __forceinline__ bool operator()(double2 e)
     {
         double3 Sp, Su, Sv;
-        surface_d(P, e.x, e.y, Sp, Su, Sv);
+        surface_full(P, e.x, e.y, Sp, Su, Sv);
         const double3 V = sub3(Sp, o);
         if (dot_d(V, d) <= 0.0) return false;
         double uu = e.x, vv = e.y, tt = len3d(V);
@@ -158,7 +157,7 @@ __device__ __noinline__ bool clip64(Sink64& sink, double tol, LocalCounters& lc)
         else
         {
             double lower, upper;
-            clip_range_d([&](int i) { return buf[i]; }, cutside, lower, upper);
+            clip_range_full(buf, cutside, lower, upper);
             const double delta = upper - lower;
             if (delta > 0.8)
             {

@@ -11,7 +11,7 @@ namespace {
 
 // One thread per ray, the whole search inline (the reference's per-ray
 // kernel shape, src/rt/RayTracer.cu:171-274): the plain query path.
-__global__ void __launch_bounds__(128) k_query_plain(DevScene S, RaysSoA rays, uint32_t n, uint32_t group0,
+__global__ void __launch_bounds__(128, 3) k_query_plain(DevScene S, RaysSoA rays, uint32_t n, uint32_t group0,
                                                      Query q, bool any, HitsSoA hits, Counters* cnt)
 {
     LocalCounters lc;
