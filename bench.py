@@ -812,10 +812,10 @@ def main():
                                                   f"{cap or 'no'} blocks per SM)"},
                              "per_ray": {"nodes": kc["nodes"] / nprim, "hash_lookups": kc["hash_lookups"] / nprim,
                                          "hash_table_reads": kc["hash_table_reads"] / nprim},
-                             "note": "the 6.6 MB scene is L2-resident and the node reads are served by L1/L2: "
-                                     "ncu shows the L1 data pipe as the busiest unit, so the algorithmic bytes "
-                                     "(28 B per ray, 64 B per inner-node visit, 8 B per backtrack) are set against "
-                                     "the measured L1 load bandwidth; the other roofs follow",
+                             "note": "the scene is L2-resident and the node reads are served by L1/L2, so the "
+                                     "algorithmic bytes (28 B per ray, 64 B per inner-node visit, 8 B per backtrack) "
+                                     "are set against the measured L1 load bandwidth; ncu shows instruction issue "
+                                     "(75%) and node-load latency as what holds the walk; the other roofs follow",
                              "l2": {"peak": onchip["l2_gbs"], "unit": "GB/s", "frac": achieved / onchip["l2_gbs"],
                                     "note": "algorithmic bytes against the L2 roof (an upper bound on the L2 "
                                             "share: part of them hit in L1)"},

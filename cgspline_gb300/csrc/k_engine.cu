@@ -44,8 +44,10 @@
 //     ancestor in the reference tree comes first.  The ancestor's key is the
 //     common prefix of the leaves' heap keys, and the perfect hash finds its
 //     node.  (Any-hit answers do not depend on the order.)
-//   * an object whose patches do not fit in the chunk is collected again on the
-//     reference tree, which parks the ray exactly where it would have parked.
+//   * an object whose patches do not fit in the chunk sends the ray's list to one
+//     of a few long lists; where none is left or that fills too, the object is
+//     collected again on the reference tree, which parks the ray exactly where it
+//     would have parked.
 //
 // Both kernels refill lanes one ray (k_collect) or one clip iteration
 // (the search kernels) at a time, so heavy-tailed per-ray work does not idle the other

@@ -561,8 +561,8 @@ int upload(cgs_scene* sc) { return upload_store(sc); }
 // BVHs of at most kHashBlockMaxKeys keys (most: one per surface) are built
 // together, one CTA each, in one launch; those of at most
 // kHashGlobalBlockMaxKeys by a cluster of CTAs and a global scratch area each,
-// in a second launch; one host round trip reads both launches'
-// results.  Larger BVHs run the multi-launch build one at a time.
+// in a launch for each number of buckets; one host round trip reads all these
+// launches' results.  Larger BVHs run the multi-launch build one at a time.
 int hash_all(cgs_scene* sc, cudaStream_t stream)
 {
     const uint32_t nb = sc->nbvh();

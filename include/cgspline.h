@@ -310,7 +310,9 @@ int cgs_camera_rays(const cgs_camera* camera, uint32_t width, uint32_t height, i
 /* Runtime settings of the query engine (no counterpart in the reference):
  * collect / resolve passes before the inline fallback (1..8), block sizes
  * (collect 128 or 256, resolve 64 or 128) and resident blocks per SM
- * (0 = as many as fit, else at most 32).  Process-wide. */
+ * (0 = as many as fit, else at most 32).  Process-wide.  A query of at most
+ * 65,536 rays (32,768 for subdivision) runs whole in one launch, one warp to a
+ * block: the pass count, block sizes and occupancies do not apply to it. */
 typedef struct cgs_engine_config {
     int passes;
     int collect_threads;
@@ -323,7 +325,7 @@ typedef struct cgs_engine_config {
      * goes through the perfect hash, as in BVH::hashIntersect.  Both visit
      * the same nodes in the same order and give the same hits. */
     int backtrack_cache;
-    /* 1: the traversal kernel reads a 32-byte compressed copy of each BVH
+    /* 1: the traversal kernel reads a 32-byte compressed copy of each walked BVH
      * node (child boxes on an 8-bit grid of the node's box, widened outward
      * so that they contain the exact boxes); 0 (default): the exact 64-byte
      * records.  The compressed boxes are met wherever the exact ones are, so
