@@ -13,6 +13,7 @@ namespace cgs {
 constexpr uint32_t EMPTY = 0xFFFFFFFFu;
 constexpr int kClipStack = 32;          // reference stack depth, src/Spline_BezierClipping.cu:577
 constexpr int kMaxClipIterations = 4096;
+constexpr int kMaxBisections = 4 * kMaxClipIterations;  // of a subdivision search
 constexpr int kMaxTraversalSteps = 1 << 20;
 constexpr float kPi = 3.14159265358979323846f;
 constexpr float kInvPi = 0.318309886183790671538f;
@@ -896,6 +897,7 @@ struct ClipState
     float2 buf[16];
     float2 emin, emax;
     int cutsideStack, sl, it;
+    int base;  // the search's stack entries are those from here on: what lies below was lent to other lanes
     float tol;
     bool found, b64;  // b64: FP64 projection and fat-line bounds (near-grazing)
     bool fresh;       // the next projection is the search's first
@@ -921,6 +923,7 @@ __device__ __forceinline__ void clip_begin(ClipState& c, const HitSink& sink, fl
     c.emax = make_float2(1.0f, 1.0f);
     c.cutsideStack = 0;
     c.sl = 0;
+    c.base = 0;
     c.it = 0;
     c.found = false;
 }
@@ -963,7 +966,14 @@ __device__ __forceinline__ void transpose_if(float2* p, bool t)
 // in hand, which end in a cut or, below the tolerance, in a root and a pop.
 // clip_patch runs them in order for one thread's search; k_clip interleaves
 // those of a warp's searches, a part at a time.
-enum ClipNext : int { kClipOver, kClipProject, kClipCut, kClipRoot };
+// From kClipOver on the search has ended, at kClipLimit and kClipFull early: at
+// its iteration limit or with its stack full (limit_error).
+enum ClipNext : int { kClipProject, kClipCut, kClipRoot, kClipOver, kClipLimit, kClipFull };
+
+__device__ __forceinline__ uint32_t limit_error(ClipNext end)
+{
+    return end == kClipLimit ? kErrClipIterations : end == kClipFull ? kErrClipStack : 0u;
+}
 
 // The largest float whose square root is below tol: sqrtf(x) < tol as x <= bound.
 __device__ __forceinline__ float below_sqrt(float tol)
@@ -980,7 +990,7 @@ __device__ __forceinline__ float below_sqrt(float tol)
 template<bool kG64> __device__ __forceinline__ ClipNext clip_test(ClipState& c, float tol2, LocalCounters& lc)
 {
     if (kG64 && c.b64 && c.it >= kGrazeIterations) return kClipOver;
-    if (c.it++ >= kMaxClipIterations) { lc.errors |= kErrClipIterations; return kClipOver; }
+    if (c.it++ >= kMaxClipIterations) return kClipLimit;
     lc.iterations++;
     // the diagonals (the corners p3 and p12 swapped where the net is transposed: the same length)
     const float2 e = c.buf[3] - c.buf[12], f = c.buf[15] - c.buf[0];
@@ -991,7 +1001,7 @@ template<bool kG64> __device__ __forceinline__ ClipNext clip_test(ClipState& c, 
 __device__ __forceinline__ ClipNext clip_pop(ClipState& c, const float4* st)
 {
     c.cutsideStack >>= 1;
-    if (--c.sl < 0) return kClipOver;
+    if (--c.sl < c.base) return kClipOver;
     const float4 e = st[c.sl];
     c.emin = make_float2(e.x, e.y);
     c.emax = make_float2(e.z, e.w);
@@ -1021,8 +1031,9 @@ template<bool kG64> __device__ __forceinline__ void clip_project(ClipState& c, c
 // Cuts the net along u or v to its fat line's range, halves it where the range
 // is wide, drops it where it is empty.  kClipCut: the net in hand is new.
 // A cut along v leaves the net transposed (c.tposed); the next cut transposes
-// it only if it needs the other orientation.
-template<bool kG64, bool kFull = false> __device__ __forceinline__ ClipNext clip_cut(ClipState& c, float4* st, LocalCounters& lc)
+// it only if it needs the other orientation.  room: how many intervals the
+// stack may hold.
+template<bool kG64, bool kFull = false> __device__ __forceinline__ ClipNext clip_cut(ClipState& c, float4* st, int room)
 {
     const bool tr = (c.cutsideStack & 1) != 0;  // this cut is along v
     transpose_if(c.buf, tr != c.tposed);
@@ -1041,7 +1052,7 @@ template<bool kG64, bool kFull = false> __device__ __forceinline__ ClipNext clip
                                  : make_float4(c.emin.x, c.emin.y, h, c.emax.y);
         if (tr) c.emin.y = h; else c.emin.x = h;
         c.cutsideStack = tr ? ((c.cutsideStack << 1) & ~3) : ((c.cutsideStack << 1) | 3);
-        if (c.sl >= kClipStack) { lc.errors |= kErrClipStack; return kClipOver; }
+        if (c.sl >= room) return kClipFull;
         st[c.sl++] = pushed;
         a = 0.5f; b = 1.0f;
     }
@@ -1086,14 +1097,15 @@ static __device__ __noinline__ bool clip_patch(HitSink& sink, float tol, float g
         next = clip_test<true>(c, tol2, lc);
     }
     // A pass is an iteration for every lane: a root and the pop after it as well as a cut.
-    while (next != kClipOver)
+    while (next < kClipOver)
     {
         if (next == kClipRoot) next = clip_root(c, st, sink);
-        else if (next == kClipCut) next = clip_cut<true, true>(c, st, lc);
-        if (next == kClipOver || (anyHit && c.found)) break;
+        else if (next == kClipCut) next = clip_cut<true, true>(c, st, kClipStack);
+        if (next >= kClipOver || (anyHit && c.found)) break;
         if (next == kClipProject) clip_project<true>(c, sink, net0);
         next = clip_test<true>(c, tol2, lc);
     }
+    lc.errors |= limit_error(next);
     return c.found;
 }
 
@@ -1155,8 +1167,7 @@ __device__ __forceinline__ ClipNext subdiv_back(ClipState& c)
 // clipping search, so a warp's lanes cut together whatever their levels.
 __device__ __forceinline__ ClipNext subdiv_cut(ClipState& c, float tol2, LocalCounters& lc)
 {
-    if (c.it >= 4 * kMaxClipIterations) { lc.errors |= kErrClipIterations; return kClipOver; }
-    c.it++;
+    if (c.it++ >= kMaxBisections) return kClipLimit;
     lc.iterations++;
     float2 bmin = c.buf[0], bmax = c.buf[0];
 #pragma unroll
@@ -1196,7 +1207,7 @@ static __device__ __noinline__ bool subdiv_patch(HitSink& sink, float tol, Local
     bool reload = false, found = false;
     for (int it = 0;; it++)
     {
-        if (it >= 4 * kMaxClipIterations) { lc.errors |= kErrClipIterations; break; }
+        if (it >= kMaxBisections) { lc.errors |= kErrClipIterations; break; }
         lc.iterations++;
         const float su = ldexpf(1.0f, -((k + 1) >> 1)), sv = ldexpf(1.0f, -(k >> 1));
         const float2 emin = make_float2(float(tu) * su, float(tv) * sv);

@@ -767,6 +767,122 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_long(DevScene S, RaysSo
 }
 
 // ------------------------------------------------------------ resolve --
+// The tail of a launch is a few long searches.  A lane left without rays takes
+// the bottom (largest) pending interval of a search in its warp that holds
+// one or more, and searches it as that search would after popping it: the same
+// sub-net, derived from the projected net, and the same cut side.  The
+// intervals searched are the same, so the roots found are.  A closest-hit search
+// needs the nearest, and of roots at the same distance the first in the search's
+// order, so each lane of it keeps a range of order numbers: a lender keeps the
+// lower half of its own (what it lends comes last) and the borrower merges its
+// root under the first of its range.  The lane that has the ray, the owner, waits
+// for its borrowers at the end of the patch's search; an any-hit subdivision, which
+// needs one root of any patch, at the end of the ray's list.
+//
+// A search's limits (iterations, stack entries) hold for the whole of it, in its
+// order: the owner adds up the iterations of the parts, and where they pass the
+// limit, or where the stack would have held nearly all that fit, it drops what
+// the parts found and searches again alone, up to the limit: the patch, or the
+// ray's list for any hit.  So no answer depends on which lanes were idle.  (With a
+// limit for each lane's part queries took 1% less, and a search that reaches it
+// gave what its warp's idle lanes made of it.)
+//
+// An any-hit clipping search waits for nobody: whichever lane finds a root marks
+// the ray occluded (writes of "occluded" never clear it), and each part has the
+// limits to itself.  (Waiting: 640,001 shadow rays 1.75 ms for 1.55, a batch of
+// renders 6.5 ms for 4.3.)
+//
+// One warp's lanes that lend or borrow.  (Packed: the L1 cache has what the
+// blocks' shared memory leaves, and the searches' stacks live there.)
+template<bool kAny> struct Lend
+{
+    uint32_t sum[32];   // owner: lanes searching for it (bits 0-7), kFound, kOverLimit, iterations of ended parts
+    uint32_t who[32];   // a lane's owner (bits 0-7) and the log2 of its range of order numbers
+    uint32_t lo[32];    // the range's first
+    uint32_t rank[32];  // owner: the order number of the best root merged so far, EMPTY: none
+    float t[32], u[32], v[32];  // and the root
+};
+template<> struct Lend<true> { uint32_t sum[32], who[32]; };
+// The stack of a search in parts: one entry more would push a cut side's bit out of its word.
+constexpr int kPartsStack = 31;
+// kOverLimit: the search's parts together are past the limit, the others are to end.
+constexpr uint32_t kKids = 0xFFu, kFound = 0x100u, kOverLimit = 0x200u, kSpentShift = 10;
+// What a lane searches: a ray's patch of its own, with intervals lent (the owner),
+// an interval borrowed, or a patch again, alone.
+enum Role : int { kOwn, kLent, kThief, kAlone };
+// Where an owner is.
+enum LendEnd { kUnended, kEndedNothing, kEndedRoot, kEndedAgain };
+__device__ __forceinline__ bool in_parts(int role) { return role == kLent || role == kThief; }
+
+// Adds a lane's root to its owner's: the nearest is kept, the first in the
+// search's order at equal distances.
+__device__ __forceinline__ void lend_merge(Lend<false>& L, uint32_t o, uint32_t rank, const HitSink& sink)
+{
+    if (L.rank[o] == EMPTY || sink.dist < L.t[o] || (sink.dist == L.t[o] && rank < L.rank[o]))
+    {
+        L.t[o] = sink.dist; L.u[o] = sink.uv.x; L.v[o] = sink.uv.y; L.rank[o] = rank;
+    }
+}
+
+// Pairs idle lanes with lanes that have an interval to lend.  src: the lane a
+// borrower takes from.
+__device__ __forceinline__ void lend_pairs(unsigned idleM, unsigned richM, bool& borrows, bool& lends, int& src)
+{
+    const unsigned lane = lane_id(), below = (1u << lane) - 1u;
+    const int pairs = min(__popc(idleM), __popc(richM));
+    const int idleRank = __popc(idleM & below), richRank = __popc(richM & below);
+    borrows = ((idleM >> lane) & 1u) && idleRank < pairs;
+    lends = ((richM >> lane) & 1u) && richRank < pairs;
+    src = borrows ? int(__fns(richM, 0, idleRank + 1)) : int(lane);
+}
+
+// Whether a lane of this role may lend once more.
+template<bool kAny> __device__ __forceinline__ bool lend_may(const Lend<kAny>& L, int role)
+{
+    if constexpr (kAny) return role != kAlone;
+    else return role == kOwn || (in_parts(role) && (L.who[lane_id()] >> 8) != 0u);
+}
+// The lender's side of a loan, before its borrower reads the lender's entries.
+template<bool kAny> __device__ __forceinline__ void lend_give(Lend<kAny>& L, int& role)
+{
+    const uint32_t lane = lane_id();
+    if (role == kOwn)
+    {
+        L.sum[lane] = 0;
+        L.who[lane] = lane | (31u << 8);
+        if constexpr (!kAny) { L.lo[lane] = 0; L.rank[lane] = EMPTY; }
+        role = kLent;
+    }
+    atomicAdd(&L.sum[L.who[lane] & 0xFFu], 1u);
+}
+// The borrower's: the upper half of the lender's order range.
+template<bool kAny> __device__ __forceinline__ void lend_take(Lend<kAny>& L, int src, int& role)
+{
+    const uint32_t lane = lane_id(), who = L.who[src] - (kAny ? 0u : 1u << 8);
+    L.who[lane] = who;
+    if constexpr (!kAny)
+    {
+        L.who[src] = who;
+        L.lo[lane] = L.lo[src] + (1u << (who >> 8));
+    }
+    role = kThief;
+}
+
+// A borrower's ray and patch, from lane src (called by the whole warp).
+__device__ __forceinline__ void lend_ray(bool borrows, int src, HitSink& sink)
+{
+    const unsigned long long sp =
+        __shfl_sync(0xFFFFFFFFu, (unsigned long long)reinterpret_cast<uintptr_t>(sink.P), src);
+    const float3 so = f3(__shfl_sync(0xFFFFFFFFu, sink.o.x, src), __shfl_sync(0xFFFFFFFFu, sink.o.y, src),
+                         __shfl_sync(0xFFFFFFFFu, sink.o.z, src));
+    const float3 sd = f3(__shfl_sync(0xFFFFFFFFu, sink.d.x, src), __shfl_sync(0xFFFFFFFFu, sink.d.y, src),
+                         __shfl_sync(0xFFFFFFFFu, sink.d.z, src));
+    const float sdist = __shfl_sync(0xFFFFFFFFu, sink.dist, src);
+    if (!borrows) return;
+    sink.P = reinterpret_cast<const float4*>(uintptr_t(sp));
+    sink.o = so; sink.d = sd; sink.dist = sdist; sink.uv = make_float2(0.0f, 0.0f);
+}
+
 // One lane's ray: where it is in its list, and the best hit so far.  Shared by
 // the two search kernels below.
 template<bool kAny> struct ListWalk
@@ -861,10 +977,35 @@ template<bool kAny> struct ListWalk
         }
     }
 
-    // A closest-hit search of the patch ended with a closer root.
-    __device__ __forceinline__ void keep(const HitSink& sink)
+    // The search of the patch ended with a (closer) root.
+    __device__ __forceinline__ void keep(float t, float u, float v) { lt = t; lu = u; lv = v; lpatch = int32_t(patch); }
+    __device__ __forceinline__ void occlude(const Eng& E, int32_t* occluded) const
     {
-        lt = sink.dist; lu = sink.uv.x; lv = sink.uv.y; lpatch = int32_t(patch);
+        occluded[rid] = 0;
+        E.status[rid] = kFinished;
+        E.count[rid] = 0;
+    }
+    // Any hit: where the ray's borrowers have ended (true), the ray is over or starts its list again.
+    __device__ __forceinline__ bool settle(const Eng& E, int32_t* occluded, LendEnd end, bool& have)
+    {
+        if (end == kUnended) return false;
+        if (end == kEndedAgain)
+        {
+            k = 0;
+            obj = -1;
+            sweep = false;
+            return true;
+        }
+        have = false;
+        if (end == kEndedRoot) occlude(E, occluded);
+        else finish(E);
+        return true;
+    }
+    // Closest hit: the sink as next() left it; the patch is to be searched again.
+    __device__ __forceinline__ void again(const HitsSoA&, HitSink& sink) const
+    {
+        sink.dist = lt;
+        sink.uv = make_float2(lu, lv);
     }
     // The end of the ray's list.
     __device__ __forceinline__ void finish(const Eng& E) { E.count[rid] = 0; }
@@ -904,9 +1045,11 @@ struct PairWalk
         hits.patch[rid] = lpatch >= 0 ? 1 : 0;
         return false;
     }
-    __device__ __forceinline__ void keep(const HitSink& sink)
+    __device__ __forceinline__ void keep(float t, float u, float v) { lt = t; lu = u; lv = v; lpatch = int32_t(patch); }
+    __device__ __forceinline__ void again(const HitsSoA& hits, HitSink& sink) const
     {
-        lt = sink.dist; lu = sink.uv.x; lv = sink.uv.y; lpatch = int32_t(patch);
+        sink.dist = hits.t[rid];
+        sink.uv = make_float2(0.0f, 0.0f);
     }
     __device__ __forceinline__ void finish(const Eng&) {}
 };
@@ -927,105 +1070,83 @@ struct PairWalk
 // held to 128 registers, four 128-thread blocks per SM.
 enum : int { kPartWalk, kPartProject, kPartCut, kPartRoot, kPartBegin64, kPartCut64, kPartMerge, kPartWait, kPartNone };
 
-// The tail of a launch is a few long searches.  A lane left without rays takes
-// the bottom (largest) pending interval of a search in its warp that holds
-// one or more, and searches it as that search would after popping it: the same
-// sub-net, derived from the projected net, and the same cut side.  The
-// intervals searched are the same, so the roots found are.  An any-hit answer
-// needs one of them, and whichever lane finds it marks the ray occluded (writes
-// of "occluded" never clear it).  A closest-hit search needs the nearest, and of
-// roots at the same distance the first in the search's order, so each lane
-// of it keeps a range of order numbers: a lender keeps the lower half of its
-// own (what it lends comes last) and the borrower merges its root under the
-// first of its range.  The lane that has the ray waits for its borrowers.  (The
-// searches' iteration limits count per lane.)
-//
-// One warp's lanes that lend or borrow; the ray's lane is the owner.
-struct Lend
-{
-    uint32_t kids[32];   // owner: lanes searching for it
-    float t[32], u[32], v[32];
-    uint32_t rank[32];   // owner: the best root merged so far and its order number
-    uint32_t lo[32], hi[32], owner[32];  // a lane's order range and its owner
-};
-
-// The lane's first loan in a search of its own.
-__device__ __forceinline__ void lend_open(Lend& L, uint32_t lane)
-{
-    L.kids[lane] = 0; L.t[lane] = INFINITY; L.rank[lane] = 0;
-    L.lo[lane] = 0; L.hi[lane] = 0xFFFFFFFFu; L.owner[lane] = lane;
-}
-
-// Adds a lane's root to its owner's.
-__device__ __forceinline__ void lend_merge(Lend& L, uint32_t lane, const HitSink& sink)
-{
-    const uint32_t o = L.owner[lane], rank = L.lo[lane];
-    if (sink.dist < L.t[o] || (sink.dist == L.t[o] && rank < L.rank[o]))
-    {
-        L.t[o] = sink.dist; L.u[o] = sink.uv.x; L.v[o] = sink.uv.y; L.rank[o] = rank;
-    }
-}
-
-// Pairs idle lanes with lanes that have an interval to lend.  src: the lane a
-// borrower takes from.
-__device__ __forceinline__ void lend_pairs(unsigned idleM, unsigned richM, bool& borrows, bool& lends, int& src)
-{
-    const unsigned lane = lane_id(), below = (1u << lane) - 1u;
-    const int pairs = min(__popc(idleM), __popc(richM));
-    const int idleRank = __popc(idleM & below), richRank = __popc(richM & below);
-    borrows = ((idleM >> lane) & 1u) && idleRank < pairs;
-    lends = ((richM >> lane) & 1u) && richRank < pairs;
-    src = borrows ? int(__fns(richM, 0, idleRank + 1)) : int(lane);
-}
-
-// A borrower's ray and patch, from lane src (called by the whole warp).
-template<bool kAny> __device__ __forceinline__ void lend_ray(bool borrows, int src, HitSink& sink, uint32_t& rid)
-{
-    const uint32_t srid = __shfl_sync(0xFFFFFFFFu, rid, src);
-    const unsigned long long sp =
-        __shfl_sync(0xFFFFFFFFu, (unsigned long long)reinterpret_cast<uintptr_t>(sink.P), src);
-    const float3 so = f3(__shfl_sync(0xFFFFFFFFu, sink.o.x, src), __shfl_sync(0xFFFFFFFFu, sink.o.y, src),
-                         __shfl_sync(0xFFFFFFFFu, sink.o.z, src));
-    const float3 sd = f3(__shfl_sync(0xFFFFFFFFu, sink.d.x, src), __shfl_sync(0xFFFFFFFFu, sink.d.y, src),
-                         __shfl_sync(0xFFFFFFFFu, sink.d.z, src));
-    const float sdist = __shfl_sync(0xFFFFFFFFu, sink.dist, src);
-    if (!borrows) return;
-    rid = srid;
-    sink.P = reinterpret_cast<const float4*>(uintptr_t(sp));
-    sink.o = so; sink.d = sd; sink.dist = sdist; sink.uv = make_float2(0.0f, 0.0f);
-}
-
-// What the two search kernels share besides their searches: the borrowers' ends.
-// A lane whose search ended goes on to `part`; called by the whole warp.
-template<class Walk> __device__ __forceinline__ void lend_settle(Lend& L, int& part, bool& thief, bool& lent,
-                                                                 const HitSink& sink, bool found, Walk& w)
+// What the two search kernels share besides their searches: the ends of searches
+// in parts.  `it` is the iterations of a lane's part, above `limit` where it ended
+// at one of the search's limits.
+// Closest hits: lanes with their part at its end (kPartMerge); the owner's
+// patch ends with the last.  Called by the whole warp.
+__device__ __forceinline__ LendEnd lend_settle(Lend<false>& L, int& part, int& role, const HitSink& sink, bool found,
+                                               uint32_t it, uint32_t limit)
 {
     const uint32_t lane = lane_id();
-    for (unsigned m = __ballot_sync(0xFFFFFFFFu, part == kPartMerge); m; m &= m - 1)
+    unsigned m = __ballot_sync(0xFFFFFFFFu, part == kPartMerge);
+    while (m)
     {
-        if (lane == uint32_t(__ffs(m) - 1))
+        for (; m; m &= m - 1)
         {
-            if (found) lend_merge(L, lane, sink);
-            if (thief) { L.kids[L.owner[lane]]--; thief = false; part = kPartNone; }
-            else part = kPartWait;
+            if (lane == uint32_t(__ffs(m) - 1))
+            {
+                const uint32_t o = L.who[lane] & 0xFFu;
+                uint32_t sum = L.sum[o] - (role == kThief ? 1u : 0u);
+                if (!(sum & kOverLimit))
+                {
+                    sum += it << kSpentShift;
+                    if ((sum >> kSpentShift) > limit) sum |= kOverLimit;
+                    if (found) lend_merge(L, o, L.lo[lane], sink);
+                }
+                L.sum[o] = sum;
+                part = role == kThief ? kPartNone : kPartWait;
+                if (role == kThief) role = kOwn;
+            }
+            __syncwarp();
         }
-        __syncwarp();
+        // the other parts of a search that is past its limit end here
+        if (in_parts(role) && part >= kPartProject && part <= kPartRoot && (L.sum[L.who[lane] & 0xFFu] & kOverLimit))
+            part = kPartMerge;
+        m = __ballot_sync(0xFFFFFFFFu, part == kPartMerge);
     }
-    if (part == kPartWait && L.kids[lane] == 0)
+    LendEnd end = kUnended;
+    if (part == kPartWait && (L.sum[lane] & kKids) == 0)
     {
-        if (L.t[lane] < INFINITY)
-        {
-            w.lt = L.t[lane]; w.lu = L.u[lane]; w.lv = L.v[lane]; w.lpatch = int32_t(w.patch);
-        }
-        lent = false;
+        end = L.sum[lane] & kOverLimit ? kEndedAgain : L.rank[lane] != EMPTY ? kEndedRoot : kEndedNothing;
+        role = kOwn;
         part = kPartWalk;
     }
     __syncwarp();
+    return end;
+}
+// Any hit: a lane's part has ended.
+__device__ __forceinline__ void lend_end_part(Lend<true>& L, int& part, int& role, bool found, uint32_t it, uint32_t limit)
+{
+    uint32_t* sum = &L.sum[L.who[lane_id()] & 0xFFu];
+    // (an owner's searches after its first loan are counted together; past the limit the sum stands)
+    if ((*(volatile uint32_t*)sum >> kSpentShift) <= limit) atomicAdd(sum, it << kSpentShift);
+    if (found) atomicOr(sum, kFound);
+    if (role == kThief)
+    {
+        atomicSub(sum, 1u);
+        role = kOwn;
+        part = kPartNone;
+    }
+    else part = found ? kPartWait : kPartWalk;
+}
+// Any hit: an owner at the end of its list looks whether its borrowers are.
+__device__ __forceinline__ LendEnd lend_wait(const Lend<true>& L, int& role, uint32_t limit)
+{
+    const uint32_t sum = *(const volatile uint32_t*)&L.sum[lane_id()];
+    if (sum & kKids) return kUnended;
+    if ((sum >> kSpentShift) > limit)
+    {
+        role = kAlone;
+        return kEndedAgain;
+    }
+    role = kOwn;
+    return sum & kFound ? kEndedRoot : kEndedNothing;
 }
 
 template<bool kAny, bool kG64, class Source, class Walk>
 __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, int pass, const Query& q,
-                                          HitsSoA& hits, int32_t* occluded, const Source& src, Lend& L,
+                                          HitsSoA& hits, int32_t* occluded, const Source& src, Lend<kAny>& L,
                                           LocalCounters& lc, Walk w)
 {
     float4 stack[kClipStack];
@@ -1033,25 +1154,37 @@ __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays
     ClipState c;
     c.b64 = false;
     c.sl = 0;
+    c.base = 0;
     HitSink sink {nullptr, f3(0, 0, 0), f3(0, 0, 1), 0.0f, make_float2(0, 0)};
     int part = kPartWalk;
     bool have = false;   // the lane has a ray
-    bool thief = false;  // the lane searches an interval borrowed from another lane's search
-    bool lent = false;   // closest hit: the lane's search has lent intervals
+    int role = kOwn;
     const float tol2 = below_sqrt(q.tol), tol2graze = kG64 ? below_sqrt(kGrazeTol) : 0.0f;
     const uint32_t m = src.m;
     for (;;)
     {
         if constexpr (!kG64)
         {
-            if (!kAny && __ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
-                lend_settle(L, part, thief, lent, sink, c.found, w);
+            if constexpr (!kAny)
+            {
+                if (__ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
+                {
+                    const LendEnd end = lend_settle(L, part, role, sink, c.found, uint32_t(c.it), kMaxClipIterations);
+                    if (end == kEndedRoot) w.keep(L.t[lane_id()], L.u[lane_id()], L.v[lane_id()]);
+                    if (end == kEndedAgain)
+                    {
+                        w.again(hits, sink);
+                        clip_begin<kG64>(c, sink, q.tol, 0.0f);
+                        part = kPartProject;
+                        role = kAlone;
+                    }
+                }
+            }
             const unsigned idleM = __ballot_sync(0xFFFFFFFFu, part == kPartNone);
             if (idleM)
             {
-                const unsigned lane = lane_id();
-                bool rich = part >= kPartProject && part <= kPartRoot && c.sl >= 1 && c.sl <= 30;
-                if (!kAny && rich && (lent || thief)) rich = L.hi[lane] - L.lo[lane] >= 2u;
+                const bool rich = part >= kPartProject && part <= kPartRoot && c.sl > c.base && c.sl < kPartsStack &&
+                                  (kAny || lend_may(L, role));
                 const unsigned richM = __ballot_sync(0xFFFFFFFFu, rich);
                 if (richM)
                 {
@@ -1062,40 +1195,32 @@ __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays
                     int bit = 0;
                     if (lends)
                     {
-                        // entry i's cut side is bit (sl - i) of the bit stack; the
-                        // bits above the bottom entry's are clear
-                        e = stack[0];
-                        bit = (c.cutsideStack >> c.sl) & 1;
-                        c.cutsideStack &= ~(1 << c.sl);
-                        for (int i = 1; i < c.sl; i++) stack[i - 1] = stack[i];
-                        c.sl--;
-                        if (!kAny)
-                        {
-                            if (!lent && !thief) lend_open(L, lane);
-                            lent = lent || !thief;
-                            atomicAdd(&L.kids[L.owner[lane]], 1u);
-                        }
+                        // entry i's cut side is bit (sl - i) of the bit stack
+                        e = stack[c.base];
+                        bit = (c.cutsideStack >> (c.sl - c.base)) & 1;
+                        if constexpr (!kAny) lend_give(L, role);
                     }
+                    const int base = c.base;
+                    if (lends) c.base++;
                     __syncwarp();
                     const float4 se =
                         make_float4(__shfl_sync(0xFFFFFFFFu, e.x, src), __shfl_sync(0xFFFFFFFFu, e.y, src),
                                     __shfl_sync(0xFFFFFFFFu, e.z, src), __shfl_sync(0xFFFFFFFFu, e.w, src));
-                    const int sbit = __shfl_sync(0xFFFFFFFFu, bit, src);
-                    lend_ray<kAny>(borrows, src, sink, w.rid);
+                    const int sbit = __shfl_sync(0xFFFFFFFFu, bit, src), sbase = __shfl_sync(0xFFFFFFFFu, base, src);
+                    lend_ray(borrows, src, sink);
+                    if constexpr (kAny)
+                    {
+                        const uint32_t rid = __shfl_sync(0xFFFFFFFFu, w.rid, src);
+                        if (borrows) { w.rid = rid; role = kThief; }
+                    }
                     if (borrows)
                     {
-                        if (!kAny)
-                        {
-                            const uint32_t mid = L.lo[src] + (L.hi[src] - L.lo[src]) / 2;
-                            L.lo[lane] = mid; L.hi[lane] = L.hi[src]; L.owner[lane] = L.owner[src];
-                            L.hi[src] = mid;
-                        }
+                        if constexpr (!kAny) lend_take(L, src, role);
                         c.emin = make_float2(se.x, se.y);
                         c.emax = make_float2(se.z, se.w);
-                        c.cutsideStack = sbit; c.sl = 0; c.it = 0; c.tol = q.tol;
+                        c.cutsideStack = sbit; c.sl = sbase; c.base = sbase; c.it = 0; c.tol = q.tol;
                         c.found = false; c.b64 = false; c.fresh = false; c.tposed = false;
                         part = kPartProject;
-                        thief = true;
                     }
                     __syncwarp();
                 }
@@ -1126,6 +1251,7 @@ __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays
                 {
                     lc.candidates++;
                     clip_begin<kG64>(c, sink, q.tol, graze_sin(q.precision));
+                    if (!kG64 && !kAny) role = kOwn;
                     part = kG64 && c.b64 ? kPartBegin64 : kPartProject;
                 }
                 else
@@ -1152,35 +1278,31 @@ __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays
                 next = kClipCut;
             }
             else
-                next = clip_cut<kG64>(c, stack, lc);
+                next = clip_cut<kG64>(c, stack, !kG64 && !kAny && in_parts(role) ? kPartsStack : kClipStack);
             if (next == kClipCut) next = clip_test<kG64>(c, kG64 && c.b64 ? tol2graze : tol2, lc);
         }
         if (kAny && c.found) next = kClipOver;  // an any-hit search ends at its first root
-        if (next != kClipOver)
+        if (next < kClipOver)
         {
             part = next == kClipRoot ? kPartRoot
                    : next == kClipProject ? kPartProject : kG64 && c.b64 ? kPartCut64 : kPartCut;
             continue;
         }
-        part = kPartWalk;
-        if (!kAny)
+        if (!kG64 && !kAny && in_parts(role))
         {
-            if (!kG64 && (lent || thief)) part = kPartMerge;
-            else if (c.found) w.keep(sink);
+            // (a limit's error is raised by the search that runs to it alone)
+            if (next == kClipFull) c.it = kMaxClipIterations + 1;
+            part = kPartMerge;
             continue;
         }
-        if (c.found)
+        part = kPartWalk;
+        lc.errors |= limit_error(next);
+        if constexpr (kAny)
         {
-            occluded[w.rid] = 0;
-            E.status[w.rid] = kFinished;
-            E.count[w.rid] = 0;
-            have = false;
+            if (c.found) { w.occlude(E, occluded); have = false; }
+            if (role == kThief) { role = kOwn; part = kPartNone; }
         }
-        if (thief)
-        {
-            thief = false;
-            part = kPartNone;
-        }
+        else if (c.found) w.keep(sink.dist, sink.uv.x, sink.uv.y);
     }
 }
 
@@ -1189,7 +1311,7 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
                                                                          const uint32_t* nDev, Eng E, int pass, Query q,
                                                                          HitsSoA hits, int32_t* occluded, Counters* cnt)
 {
-    __shared__ Lend lend[kAny || kG64 ? 1 : kResolveThreads / 32];
+    __shared__ Lend<kAny> lend[kAny || kG64 ? 1 : kResolveThreads / 32];
     LocalCounters lc;
     clip_rays<kAny, kG64>(S, rays, E, pass, q, hits, occluded, PassSource<1>(E, pass, n0, nDev),
                           lend[kAny || kG64 ? 0 : threadIdx.x / 32], lc, ListWalk<kAny> {});
@@ -1206,29 +1328,43 @@ __global__ void __launch_bounds__(kResolveThreads, kG64 ? 3 : 4) k_clip(DevScene
 template<bool kAny, class Source, class Walk>
 __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA& rays, const Eng& E, int pass,
                                                const Query& q, HitsSoA& hits, int32_t* occluded, const Source& src,
-                                               Lend& L, LocalCounters& lc, Walk w)
+                                               Lend<kAny>& L, LocalCounters& lc, Walk w)
 {
     ClipState c;
     HitSink sink {nullptr, f3(0, 0, 0), f3(0, 0, 1), 0.0f, make_float2(0, 0)};
     int part = kPartWalk;
-    bool have = false, thief = false, lent = false;
+    bool have = false;
+    int role = kOwn;
     const float tol2 = below_sqrt(q.tol);
     c.sl = 0;
     c.found = false;
     const uint32_t m = src.m;
     for (;;)
     {
-        if (!kAny && __ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
-            lend_settle(L, part, thief, lent, sink, c.found, w);
+        if constexpr (kAny)
+        {
+            if (part == kPartWait && w.settle(E, occluded, lend_wait(L, role, kMaxBisections), have))
+                part = kPartWalk;
+        }
+        else if (__ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
+        {
+            const LendEnd end = lend_settle(L, part, role, sink, c.found, uint32_t(c.it), kMaxBisections);
+            if (end == kEndedRoot) w.keep(L.t[lane_id()], L.u[lane_id()], L.v[lane_id()]);
+            if (end == kEndedAgain)
+            {
+                w.again(hits, sink);
+                subdiv_begin(c);
+                part = kPartProject;
+                role = kAlone;
+            }
+        }
         const unsigned idleM = __ballot_sync(0xFFFFFFFFu, part == kPartNone);
         if (idleM)
         {
-            const unsigned lane = lane_id();
             // level j's bit of the trail is bit k - 1 - j: the first level with a 0 bit
             const uint32_t trail = uint32_t(c.cutsideStack);
             const int k = c.sl, j = k > 0 ? __clz(~(trail << (32 - k))) : 0;
-            bool rich = part >= kPartProject && part <= kPartRoot && j < k;
-            if (!kAny && rich && (lent || thief)) rich = L.hi[lane] - L.lo[lane] >= 2u;
+            const bool rich = part >= kPartProject && part <= kPartRoot && j < k && lend_may(L, role);
             const unsigned richM = __ballot_sync(0xFFFFFFFFu, rich);
             if (richM)
             {
@@ -1244,31 +1380,20 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
                     tv = (tv >> (k / 2 - (j + 1) / 2)) | (j % 2 == 0 ? 0u : 1u);
                     level = j + 1;
                     c.cutsideStack = int(trail | (1u << (k - 1 - j)));
-                    if (!kAny)
-                    {
-                        if (!lent && !thief) lend_open(L, lane);
-                        lent = lent || !thief;
-                        atomicAdd(&L.kids[L.owner[lane]], 1u);
-                    }
+                    lend_give(L, role);
                 }
                 __syncwarp();
                 const uint32_t su = __shfl_sync(0xFFFFFFFFu, tu, src), sv = __shfl_sync(0xFFFFFFFFu, tv, src);
                 const int sk = __shfl_sync(0xFFFFFFFFu, level, src);
-                lend_ray<kAny>(borrows, src, sink, w.rid);
+                lend_ray(borrows, src, sink);
                 if (borrows)
                 {
-                    if (!kAny)
-                    {
-                        const uint32_t mid = L.lo[src] + (L.hi[src] - L.lo[src]) / 2;
-                        L.lo[lane] = mid; L.hi[lane] = L.hi[src]; L.owner[lane] = L.owner[src];
-                        L.hi[src] = mid;
-                    }
+                    lend_take(L, src, role);
                     // every level above is done here: the trail is all ones
                     c.cutsideStack = int(sk < 32 ? (1u << sk) - 1u : 0xFFFFFFFFu);
                     c.sl = sk; c.it = 0; c.fresh = true; c.found = false;
                     c.emin = make_float2(__uint_as_float(su), __uint_as_float(sv));
                     part = kPartProject;
-                    thief = true;
                 }
                 __syncwarp();
             }
@@ -1290,6 +1415,7 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
             {
                 if (idx < m) have = w.take(rays, E, pass, src.ray(idx), lc);
                 else part = kPartNone;
+                if (kAny) role = kOwn;
             }
             if (part == kPartWalk && have)
             {
@@ -1297,8 +1423,10 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
                 {
                     lc.candidates++;
                     subdiv_begin(c);
+                    if (!kAny) role = kOwn;
                     part = kPartProject;
                 }
+                else if (kAny && role == kLent) part = kPartWait;
                 else
                 {
                     have = false;
@@ -1317,30 +1445,22 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
             for (int s = 0; s < int(E.subdivLevels) && next == kClipCut; s++) next = subdiv_cut(c, tol2, lc);
         }
         if (kAny && c.found) next = kClipOver;  // an any-hit search ends at its first root
-        if (next != kClipOver)
+        if (next < kClipOver)
         {
             part = next == kClipRoot ? kPartRoot : next == kClipProject ? kPartProject : kPartCut;
             continue;
         }
-        part = kPartWalk;
-        if (!kAny)
+        if (in_parts(role))
         {
-            if (lent || thief) part = kPartMerge;
-            else if (c.found) w.keep(sink);
+            if constexpr (kAny) lend_end_part(L, part, role, c.found, uint32_t(c.it), kMaxBisections);
+            else part = kPartMerge;
             continue;
         }
-        if (c.found)
-        {
-            occluded[w.rid] = 0;
-            E.status[w.rid] = kFinished;
-            E.count[w.rid] = 0;
-            have = false;
-        }
-        if (thief)
-        {
-            thief = false;
-            part = kPartNone;
-        }
+        part = kPartWalk;
+        lc.errors |= limit_error(next);
+        if (!c.found) continue;
+        if constexpr (kAny) { w.occlude(E, occluded); have = false; }
+        else w.keep(sink.dist, sink.uv.x, sink.uv.y);
     }
 }
 
@@ -1349,10 +1469,10 @@ __global__ void __launch_bounds__(kResolveThreads, 4) k_subdivide(DevScene S, Ra
                                                                   const uint32_t* nDev, Eng E, int pass, Query q,
                                                                   HitsSoA hits, int32_t* occluded, Counters* cnt)
 {
-    __shared__ Lend lend[kAny ? 1 : kResolveThreads / 32];
+    __shared__ Lend<kAny> lend[kResolveThreads / 32];
     LocalCounters lc;
     subdivide_rays<kAny>(S, rays, E, pass, q, hits, occluded, PassSource<1>(E, pass, n0, nDev),
-                         lend[kAny ? 0 : threadIdx.x / 32], lc, ListWalk<kAny> {});
+                         lend[threadIdx.x / 32], lc, ListWalk<kAny> {});
     flush_counters(cnt, lc, 0);
 }
 
@@ -1539,7 +1659,7 @@ __global__ void __launch_bounds__(32, 8) k_small(DevScene S,
 {
     __shared__ uint32_t ring[kRing * 32], fetch;
     static_assert(kRing * 32 >= kPolishList);
-    __shared__ Lend lend;
+    __shared__ Lend<kAny> lend;
     const uint32_t n = nDev ? *nDev : n0, lane = threadIdx.x;
     const uint32_t share = (n + gridDim.x - 1) / gridDim.x, base = blockIdx.x * share;
     if (base >= n) return;
@@ -1599,7 +1719,7 @@ __global__ void __launch_bounds__(32, 16) k_pairs(DevScene S, RaysSoA rays, uint
                                                   Counters* cnt)
 {
     __shared__ uint32_t fetch;
-    __shared__ Lend lend;
+    __shared__ Lend<false> lend;
     const uint32_t lane = threadIdx.x, share = (n + gridDim.x - 1) / gridDim.x, base = blockIdx.x * share;
     if (base >= n) return;
     const WarpSource src {&fetch, min(share, n - base), base, nullptr};

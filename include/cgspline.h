@@ -135,9 +135,11 @@ typedef struct cgs_counters {
                                  BVH::hashIntersect) */
     uint64_t candidates;      /* (ray, patch) pairs searched */
     uint64_t iterations;      /* clip / subdivision iterations */
-    uint64_t device_errors;   /* bit mask: 1 clip stack full, 2 clip iteration limit,
-                                 4 traversal step limit, 8 ray of an unknown group,
-                                 16 a patch id past its surface's patch count */
+    uint64_t device_errors;   /* bit mask: 1 clip stack full, 2 iteration limit of a patch's
+                                 search (4,096 clipping iterations or 16,384 bisections: it
+                                 ends with the roots it has; an any-hit clipping search may
+                                 go on past it), 4 traversal step limit, 8 ray of an unknown
+                                 group, 16 a patch id past its surface's patch count */
     uint64_t kernel_launches;
     uint64_t hash_table_reads; /* backtracks answered through the perfect hash; the rest
                                   came from the traversal's backtrack cache */

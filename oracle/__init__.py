@@ -48,6 +48,7 @@ def set_graze64_ray(on: int):
     FP32 one (0)."""
     lib().ora_set_graze64_ray(int(on))
 GRAZE_5, GRAZE_30 = 0.0871557427, 0.5
+SEARCH_LIMITS = (4096, 16384)  # the GPU's FP32 searches: clipping iterations, bisections
 FP32, FP32_POLISH64, FP64 = 0, 1, 2
 
 
@@ -83,6 +84,7 @@ def lib():
         L.ora_scene_build.argtypes = [P]
         L.ora_scene_set_split.argtypes = [P, C.c_int]
         L.ora_set_graze_sin.argtypes = [C.c_float]
+        L.ora_set_search_limits.argtypes = [C.c_uint64, C.c_uint64]
         L.ora_philox.argtypes = [u32, C.c_uint32, C.c_uint32]
         L.ora_bvh_sizes.argtypes = [P, C.c_int, u32]
         L.ora_bvh_export.argtypes = [P, C.c_int, u32, u32, u32, u32, u32, u32]
@@ -170,11 +172,14 @@ class OracleScene:
                     A=int(par[0]), B=int(par[1]), N=int(par[2]), mask=int(par[3]))
 
     def intersect(self, rays, method=CLIP_HOST, precision=FP32, tol=2.0 ** -12, tol64=1e-9, any_hit=False,
-                  nthreads=None, counters=False, graze_sin=GRAZE_30):
+                  nthreads=None, counters=False, graze_sin=GRAZE_30, search_limits=(0, 0)):
         """graze_sin: the grazing margin of CLIP_GRAZE64 (GRAZE_5 restates the
-        GPU's FP32_POLISH64 level, GRAZE_30 its FP32_GRAZE64 level)."""
+        GPU's FP32_POLISH64 level, GRAZE_30 its FP32_GRAZE64 level).
+        search_limits: iterations after which a clipping / subdivision search
+        of a patch ends with the roots it has (the GPU's: SEARCH_LIMITS; 0: none)."""
         L = lib()
         L.ora_set_graze_sin(graze_sin)
+        L.ora_set_search_limits(*search_limits)
         rays = np.ascontiguousarray(rays, np.float32)
         n = rays.shape[1]
         of = np.zeros((3, n), np.float32)
@@ -182,6 +187,7 @@ class OracleScene:
         cnt = np.zeros(8, np.uint64) if counters else None
         nt = nthreads or os.cpu_count() or 1
         r = L.ora_intersect(self.h, rays, n, method, precision, tol, tol64, int(any_hit), of, oi, _ptr(cnt), nt)
+        L.ora_set_search_limits(0, 0)
         if r:
             raise RuntimeError(f"ora_intersect failed ({r})")
         out = dict(t=of[0], u=of[1], v=of[2], patch=oi[0], object=oi[1])

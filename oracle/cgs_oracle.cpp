@@ -405,6 +405,11 @@ template<class R, bool kExact = false> inline void clip_range(const V2<R>* p, in
 
 struct ClipStats { uint64_t iterations = 0, pushes = 0, maxDepth = 0, overflow = 0; };
 
+// The CUDA path's limits on one patch search (clip2d_device in FP32, subdiv2d):
+// past this many iterations a search ends with the roots it has.  0 (the
+// reference's own searches): none.
+static uint64_t g_clipLimit = 0, g_subdivLimit = 0;
+
 // doBezierClipping2D_host, src/Spline_BezierClipping.cu:174-445 (the CPU
 // path of the reference: full sub-nets on an unbounded stack).
 template<class R, class F, bool kExact = false> bool clip2d_host(F& onHit, const V2<R>* patch, R tol, ClipStats* st)
@@ -521,6 +526,7 @@ template<class R, class F, bool kBounds64 = false> bool clip2d_device(F& onHit, 
     {
         // the near-grazing variant keeps what it found after 1024 iterations
         if (kBounds64 && it++ >= 1024) return found;
+        if (!kBounds64 && g_clipLimit && uint64_t(it++) >= g_clipLimit) return found;
         if (st) st->iterations++;
         const int cutside = cutsideStack & 1;
         R d0 = length(buf[3] - buf[12]);
@@ -606,8 +612,9 @@ template<class R, class F> bool subdiv2d(F& onHit, const V2<R>* patch, R tol, Cl
     bool reload = false;
     V2<R> buf[16];
     for (int i = 0; i < 16; i++) buf[i] = patch[i];
-    for (;;)
+    for (uint64_t it = 0;; it++)
     {
+        if (g_subdivLimit && it >= g_subdivLimit) break;
         if (st) st->iterations++;
         const R su = std::ldexp(R(1), -((k + 1) / 2));
         const R sv = std::ldexp(R(1), -(k / 2));
@@ -1774,6 +1781,8 @@ void ora_scene_set_split(void* s_, int mode) { static_cast<Scene*>(s_)->splitMod
 void ora_philox(uint32_t* ctr4, uint32_t k0, uint32_t k1) { philox(ctr4, k0, k1); }
 // the grazing margin of kClipGraze (process-wide; not thread-safe against running queries)
 void ora_set_graze_sin(float s) { g_grazeSin = s; }
+// iteration limits of one patch search, 0 = none (process-wide, as above)
+void ora_set_search_limits(uint64_t clip, uint64_t subdiv) { g_clipLimit = clip; g_subdivLimit = subdiv; }
 // the near-grazing test of CLIP_GRAZE64 (process-wide; see grazing())
 void ora_set_graze_mode(int m) { g_grazeMode = m; }
 // CLIP_GRAZE64: project a near-grazing candidate from the object-space ray
