@@ -13,6 +13,7 @@ namespace cgs {
 constexpr uint32_t EMPTY = 0xFFFFFFFFu;
 constexpr int kClipStack = 32;          // reference stack depth, src/Spline_BezierClipping.cu:577
 constexpr int kMaxClipIterations = 4096;
+constexpr int kMaxDepth = 64;  // of a render's bounces
 constexpr int kMaxBisections = 4 * kMaxClipIterations;  // of a subdivision search
 constexpr int kMaxTraversalSteps = 1 << 20;
 constexpr float kPi = 3.14159265358979323846f;
@@ -106,7 +107,8 @@ __device__ __forceinline__ float3 group_ambient(const DevScene& S, uint32_t g)
 struct Counters
 {
     unsigned long long nodes, hashLookups, candidates, iterations, rays, errors, tableReads;
-    unsigned long long longLists;  // long candidate lists taken (the query engine's allocator)
+    // long candidate lists taken (the query engine's allocator), by each query of the call: a render's of level l are 2 l and 2 l + 1
+    uint32_t longNext[2 * (kMaxDepth + 1)];
 };
 
 struct LocalCounters

@@ -104,11 +104,11 @@ struct Eng  // per-ray engine state, SoA over the query's capacity
     uint32_t subdivLevels; // subdivision searches: bisection levels a lane runs per resolve round
     // Long lists, for the few rays whose candidates on a walk tree outgrow their
     // chunk: kLongList entries each, taken by *longNext, nlong of them (none left:
-    // the ray goes back to the reference tree).
+    // the ray goes back to the reference tree).  Each query has them all.
     uint2* longs;
     uint32_t nlong;
     uint32_t allMarkers;  // lists keep the markers of objects that the ray meets no patch of (cgs_traverse)
-    unsigned long long* longNext;
+    uint32_t* longNext;
     __device__ __forceinline__ uint2* list_of(uint32_t rid) const
     {
         uint2* l = list + size_t(rid) * kChunk;
@@ -328,12 +328,13 @@ __device__ __forceinline__ void collect_rays(const DevScene& S, const RaysSoA& r
                 // hit as one chunk by chunk, which would cull some of them first
                 if (cap == kChunk && E.nlong)
                 {
-                    const unsigned long long at = atomicAdd(E.longNext, 1ull);
+                    // (looked at first: the count stops soon after the last)
+                    const uint32_t at = *(volatile uint32_t*)E.longNext < E.nlong ? atomicAdd(E.longNext, 1u) : E.nlong;
                     if (at < E.nlong)
                     {
                         uint2* l = E.longs + size_t(at) * kLongList;
                         for (uint32_t k = 0; k < ncand; k++) l[k] = list[k];
-                        list[0] = make_uint2(kLong, uint32_t(at));
+                        list[0] = make_uint2(kLong, at);
                         list = l;
                         cap = kLongList;
                         continue;
@@ -1898,7 +1899,7 @@ size_t engine_words(uint32_t capacity, int)
 
 cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Query q, bool any,
                       HitsSoA hits, int32_t* occluded, uint32_t* scratch, uint32_t capacity, int, Counters* cnt,
-                      cudaStream_t stream, int* launches)
+                      cudaStream_t stream, int* launches, uint32_t turn)
 {
     if (nDev) n = capacity;  // grid sizing only; kernels read *nDev
     if (n == 0) return cudaSuccess;
@@ -1918,8 +1919,8 @@ cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_
         E.originLast = uint32_t(ec.originLast);
         E.subdivLevels = uint32_t(ec.subdivLevels);
     }
-    E.longNext = &cnt->longLists;
-    if (!cnt) E.nlong = 0;
+    if (cnt) E.longNext = &cnt->longNext[turn];
+    else E.nlong = 0;
     int nl = 0;
     if (any) q.method != 0 ? launch<true, false, true>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl)
                            : launch<true, false>(S, rays, n, nDev, q, hits, occluded, E, cnt, stream, nl);

@@ -494,7 +494,7 @@ cudaError_t launch_render_wavefront(const DevScene& S, const RenderBatch& b, con
     {
         const HitsSoA hit = wb.hit[level & 1];
         cudaError_t e = run_query(S, q[cur].rays(), 0, wb.count + cur, b.q, false, hit, nullptr, wb.engine,
-                                  wb.engineCapacity, kEnginePasses, counters, stream, &nl);
+                                  wb.engineCapacity, kEnginePasses, counters, stream, &nl, 2 * level);
         if (e != cudaSuccess) return e;
         if (two && level > 0) cudaStreamWaitEvent(stream, wb.join, 0);
         cudaMemsetAsync(wb.count + (cur ^ 1), 0, sizeof(uint32_t), stream);
@@ -510,7 +510,7 @@ cudaError_t launch_render_wavefront(const DevScene& S, const RenderBatch& b, con
         }
         e = run_query(S, shadowRays, 0, wb.count + 2, qa, true, HitsSoA {}, wb.occluded,
                       two ? wb.engine2 : wb.engine, two ? wb.engine2Capacity : wb.engineCapacity, kEnginePasses,
-                      counters, side, &nl);
+                      counters, side, &nl, 2 * level + 1);
         if (e != cudaSuccess) return e;
         k_wf_visibility<<<gFlat, 256, 0, side>>>(wb.occluded, wb.shadowSlot, wb.count + 2, scap, wb.visible);
         k_wf_resolve<<<gFlat, 256, 0, side>>>(S, q[cur], wb.count + cur, hit, wb.contrib, wb.visible, wb.base, lcap,

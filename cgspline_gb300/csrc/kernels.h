@@ -58,11 +58,12 @@ cudaError_t launch_query_fp64(const DevScene& S, RaysSoA rays, uint32_t n, const
 // ---------------------------------------------------------- query engine --
 // Closest / any hit of n rays (n from the host, or *nDev when nDev != null;
 // capacity bounds both) by alternating traversal and clip passes
-// (k_engine.cu).  scratch holds engine_words(capacity, passes) words.
+// (k_engine.cu).  scratch holds engine_words(capacity, passes) words.  turn:
+// the query's number among those on these counters since they were cleared.
 size_t engine_words(uint32_t capacity, int passes);
 cudaError_t run_query(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Query q, bool any,
                       HitsSoA hits, int32_t* occluded, uint32_t* scratch, uint32_t capacity, int passes,
-                      Counters* counters, cudaStream_t stream, int* launches);
+                      Counters* counters, cudaStream_t stream, int* launches, uint32_t turn = 0);
 // The first collect pass of run_query alone (no clipping): each ray's
 // candidate list of that pass, its length copied to listLengths (device, may
 // be null).  For timing and profiling the traversal kernel.
