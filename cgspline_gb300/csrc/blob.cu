@@ -208,12 +208,7 @@ int cgs_scene_load(cgs_scene** out, const char* path, int device)
     s->current = ng - 1;
     s->bvhBuilt = true;
     // the walk trees are not part of the file: they follow from the patches
-    if (s->splitMode == CGS_SPLIT_REFERENCE)
-        for (Surface& sf : s->surfaces)
-        {
-            build_walk_bvh(sf, sf.walk);
-            check_walk_bvh(sf);
-        }
+    if (s->splitMode == CGS_SPLIT_REFERENCE) build_walk_bvhs(s);
     if (cudaSetDevice(s->device) != cudaSuccess || (st = upload_store(s)) != CGS_OK)
     {
         std::fclose(f);

@@ -119,13 +119,32 @@ DevMaterial to_dev(const cgs_material& m)
     return d;
 }
 
+// Runs fn(0) .. fn(n - 1) on the host's cores, in any order; on this thread
+// alone where there is little to do, on fewer where no more threads are to be had.
+unsigned host_cores() { return std::max(1u, std::min(64u, std::thread::hardware_concurrency())); }
+template<class F> void on_host_cores(size_t n, bool parallel, F&& fn)
+{
+    std::atomic<size_t> next {0};
+    auto worker = [&]() { for (size_t w; (w = next.fetch_add(1)) < n;) fn(w); };
+    const size_t nt = parallel ? std::min<size_t>(n, host_cores()) : 1;
+    std::vector<std::thread> pool;
+    pool.reserve(nt);
+    try
+    {
+        for (size_t t = 1; t < nt; t++) pool.emplace_back(worker);
+    }
+    catch (const std::system_error&) {}
+    worker();
+    for (auto& th : pool) th.join();
+}
+
 // BezierSurface::buildBVH (src/rt/Primitive.cu:199-220): per-patch bounds of
 // the 16 projected points and their mean as the centroid.
-std::vector<Element> surface_elements(const Surface& s)
+// cores: on all of the host's.
+std::vector<Element> surface_elements(const Surface& s, bool cores = false)
 {
     std::vector<Element> el(s.patchCount());
-    for (uint32_t i = 0; i < el.size(); i++)
-    {
+    auto fill = [&](uint32_t i) {
         Element& e = el[i];
         e.bounds = Box {};
         e.centroid[0] = e.centroid[1] = e.centroid[2] = 0.0f;
@@ -138,7 +157,11 @@ std::vector<Element> surface_elements(const Surface& s)
             e.bounds.inflate(p);
             for (int k = 0; k < 3; k++) e.centroid[k] = e.centroid[k] + inv * p[k];
         }
-    }
+    };
+    const size_t chunk = 4096, n = el.size();
+    on_host_cores((n + chunk - 1) / chunk, cores, [&](size_t c) {
+        for (size_t i = c * chunk; i < std::min(n, (c + 1) * chunk); i++) fill(uint32_t(i));
+    });
     return el;
 }
 
@@ -310,19 +333,6 @@ __global__ void k_gather_patches(const float4* __restrict__ points, const uint32
         patches[i] = points[index[i]];
 }
 
-// Runs fn(0) .. fn(n - 1) on the host's cores, in any order; on this thread
-// alone where there is little to do.
-template<class F> void on_host_cores(size_t n, bool parallel, F&& fn)
-{
-    std::atomic<size_t> next {0};
-    auto worker = [&]() { for (size_t w; (w = next.fetch_add(1)) < n;) fn(w); };
-    const size_t nt = parallel ? std::min<size_t>(n, std::max(1u, std::min(64u, std::thread::hardware_concurrency()))) : 1;
-    std::vector<std::thread> pool;
-    for (size_t t = 1; t < nt; t++) pool.emplace_back(worker);
-    worker();
-    for (auto& th : pool) th.join();
-}
-
 // Lights of all groups, concatenated; groupLights[g] = (first, count);
 // groupEnv[g] = background rgb, ambient rgb.
 int upload_lights(cgs_scene* sc)
@@ -348,22 +358,118 @@ int upload_lights(cgs_scene* sc)
 
 }  // namespace
 
+namespace {
+
+// The longest-axis tree of halves, one element to a leaf (which names it), in
+// place: a subtree of n elements has 2 n - 1 nodes, so every node's place in
+// pre-order is known beforehand and subtrees can be built by different cores.
+struct WalkTree
+{
+    struct Part { Element* e; size_t count; uint32_t key, at; };
+    std::vector<Node>& nodes;
+    std::vector<uint32_t>& keys;
+
+    // One node: false for a leaf, else its halves.
+    bool split(const Part& p, Part& l, Part& r) const
+    {
+        keys[p.at] = p.key;
+        Node& n = nodes[p.at];
+        if (p.count == 1)
+        {
+            Box box;
+            box.inflate(p.e->bounds);
+            n = Node {box, Box {}, EMPTY, p.e->index};
+            return false;
+        }
+        Box box;
+        for (size_t i = 0; i < p.count; i++) box.inflate(p.e[i].centroid);
+        const float v[3] = {box.hi[0] - box.lo[0], box.hi[1] - box.lo[1], box.hi[2] - box.lo[2]};
+        const int dim = v[2] > v[1] ? (v[0] > v[2] ? 0 : 2) : (v[0] > v[1] ? 0 : 1);  // as HostBVH::split
+        const size_t middle = p.count / 2;
+        std::nth_element(p.e, p.e + middle, p.e + p.count,
+                         [=](const Element& a, const Element& b) { return a.centroid[dim] < b.centroid[dim]; });
+        l = Part {p.e, middle, p.key << 1, p.at + 1};
+        r = Part {p.e + middle, p.count - middle, (p.key << 1) ^ 1u, p.at + uint32_t(2 * middle)};
+        n = Node {Box {}, Box {}, l.at, r.at};
+        return true;
+    }
+    // An inner node's boxes, its children's being done.
+    void join(uint32_t at) const
+    {
+        Node& n = nodes[at];
+        const Node &l = nodes[n.left], &r = nodes[n.right];
+        n.leftBox = l.leftBox;
+        n.rightBox = r.leftBox;
+        if (l.left != EMPTY) n.leftBox.inflate(l.rightBox);
+        if (r.left != EMPTY) n.rightBox.inflate(r.rightBox);
+    }
+    void build(const Part& p) const
+    {
+        Part l, r;
+        if (!split(p, l, r)) return;
+        build(l);
+        build(r);
+        join(p.at);
+    }
+    // The same by all cores: level by level until there are enough subtrees.
+    void build_on_cores(const Part& root) const
+    {
+        std::vector<Part> parts {root};
+        std::vector<uint32_t> inner;
+        while (parts.size() < 4 * host_cores())
+        {
+            std::vector<Part> next(2 * parts.size());
+            on_host_cores(parts.size(), true, [&](size_t i) {
+                if (!split(parts[i], next[2 * i], next[2 * i + 1])) next[2 * i].count = 0;
+            });
+            for (const Part& p : parts) if (p.count > 1) inner.push_back(p.at);
+            parts.clear();
+            for (size_t i = 0; i < next.size(); i += 2)
+                if (next[i].count) { parts.push_back(next[i]); parts.push_back(next[i + 1]); }
+            if (parts.empty()) break;
+        }
+        on_host_cores(parts.size(), true, [&](size_t i) { build(parts[i]); });
+        for (size_t i = inner.size(); i > 0; i--) join(inner[i - 1]);
+    }
+};
+
+}  // namespace
+
 // A second tree over a surface's patches for the query engine to walk: the
 // same median halves, split on the longest axis.  Halving n elements gives
 // the same heap keys in the same pre-order whatever the axis, so a hash table
 // of the one tree's keys finds the other's nodes.
-void cgs::build_walk_bvh(const Surface& s, HostBVH& out)
+void cgs::build_walk_bvh(const Surface& s, HostBVH& out, bool cores)
 {
-    std::vector<Element> el = surface_elements(s);
+    std::vector<Element> el = surface_elements(s, cores);
     out = HostBVH {};
+    out.split_mode = CGS_SPLIT_LONGEST;
+    if (el.empty()) return;
     for (const Element& e : el)
         for (int k = 0; k < 3; k++)
             if (!std::isfinite(e.bounds.lo[k]) || !std::isfinite(e.bounds.hi[k])) return;
-    out.split_mode = CGS_SPLIT_LONGEST;
-    out.build(el);
-    for (Node& n : out.nodes)
-        if (n.left == EMPTY) n.right = out.indices[n.right];  // a leaf names its patch
-    out.indices.clear();
+    out.nodes.resize(2 * el.size() - 1);
+    out.keys.resize(2 * el.size() - 1);
+    const WalkTree tree {out.nodes, out.keys};
+    const WalkTree::Part root {el.data(), el.size(), 1u, 0u};
+    if (cores) tree.build_on_cores(root);
+    else tree.build(root);
+}
+
+// The walk trees of a store read from a blob: surfaces side by side, and one
+// that has more than a core's share of the patches by all cores before them.
+// (One thread takes 1.6 s per million patches.)
+void cgs::build_walk_bvhs(cgs_scene* sc)
+{
+    size_t patches = 0;
+    for (const Surface& s : sc->surfaces) patches += s.patchCount();
+    std::vector<Surface*> few;
+    for (Surface& s : sc->surfaces)
+        if (s.patchCount() >= 16384 && size_t(s.patchCount()) * host_cores() > patches) build_walk_bvh(s, s.walk, true);
+        else few.push_back(&s);
+    std::sort(few.begin(), few.end(), [](const Surface* a, const Surface* b) { return a->patchCount() > b->patchCount(); });
+    on_host_cores(few.size(), patches > 250, [&](size_t w) { build_walk_bvh(*few[w], few[w]->walk); });
+    on_host_cores(sc->surfaces.size(), patches > 250, [&](size_t i) { check_walk_bvh(sc->surfaces[i]); });
 }
 
 // What the walk relies on: both trees have the same keys in the same order and

@@ -244,8 +244,10 @@ namespace cgs {
 
 void camera_setup(const cgs_camera& c, uint32_t w, uint32_t h, int flip, CameraSetup& s);
 int upload_store(cgs_scene* sc);
-// The walk tree of a surface (Surface::walk), for stores of the reference split.
-void build_walk_bvh(const Surface& s, HostBVH& out);
+// The walk tree of a surface (Surface::walk), for stores of the reference split; cores: by all of the host's.
+void build_walk_bvh(const Surface& s, HostBVH& out, bool cores = false);
+// Those of all surfaces, checked (check_walk_bvh).
+void build_walk_bvhs(cgs_scene* sc);
 // Drops s.walk unless the leaves and keys of s.bvh, read from a blob, are those of the walk tree and its
 // boxes nest.
 void check_walk_bvh(Surface& s);
