@@ -1,6 +1,8 @@
 // api.cu -- queries and rendering entry points of libcgspline_gb300.so:
 // closest / any-hit ray queries, (ray, patch) pair clipping, single and
 // batched frame renders, and the standalone perfect-hash build.
+#include <cuda.h>
+
 #include "scene_impl.h"
 
 #include <map>
@@ -355,14 +357,51 @@ void query_end(cgs_scene* s, cudaStream_t st, bool captured)
     }
 }
 
-// How many of the rows of n words from rows[0] on lie one after another in
-// memory: those go in one copy (a copy of a few rays costs about 6 us of calls,
-// and a query took twelve: 33 rays 162 us, 130 us with three).
+// Which page-locked (or other CUDA) allocation p lies in; 0: ordinary host memory.
+uint64_t host_allocation(const void* p)
+{
+    using Get = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Get get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found);
+        if (e != cudaSuccess || found != cudaDriverEntryPointSuccess) { cudaGetLastError(); f = nullptr; }
+        return reinterpret_cast<Get>(f);
+    }();
+    unsigned long long id = 0;
+    if (!get) return uint64_t(reinterpret_cast<uintptr_t>(p));  // unknown: no two rows are in one
+    return get(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, CUdeviceptr(reinterpret_cast<uintptr_t>(p))) == CUDA_SUCCESS ? id : 0;
+}
+
+// How many of the rows of n words from rows[0] on lie one after another in one
+// allocation: those go in one copy (a copy costs about 6 us of calls).  Rows that
+// only happen to be neighbours, page-locked one by one or not at all, do not: a
+// copy may not span such ranges.  A row by itself lies in one of them, so its
+// first word tells which (0.4 us a row).
 template<class T> int adjacent_rows(const T* const* rows, int count, uint32_t n)
 {
     int run = 1;
-    while (rows[0] && run < count && rows[run] == rows[run - 1] + n) run++;
+    if (!rows[0] || count < 2 || rows[1] != rows[0] + n) return run;
+    const uint64_t allocation = host_allocation(rows[0]);
+    while (run < count && rows[run] == rows[run - 1] + n && host_allocation(rows[run]) == allocation) run++;
     return run;
+}
+
+// A host query of at most this many rays goes through page-locked rows of the
+// scene's own, three copies whatever the caller's rows lie in: 33 rays 162 us a
+// query with a copy for each row, 128 us with neighbouring rows copied together
+// where they lie, 117 us so.
+constexpr uint32_t kHostStageRays = 1024;
+
+uint32_t* host_stage(cgs_scene* s, uint32_t n)
+{
+    if (n > kHostStageRays) return nullptr;
+    if (!s->hostStage && cudaMallocHost(&s->hostStage, 12ull * kHostStageRays * 4) != cudaSuccess)
+    {
+        cudaGetLastError();
+        s->hostStage = nullptr;
+    }
+    return s->hostStage;
 }
 
 }  // namespace cgs
@@ -439,6 +478,7 @@ int cgs_intersect_host(cgs_scene* s, const cgs_rays* rays, uint32_t n, int metho
     cudaStream_t st = (cudaStream_t)stream;
     cgs_rays dr {};
     cgs_hits dh {};
+    uint32_t* stage = nullptr;
     {
         std::lock_guard<std::mutex> g(s->mu);
         CGS_TRY(cudaSetDevice(s->device));
@@ -448,7 +488,15 @@ int cgs_intersect_host(cgs_scene* s, const cgs_rays* rays, uint32_t n, int metho
         const float* src[7] = {rays->ox, rays->oy, rays->oz, rays->dx, rays->dy, rays->dz, rays->tmax};
         for (int k = 0; k < 6; k++)
             if (!src[k]) return CGS_ERR_INVALID_ARGUMENT;
-        for (int k = 0, run; k < 7; k += run)
+        stage = host_stage(s, n);
+        if (stage)
+        {
+            for (int k = 0; k < 7; k++)
+                if (src[k]) std::memcpy(stage + size_t(k) * n, src[k], n * sizeof(float));
+            CGS_TRY(cudaMemcpyAsync(s->rayStage.p, stage, (src[6] ? 7ull : 6ull) * n * sizeof(float),
+                                    cudaMemcpyHostToDevice, st));
+        }
+        for (int k = 0, run; !stage && k < 7; k += run)
         {
             run = adjacent_rows(src + k, 7 - k, n);
             if (src[k])
@@ -467,6 +515,21 @@ int cgs_intersect_host(cgs_scene* s, const cgs_rays* rays, uint32_t n, int metho
         dh = cgs_hits {s->hitF.p, s->hitF.p + n, s->hitF.p + 2ull * n, s->hitI.p, s->hitI.p + n};
     }
     int r = cgs_intersect(s, &dr, n, method, precision, tol, any_hit, &dh, stream);
+    if (stage)
+    {
+        uint32_t* out = stage + 7ull * n;
+        if (!r && cudaMemcpyAsync(out, s->hitI.p, (any_hit ? 1ull : 2ull) * n * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            r = CGS_ERR_CUDA;
+        if (!r && !any_hit && cudaMemcpyAsync(out + 2ull * n, s->hitF.p, 3ull * n * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            r = CGS_ERR_CUDA;
+        // (on an error too: the stage is the next call's)
+        const cudaError_t e = cudaStreamSynchronize(st);
+        if (r || e != cudaSuccess) return r ? r : cuda_status(e);
+        void* dst[5] = {hits->patch, hits->object, hits->t, hits->u, hits->v};
+        for (int k = 0; k < (any_hit ? 1 : 5); k++)
+            if (dst[k]) std::memcpy(dst[k], out + size_t(k) * n, n * 4ull);
+        return CGS_OK;
+    }
     if (r) return r;
     const int32_t* whole[2] = {hits->patch, any_hit ? nullptr : hits->object};
     for (int k = 0, run; k < 2; k += run)

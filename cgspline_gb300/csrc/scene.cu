@@ -871,6 +871,7 @@ cgs_scene::~cgs_scene()
                     &hashJobs, &leafKeys,
                     &engine, &fbStage})
         b->release();
+    if (hostStage) cudaFreeHost(hostStage);
     rayStage.release(); hitF.release(); linStage.release(); groupEnv.release();
     groupLights.release(); bvhs.release(); dobjects.release(); materials.release(); dlights.release();
     scratch64.release(); counters.release(); hitI.release();

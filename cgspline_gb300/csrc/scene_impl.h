@@ -205,6 +205,7 @@ struct cgs_scene
 
     // query staging and engine scratch
     cgs::DBuf<float> rayStage, hitF;
+    uint32_t* hostStage = nullptr;  // page-locked rows of a host query of few rays
     cgs::DBuf<int32_t> hitI;
     cgs::DBuf<uint32_t> groupStage, engine;
     uint32_t engineCapacity = 0;
