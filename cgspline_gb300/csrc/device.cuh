@@ -525,13 +525,21 @@ __device__ __forceinline__ double scale2(double x, int k)
     return __hiloint2double(__double2hiint(x) + k * 0x100000, __double2loint(x));
 }
 
+// Whether x has a significand of all ones.
+__device__ __forceinline__ bool all_ones(double x)
+{
+    return ((uint32_t(__double2hiint(x)) | 0xFFF00000u) & uint32_t(__double2loint(x))) == 0xFFFFFFFFu;
+}
+
 // a / b, rounded to nearest: a reciprocal by Newton's iteration from FP32, then
 // the quotient corrected by its remainder (P. W. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34,
-// 1990).  Seven FP64 instructions; outside the exponents that this is safe for, the operator.
+// 1990), which takes a reciprocal rounded to nearest: the iteration gives that
+// for every significand but one of all ones.  Seven FP64 instructions; there, and
+// outside the exponents that this is safe for, the operator.
 __device__ __forceinline__ double quotient(double a, double b)
 {
-    if (exponent_bits(b) - 923u >= 200u || exponent_bits(a) - 523u >= 1000u) return a / b;
+    if (exponent_bits(b) - 923u >= 200u || exponent_bits(a) - 523u >= 1000u || all_ones(b)) return a / b;
     double y = widen(1.0f / narrow(b));
     y = fma(y, fma(-b, y, 1.0), y);
     y = fma(y, fma(-b, y, 1.0), y);
@@ -559,6 +567,7 @@ __device__ __forceinline__ double2 unit2d(double2 L)
     g = fma(g, r, g);
     h = fma(h, r, h);
     const double l = fma(fma(-g, g, s), h, g);
+    if (all_ones(l)) return make_double2(L.x / l, L.y / l);
     double y = scale2(h, 1);
     y = fma(y, fma(-l, y, 1.0), y);
     const double qx = L.x * y, qy = L.y * y;
@@ -637,10 +646,11 @@ __device__ __forceinline__ void hull_scan_d(const double* ybot, const double* yt
         const float f3 = narrow(Y[k]);
         if (k < 7)
         {
-            // the turn's sign in FP32 where it is past the rounding of its inputs and terms, else in FP64
+            // the turn's sign in FP32 where it is past the rounding of its inputs (to denormals too) and
+            // terms, else in FP64
             const float turn = minusf(i2, i1) * (f3 - f1) - (f2 - f1) * minusf(at[k], i1);
             keep = turn > 0.0f;
-            if (!(fabsf(turn) > 0x1p-20f * (fabsf(f1) + fabsf(f2) + fabsf(f3))))
+            if (!(fabsf(turn) > 0x1p-20f * (fabsf(f1) + fabsf(f2) + fabsf(f3)) + 0x1p-126f))
                 keep = not_negative(minus(i2, i1) * (Y[k] - y1) - (y2 - y1) * minus(at[k], i1));
         }
         // as in hull_scan; ends whose exponents differ by 50 or less do not round away in their difference
