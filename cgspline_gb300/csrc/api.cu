@@ -707,7 +707,9 @@ int cgs_engine_config_set(const cgs_engine_config* in)
 // candidate renders the batch (wavefront schedule) `repeats` + 2 times, the
 // last `repeats` timed with CUDA events on `stream`; its median is its score.
 // Two rounds visit the knobs in turn, each set to its fastest value with the
-// others held; scores are kept, so a setting is timed once.
+// others held; scores are kept, so a setting is timed once.  Block sizes and
+// occupancies are left as they are where the batch's queries are one launch each
+// (they would be chosen by noise, for every later batch).
 int cgs_autotune_render(cgs_scene* s, const cgs_render_request* reqs, uint32_t n, const cgs_render_options* opt,
                         int repeats, cgs_engine_config* best, double* best_ms, void* stream)
 {
@@ -781,11 +783,14 @@ int cgs_autotune_render(cgs_scene* s, const cgs_render_request* reqs, uint32_t n
         {&Point::width, {1, 8, 16}},    {&Point::order, {0, 1}},    {&Point::olast, {0, 1}}};
     // the subdivision levels per round matter only to a subdivision batch
     if (opt->method == CGS_METHOD_SUBDIV) knobs.push_back({&Point::levels, {1, 4, 16, 64}});
+    const uint32_t closest = s->slot.wb.engineCapacity, any = s->slot.wb.side ? s->slot.wb.engine2Capacity : closest;
+    const bool whole = one_launch(closest, opt->method, false, true) && one_launch(any, opt->method, true, true);
     for (int round = 0; round < 2 && status == CGS_OK; round++)
         for (const auto& [field, values] : knobs)
             for (int v : values)
             {
                 if (status != CGS_OK) break;
+                if (whole && !cur.cq && (field == &Point::ct || field == &Point::rt || field == &Point::capped)) continue;
                 Point p = cur;
                 p.*field = v;
                 const double ms = score(p);

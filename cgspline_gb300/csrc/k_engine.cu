@@ -1797,9 +1797,7 @@ void launch(const DevScene& S, RaysSoA rays, uint32_t n, const uint32_t* nDev, Q
             int32_t* occluded, Eng E, Counters* cnt, cudaStream_t stream, int& nl)
 {
     const EngineConfig c = engine_config();
-    // a render's shadow queue is sized for a ray per sample and light and holds the ones that face it
-    const uint32_t small = (kSub ? kSmallSubdivRays : kSmallRays) * (kAny && nDev ? 2 : 1);
-    if (n <= small && !c.compressedNodes)
+    if (one_launch(n, kSub ? 1 : 0, kAny, nDev != nullptr) && !c.compressedNodes)
     {
         static const int warps = resident((const void*)k_small<kAny, kG64, kSub>, 32);
         k_small<kAny, kG64, kSub><<<int(std::min<uint32_t>(n, uint32_t(warps))), 32, 0, stream>>>(
@@ -1859,6 +1857,12 @@ std::mutex gConfigMu;
 EngineConfig gConfig;
 uint64_t gConfigGen = 1;
 }  // namespace
+
+bool one_launch(uint32_t n, int method, bool any, bool deviceCount)
+{
+    // a render's shadow queue is sized for a ray per sample and light and holds the ones that face it
+    return n <= (method != 0 ? kSmallSubdivRays : kSmallRays) * (any && deviceCount ? 2 : 1);
+}
 
 EngineConfig engine_config()
 {

@@ -56,6 +56,8 @@ cudaError_t launch_query_fp64(const DevScene& S, RaysSoA rays, uint32_t n, const
                               HitsSoA hits, Counters* counters, cudaStream_t stream);
 
 // ---------------------------------------------------------- query engine --
+// Whether a query of n rays (with device counts: at most n) on the exact nodes is one launch.
+bool one_launch(uint32_t n, int method, bool any, bool deviceCount);
 // Closest / any hit of n rays (n from the host, or *nDev when nDev != null;
 // capacity bounds both) by alternating traversal and clip passes
 // (k_engine.cu).  scratch holds engine_words(capacity, passes) words.  turn:

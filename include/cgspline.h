@@ -331,7 +331,9 @@ typedef struct cgs_engine_config {
      * node (child boxes on an 8-bit grid of the node's box, widened outward
      * so that they contain the exact boxes); 0 (default): the exact 64-byte
      * records.  The compressed boxes are met wherever the exact ones are, so
-     * both settings give the same hits; the exported BVH is the exact one.
+     * both settings give the same hits, but for rays that run in the faces of
+     * boxes: they meet candidates that the exact boxes just miss.  The
+     * exported BVH is the exact one.
      * The autotuner tries both. */
     int compressed_nodes;
     /* Candidate-list entries a ray may fill in the first collect pass before
@@ -378,6 +380,8 @@ int cgs_engine_config_set(const cgs_engine_config* config);
  * subdivision batch, 1, 4, 16 or 64 subdivision levels per round),
  * then passes 2, 4, 8 x first chunk 8, 16, 32, 64 as pairs, each knob set to its fastest
  * value with the others held; a setting already timed is not timed again.
+ * Block sizes and blocks per SM stay as they are where the batch's queries run
+ * whole in one launch each.
  * Synchronises `stream`. */
 int cgs_autotune_render(cgs_scene* scene, const cgs_render_request* requests, uint32_t n,
                         const cgs_render_options* options, int repeats, cgs_engine_config* best,
