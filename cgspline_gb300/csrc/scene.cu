@@ -265,23 +265,22 @@ __device__ bool axis_grid(double lo, double hi, float& P, int& e)
 // compressed mirror from qbase on (EMPTY: it has none there), the BVH that they belong to.
 struct PackJob { uint32_t first, count, qbase, bvh; };
 
-// The node records of a store from the host trees' nodes: a thread per node,
-// all trees in one launch (their jobs in ascending order).  failed[bvh] is set
-// where a node has no compressed record.  Bound by the upload of its input;
-// packing on the host, one thread over 120,000 nodes, was most of the 8.4 ms that
-// the upload and hash build of a 30,000-patch store took (2.0 ms now).
-__global__ void k_pack_nodes(const Node* __restrict__ raw, const PackJob* __restrict__ jobs, uint32_t njobs, uint32_t total,
-                             float4* nodes, uint4* qnodes, uint32_t* failed)
+// A node's 64-byte record on the device: the host's node and padding.
+struct NodeRecord { Node node; uint32_t pad[2]; };
+static_assert(sizeof(Node) == 56 && sizeof(NodeRecord) == 4 * sizeof(float4));
+
+// The compressed mirror of a store's nodes: a thread per node, all trees in one
+// launch (their jobs in ascending order).  failed[bvh] is set where a node has no
+// compressed record.  Bound by its launch; on the host, one thread over 120,000
+// nodes, it was most of the 8.4 ms that the upload and hash build of a
+// 30,000-patch store took (2.0 ms now).
+__global__ void k_pack_nodes(const NodeRecord* __restrict__ nodes, const PackJob* __restrict__ jobs, uint32_t njobs,
+                             uint32_t total, uint4* qnodes, uint32_t* failed)
 {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x)
     {
-        const Node n = raw[g];
+        const Node n = nodes[g].node;
         const Box &L = n.leftBox, &R = n.rightBox;
-        float4* q = nodes + 4ull * g;
-        q[0] = make_float4(L.lo[0], L.lo[1], L.lo[2], L.hi[0]);
-        q[1] = make_float4(L.hi[1], L.hi[2], R.lo[0], R.lo[1]);
-        q[2] = make_float4(R.lo[2], R.hi[0], R.hi[1], R.hi[2]);
-        q[3] = make_float4(__uint_as_float(n.left), __uint_as_float(n.right), 0.0f, 0.0f);
         uint32_t lo = 0, hi = njobs;
         while (hi - lo > 1)
         {
@@ -323,14 +322,6 @@ __global__ void k_pack_nodes(const Node* __restrict__ raw, const PackJob* __rest
         w[0] = make_uint4(P[0], P[1], P[2], ex[0] | (ex[1] << 8) | (ex[2] << 16) | ((leaf ? kQLeaf : 0u) << 24));
         w[1] = make_uint4(bytes[0], bytes[1], bytes[2], n.right);
     }
-}
-
-// De-indexed patches: 16 points each.
-__global__ void k_gather_patches(const float4* __restrict__ points, const uint32_t* __restrict__ index, size_t n,
-                                 float4* patches)
-{
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
-        patches[i] = points[index[i]];
 }
 
 // Lights of all groups, concatenated; groupLights[g] = (first, count);
@@ -546,17 +537,12 @@ int cgs::upload_store(cgs_scene* sc)
         d.Nmagic = fastmod_magic(std::max<uint32_t>(n, 1));
     }
     for (uint32_t g = 0; g < sc->groups.size(); g++) gtop.push_back(ns + g);
-    std::vector<size_t> pointBase;
-    size_t points = 0;
     uint32_t patches = 0;
     for (const Surface& s : sc->surfaces)
     {
         pbase.push_back(patches);
-        pointBase.push_back(points);
         patches += s.patchCount();
-        points += s.points.size() / 4;
     }
-    if (points > 0xFFFFFFFFull) return CGS_ERR_INVALID_ARGUMENT;
     for (const Object& ob : sc->objects)
     {
         DevObject d {};
@@ -575,41 +561,51 @@ int cgs::upload_store(cgs_scene* sc)
             d.patchMaterialBase = -1;
         ho.push_back(d);
     }
-    // The host trees and control points as they are, in one staging area: nodes,
-    // points, point indices, leaf lists, leaf keys.  Each surface and group is
-    // copied into its places by one of the host's cores; the device makes its
-    // records from them (k_pack_nodes, k_gather_patches).
+    // The device's arrays in one staging area on the host, filled by its cores:
+    // de-indexed patches (16 points each), node records, leaf lists, leaf keys.  They
+    // go to their places as they are, so a store needs no more device memory while it
+    // is made than afterwards.
     auto place = [cursor = size_t(0)](size_t bytes) mutable {
         const size_t at = cursor;
         cursor = (cursor + bytes + 255) & ~size_t(255);
         return at;
     };
-    const size_t oPoints = place(points * sizeof(float4)), oIndex = place(size_t(patches) * 64),
-                 oNodes = place(size_t(nodeCursor) * sizeof(Node)), oJobs = place(jobs.size() * sizeof(PackJob)),
-                 oFailed = place(nb * sizeof(uint32_t)), raw = place(0), oList = place(size_t(indexCursor) * 4),
-                 oKeys = place(sc->walkTrees ? size_t(patches) * 4 : 0), total = place(0);
+    const size_t oPatches = place(size_t(patches) * 256), oNodes = place(size_t(nodeCursor) * sizeof(NodeRecord)),
+                 oList = place(size_t(indexCursor) * 4), oKeys = place(sc->walkTrees ? size_t(patches) * 4 : 0),
+                 total = place(0);
     std::unique_ptr<uint8_t[]> stage(new (std::nothrow) uint8_t[std::max<size_t>(total, 1)]);
     if (!stage) return CGS_ERR_OUT_OF_MEMORY;
     uint8_t* h = stage.get();
-    std::memcpy(h + oJobs, jobs.data(), jobs.size() * sizeof(PackJob));
-    std::memset(h + oFailed, 0, nb * sizeof(uint32_t));
-    on_host_cores(nb, total > (1u << 20), [&](size_t k) {
-        const HostBVH& b = sc->bvh(uint32_t(k));
+    // one piece of work is a range of a tree's nodes and of its surface's patches
+    struct Piece { uint32_t k, first; };
+    constexpr uint32_t kPiece = 8192;
+    std::vector<Piece> pieces;
+    for (uint32_t k = 0; k < nb; k++)
+        for (uint32_t first = 0; first == 0 || first < sc->bvh(k).nodes.size(); first += kPiece) pieces.push_back({k, first});
+    on_host_cores(pieces.size(), total > (1u << 20), [&](size_t i) {
+        const uint32_t k = pieces[i].k, first = pieces[i].first;
+        const HostBVH& b = sc->bvh(k);
         const DevBVH& d = sc->hbvh[k];
-        Node* nodes = reinterpret_cast<Node*>(h + oNodes);
-        std::copy(b.nodes.begin(), b.nodes.end(), nodes + d.nodeBase);
-        std::copy(b.indices.begin(), b.indices.end(), reinterpret_cast<uint32_t*>(h + oList) + d.indexBase);
-        if (k >= ns) return;
-        const Surface& s = sc->surfaces[k];
-        std::memcpy(h + oPoints + pointBase[k] * sizeof(float4), s.points.data(), s.points.size() * sizeof(float));
-        uint32_t* index = reinterpret_cast<uint32_t*>(h + oIndex) + size_t(pbase[k]) * 16;
-        for (size_t i = 0; i < s.indices.size(); i++) index[i] = uint32_t(pointBase[k]) + s.indices[i];
-        if (!sc->walkTrees) return;
-        uint32_t* keys = reinterpret_cast<uint32_t*>(h + oKeys) + pbase[k];
-        if (d.walkBase == EMPTY) { std::fill(keys, keys + s.patchCount(), 0u); return; }
-        std::copy(s.walk.nodes.begin(), s.walk.nodes.end(), nodes + d.walkBase);
-        for (size_t i = 0; i < b.nodes.size(); i++)
-            if (b.nodes[i].left == EMPTY) keys[b.indices[b.nodes[i].right]] = b.keys[i];
+        NodeRecord* nodes = reinterpret_cast<NodeRecord*>(h + oNodes);
+        const bool walk = d.walkBase != EMPTY;
+        const Surface* s = k < ns ? &sc->surfaces[k] : nullptr;
+        uint32_t* keys = reinterpret_cast<uint32_t*>(h + oKeys) + (s ? pbase[k] : 0);
+        for (size_t j = first; j < std::min<size_t>(b.nodes.size(), first + kPiece); j++)
+        {
+            nodes[d.nodeBase + j] = NodeRecord {b.nodes[j], {0, 0}};
+            if (!walk) continue;
+            nodes[d.walkBase + j] = NodeRecord {s->walk.nodes[j], {0, 0}};
+            if (b.nodes[j].left == EMPTY) keys[b.indices[b.nodes[j].right]] = b.keys[j];
+        }
+        if (first == 0)
+            std::copy(b.indices.begin(), b.indices.end(), reinterpret_cast<uint32_t*>(h + oList) + d.indexBase);
+        if (!s) return;
+        // (a tree has up to twice as many nodes as its surface patches: the last piece takes the rest)
+        const bool last = size_t(first) + kPiece >= b.nodes.size();
+        const uint32_t p0 = std::min(first, s->patchCount()), p1 = last ? s->patchCount() : std::min(first + kPiece, s->patchCount());
+        float* out = reinterpret_cast<float*>(h + oPatches) + 64ull * (size_t(pbase[k]) + p0);
+        for (size_t j = 16ull * p0; j < 16ull * p1; j++, out += 4) std::memcpy(out, &s->points[4ull * s->indices[j]], 16);
+        if (sc->walkTrees && !walk) std::fill(keys + p0, keys + p1, 0u);
     });
     CGS_TRY(sc->patches.reserve(size_t(patches) * 16));
     CGS_TRY(sc->nodes.reserve(4ull * nodeCursor));
@@ -625,21 +621,24 @@ int cgs::upload_store(cgs_scene* sc)
     CGS_TRY(sc->materials.reserve(hm.size()));
     CGS_TRY(sc->counters.reserve(1));
     if (sc->walkTrees) CGS_TRY(sc->leafKeys.reserve(patches));
+    // the jobs and the flags that they raise, in one small array
     struct Temp
     {
-        DBuf<uint8_t> b;
+        DBuf<uint32_t> b;
         ~Temp() { b.release(); }
     } temp;
-    CGS_TRY(temp.b.reserve(raw));
-    uint8_t* dv = temp.b.p;
-    CGS_TRY(cudaMemcpy(dv, h, raw, cudaMemcpyHostToDevice));
-    const uint32_t blocks = 1216;
-    k_gather_patches<<<blocks, 256>>>(reinterpret_cast<const float4*>(dv + oPoints),
-                                      reinterpret_cast<const uint32_t*>(dv + oIndex), size_t(patches) * 16, sc->patches.p);
-    k_pack_nodes<<<blocks, 128>>>(reinterpret_cast<const Node*>(dv + oNodes), reinterpret_cast<const PackJob*>(dv + oJobs),
-                                  uint32_t(jobs.size()), nodeCursor, sc->nodes.p, sc->qnodes.p,
-                                  reinterpret_cast<uint32_t*>(dv + oFailed));
+    const size_t jobWords = jobs.size() * sizeof(PackJob) / 4;
+    std::vector<uint32_t> jobStage(jobWords + nb, 0u);
+    std::memcpy(jobStage.data(), jobs.data(), jobs.size() * sizeof(PackJob));
+    CGS_TRY(temp.b.reserve(jobStage.size()));
+    uint32_t* dFailed = temp.b.p + jobWords;
+    CGS_TRY(cudaMemcpy(temp.b.p, jobStage.data(), jobStage.size() * 4, cudaMemcpyHostToDevice));
+    CGS_TRY(cudaMemcpy(sc->nodes.p, h + oNodes, size_t(nodeCursor) * sizeof(NodeRecord), cudaMemcpyHostToDevice));
+    k_pack_nodes<<<(nodeCursor + 127) / 128, 128>>>(reinterpret_cast<const NodeRecord*>(sc->nodes.p),
+                                                    reinterpret_cast<const PackJob*>(temp.b.p), uint32_t(jobs.size()),
+                                                    nodeCursor, sc->qnodes.p, dFailed);
     CGS_TRY(cudaGetLastError());
+    CGS_TRY(cudaMemcpy(sc->patches.p, h + oPatches, size_t(patches) * 256, cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->indices.p, h + oList, size_t(indexCursor) * 4, cudaMemcpyHostToDevice));
     if (sc->walkTrees) CGS_TRY(cudaMemcpy(sc->leafKeys.p, h + oKeys, size_t(patches) * 4, cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->patchBase.p, pbase.data(), pbase.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -649,7 +648,7 @@ int cgs::upload_store(cgs_scene* sc)
     CGS_TRY(cudaMemcpy(sc->materials.p, hm.data(), hm.size() * sizeof(DevMaterial), cudaMemcpyHostToDevice));
     CGS_TRY(cudaMemcpy(sc->groupTop.p, gtop.data(), gtop.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     std::vector<uint32_t> failed(nb);
-    CGS_TRY(cudaMemcpy(failed.data(), dv + oFailed, nb * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    CGS_TRY(cudaMemcpy(failed.data(), dFailed, nb * sizeof(uint32_t), cudaMemcpyDeviceToHost));
     for (uint32_t k = 0; k < nb; k++) sc->hbvh[k].compressed = failed[k] ? 0u : 1u;
     CGS_TRY(cudaMemcpy(sc->bvhs.p, sc->hbvh.data(), nb * sizeof(DevBVH), cudaMemcpyHostToDevice));
     int r = upload_lights(sc);
