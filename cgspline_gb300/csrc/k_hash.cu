@@ -698,7 +698,7 @@ cudaError_t hash_build_blocks(const uint32_t* keys, const HashJob* jobs, uint32_
     // clusters, builds in 12.2 ms; with clusters of 16 for all 23.7 ms, with one CTA a
     // BVH 20.8 ms.  One such BVH alone is fastest with 16 (39,199 keys: 1.8 ms, 16.1 ms
     // with one CTA).
-    const uint32_t room = 144u / std::max(batch, njobs);
+    const uint32_t room = uint32_t(device_sms()) / 16u * 16u / std::max(batch, njobs);
     switch (std::max(nb / 2048u, std::min(bit_floor_u32(std::max(room, 1u)), 16u)))
     {
     case 0: case 1: case 2: return launch(k_hash_block<2>, 2u, false);
