@@ -118,7 +118,9 @@ struct Eng  // per-ray engine state, SoA over the query's capacity
 };
 
 constexpr size_t kWordsPerRay = 2 + 2 * kChunk + 18;
-constexpr uint32_t long_lists(uint32_t cap) { return cap / 48 + 32; }
+// Long lists of a scratch area for cap rays: 43 bytes a ray, 7% of its scratch (a
+// single ray has one: servers of a few KB run too).
+constexpr uint32_t long_lists(uint32_t cap) { return cap / 48 + (cap < 32 ? cap : 32); }
 
 Eng carve(uint32_t* base, uint32_t cap)
 {
