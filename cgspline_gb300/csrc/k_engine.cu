@@ -787,8 +787,8 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_long(DevScene S, RaysSo
 // limit, or where the stack would have held nearly all that fit, it drops what
 // the parts found and searches again alone, up to the limit: the patch, or the
 // ray's list for any hit.  So no answer depends on which lanes were idle.  (With a
-// limit for each lane's part queries took 1% less, and a search that reaches it
-// gave what its warp's idle lanes made of it.)
+// limit for each lane's part a search that reaches it gave what its warp's idle
+// lanes made of it.)
 //
 // An any-hit clipping search waits for nobody: whichever lane finds a root marks
 // the ray occluded (writes of "occluded" never clear it), and each part has the
@@ -810,12 +810,12 @@ template<> struct Lend<true> { uint32_t sum[32], who[32]; };
 constexpr int kPartsStack = 31;
 // kOverLimit: the search's parts together are past the limit, the others are to end.
 constexpr uint32_t kKids = 0xFFu, kFound = 0x100u, kOverLimit = 0x200u, kSpentShift = 10;
-// What a lane searches: a ray's patch of its own, with intervals lent (the owner),
-// an interval borrowed, or a patch again, alone.
-enum Role : int { kOwn, kLent, kThief, kAlone };
+// What a lane searches: a ray's patch of its own, a patch again and alone, a patch
+// with intervals lent (the owner), or an interval borrowed.
+enum Role : int { kOwn, kAlone, kLent, kThief };
 // Where an owner is.
 enum LendEnd { kUnended, kEndedNothing, kEndedRoot, kEndedAgain };
-__device__ __forceinline__ bool in_parts(int role) { return role == kLent || role == kThief; }
+__device__ __forceinline__ bool in_parts(int role) { return role >= kLent; }
 
 // Adds a lane's root to its owner's: the nearest is kept, the first in the
 // search's order at equal distances.
@@ -1168,9 +1168,11 @@ __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays
     {
         if constexpr (!kG64)
         {
+            // lanes in none of the searches' parts: one vote while there are none
+            const unsigned resting = __ballot_sync(0xFFFFFFFFu, part >= kPartMerge);
             if constexpr (!kAny)
             {
-                if (__ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
+                if (resting && __ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
                 {
                     const LendEnd end = lend_settle(L, part, role, sink, c.found, uint32_t(c.it), kMaxClipIterations);
                     if (end == kEndedRoot) w.keep(L.t[lane_id()], L.u[lane_id()], L.v[lane_id()]);
@@ -1183,7 +1185,7 @@ __device__ __forceinline__ void clip_rays(const DevScene& S, const RaysSoA& rays
                     }
                 }
             }
-            const unsigned idleM = __ballot_sync(0xFFFFFFFFu, part == kPartNone);
+            const unsigned idleM = resting ? __ballot_sync(0xFFFFFFFFu, part == kPartNone) : 0u;
             if (idleM)
             {
                 const bool rich = part >= kPartProject && part <= kPartRoot && c.sl > c.base && c.sl < kPartsStack &&
@@ -1344,12 +1346,13 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
     const uint32_t m = src.m;
     for (;;)
     {
+        const unsigned resting = __ballot_sync(0xFFFFFFFFu, part >= kPartMerge);
         if constexpr (kAny)
         {
             if (part == kPartWait && w.settle(E, occluded, lend_wait(L, role, kMaxBisections), have))
                 part = kPartWalk;
         }
-        else if (__ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
+        else if (resting && __ballot_sync(0xFFFFFFFFu, part == kPartMerge || part == kPartWait))
         {
             const LendEnd end = lend_settle(L, part, role, sink, c.found, uint32_t(c.it), kMaxBisections);
             if (end == kEndedRoot) w.keep(L.t[lane_id()], L.u[lane_id()], L.v[lane_id()]);
@@ -1361,7 +1364,7 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
                 role = kAlone;
             }
         }
-        const unsigned idleM = __ballot_sync(0xFFFFFFFFu, part == kPartNone);
+        const unsigned idleM = resting ? __ballot_sync(0xFFFFFFFFu, part == kPartNone) : 0u;
         if (idleM)
         {
             // level j's bit of the trail is bit k - 1 - j: the first level with a 0 bit
@@ -1445,7 +1448,12 @@ __device__ __forceinline__ void subdivide_rays(const DevScene& S, const RaysSoA&
         else
         {
             next = kClipCut;
-            for (int s = 0; s < int(E.subdivLevels) && next == kClipCut; s++) next = subdiv_cut(c, tol2, lc);
+            const int levels = int(E.subdivLevels);
+            for (int s = 0; s < levels; s++)
+            {
+                next = subdiv_cut(c, tol2, lc);
+                if (next != kClipCut) break;
+            }
         }
         if (kAny && c.found) next = kClipOver;  // an any-hit search ends at its first root
         if (next < kClipOver)
