@@ -525,24 +525,26 @@ __device__ __forceinline__ double scale2(double x, int k)
     return __hiloint2double(__double2hiint(x) + k * 0x100000, __double2loint(x));
 }
 
-// Whether x has a significand of all ones.
-__device__ __forceinline__ bool all_ones(double x)
+// The reciprocal y of b by Newton's iteration, rounded to nearest: the iteration
+// is one unit low where b has a significand of all ones (1 / b is 2^-k and a
+// little more than half a unit), right for every other.
+__device__ __forceinline__ double rounded_reciprocal(double y, double b)
 {
-    return ((uint32_t(__double2hiint(x)) | 0xFFF00000u) & uint32_t(__double2loint(x))) == 0xFFFFFFFFu;
+    const bool ones = ((uint32_t(__double2hiint(b)) | 0xFFF00000u) & uint32_t(__double2loint(b))) == 0xFFFFFFFFu;
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0));
 }
 
 // a / b, rounded to nearest: a reciprocal by Newton's iteration from FP32, then
 // the quotient corrected by its remainder (P. W. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34,
-// 1990), which takes a reciprocal rounded to nearest: the iteration gives that
-// for every significand but one of all ones.  Seven FP64 instructions; there, and
+// 1990), which takes a reciprocal rounded to nearest.  Seven FP64 instructions;
 // outside the exponents that this is safe for, the operator.
 __device__ __forceinline__ double quotient(double a, double b)
 {
-    if (exponent_bits(b) - 923u >= 200u || exponent_bits(a) - 523u >= 1000u || all_ones(b)) return a / b;
+    if (exponent_bits(b) - 923u >= 200u || exponent_bits(a) - 523u >= 1000u) return a / b;
     double y = widen(1.0f / narrow(b));
     y = fma(y, fma(-b, y, 1.0), y);
-    y = fma(y, fma(-b, y, 1.0), y);
+    y = rounded_reciprocal(fma(y, fma(-b, y, 1.0), y), b);
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
@@ -567,9 +569,8 @@ __device__ __forceinline__ double2 unit2d(double2 L)
     g = fma(g, r, g);
     h = fma(h, r, h);
     const double l = fma(fma(-g, g, s), h, g);
-    if (all_ones(l)) return make_double2(L.x / l, L.y / l);
     double y = scale2(h, 1);
-    y = fma(y, fma(-l, y, 1.0), y);
+    y = rounded_reciprocal(fma(y, fma(-l, y, 1.0), y), l);
     const double qx = L.x * y, qy = L.y * y;
     return make_double2(fma(fma(-l, qx, L.x), y, qx), fma(fma(-l, qy, L.y), y, qy));
 }
