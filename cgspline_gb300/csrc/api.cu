@@ -390,8 +390,9 @@ template<class T> int adjacent_rows(const T* const* rows, int count, uint32_t n)
 // A host query of at most this many rays goes through page-locked rows of the
 // scene's own, three copies whatever the caller's rows lie in: 33 rays 162 us a
 // query with a copy for each row, 128 us with neighbouring rows copied together
-// where they lie, 117 us so.
-constexpr uint32_t kHostStageRays = 1024;
+// where they lie, 117 us so; at 1,104 rays the rows' own copies are ahead again,
+// 485 us for 492.
+constexpr uint32_t kHostStageRays = 512;
 
 uint32_t* host_stage(cgs_scene* s, uint32_t n)
 {

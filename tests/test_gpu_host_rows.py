@@ -31,7 +31,7 @@ class Rows:
             assert int(self.rt.cudaHostUnregister(p)) == 0
 
 
-@pytest.mark.parametrize("n", [N, N - 1, 33])
+@pytest.mark.parametrize("n", [N, N - 1, 513, 512, 33])
 @pytest.mark.parametrize("any_hit", [False, True])
 def test_rows_of_several_allocations(n, any_hit):
     torch = pytest.importorskip("torch")
@@ -46,8 +46,8 @@ def test_rows_of_several_allocations(n, any_hit):
         rays, out = Rows(torch, 7, locked), Rows(torch, 5, locked)
         try:
             # rows of n: the first of whole pages as they lie; shorter ones at the pages' starts are not neighbours,
-            # so those are laid out end to end within what one row holds
-            if n == 33:
+            # so those are laid out end to end
+            if n < 1000:
                 base, res = rays.array.reshape(-1)[: 7 * n].reshape(7, n), out.array.reshape(-1)[: 5 * n].reshape(5, n)
             else:
                 base, res = rays.array[:, :n], out.array[:, :n]
