@@ -139,16 +139,15 @@ template<class F> void on_host_cores(size_t n, bool parallel, F&& fn)
 }
 
 // BezierSurface::buildBVH (src/rt/Primitive.cu:199-220): per-patch bounds of
-// the 16 projected points and their mean as the centroid.
-// cores: on all of the host's.
-std::vector<Element> surface_elements(const Surface& s, bool cores = false)
+// the 16 projected points and their mean as the centroid, of patches first to last - 1.
+void fill_elements(const Surface& s, std::vector<Element>& el, size_t first, size_t last)
 {
-    std::vector<Element> el(s.patchCount());
-    auto fill = [&](uint32_t i) {
+    for (size_t i = first; i < last; i++)
+    {
         Element& e = el[i];
         e.bounds = Box {};
         e.centroid[0] = e.centroid[1] = e.centroid[2] = 0.0f;
-        e.index = i;
+        e.index = uint32_t(i);
         const float inv = 1.0f / 16.0f;
         for (int j = 0; j < 16; j++)
         {
@@ -157,11 +156,16 @@ std::vector<Element> surface_elements(const Surface& s, bool cores = false)
             e.bounds.inflate(p);
             for (int k = 0; k < 3; k++) e.centroid[k] = e.centroid[k] + inv * p[k];
         }
-    };
-    const size_t chunk = 4096, n = el.size();
-    on_host_cores((n + chunk - 1) / chunk, cores, [&](size_t c) {
-        for (size_t i = c * chunk; i < std::min(n, (c + 1) * chunk); i++) fill(uint32_t(i));
-    });
+    }
+}
+
+// cores: by all of the host's.
+std::vector<Element> surface_elements(const Surface& s, bool cores = false)
+{
+    std::vector<Element> el(s.patchCount());
+    const size_t n = el.size(), chunk = cores ? 4096 : std::max<size_t>(n, 1);
+    on_host_cores((n + chunk - 1) / chunk, cores,
+                  [&](size_t c) { fill_elements(s, el, c * chunk, std::min(n, (c + 1) * chunk)); });
     return el;
 }
 
@@ -439,12 +443,18 @@ void cgs::build_walk_bvh(const Surface& s, HostBVH& out, bool cores)
     for (const Element& e : el)
         for (int k = 0; k < 3; k++)
             if (!std::isfinite(e.bounds.lo[k]) || !std::isfinite(e.bounds.hi[k])) return;
-    out.nodes.resize(2 * el.size() - 1);
-    out.keys.resize(2 * el.size() - 1);
-    const WalkTree tree {out.nodes, out.keys};
-    const WalkTree::Part root {el.data(), el.size(), 1u, 0u};
-    if (cores) tree.build_on_cores(root);
-    else tree.build(root);
+    if (cores)
+    {
+        out.nodes.resize(2 * el.size() - 1);
+        out.keys.resize(2 * el.size() - 1);
+        WalkTree {out.nodes, out.keys}.build_on_cores({el.data(), el.size(), 1u, 0u});
+        return;
+    }
+    // by one core: the nodes in order, each written once (4.5 M patches by 16 cores 172 ms, in place 186 ms)
+    out.build(el);
+    for (Node& n : out.nodes)
+        if (n.left == EMPTY) n.right = out.indices[n.right];  // a leaf names its patch
+    out.indices.clear();
 }
 
 // The walk trees of a store read from a blob: surfaces side by side, and one
