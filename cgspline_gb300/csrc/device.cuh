@@ -107,7 +107,8 @@ __device__ __forceinline__ float3 group_ambient(const DevScene& S, uint32_t g)
 struct Counters
 {
     unsigned long long nodes, hashLookups, candidates, iterations, rays, errors, tableReads;
-    // long candidate lists taken (the query engine's allocator), by each query of the call: a render's of level l are 2 l and 2 l + 1
+    // long candidate lists taken (the query engine's allocator) by each query of the
+    // call: a render's queries of level l are 2 l and 2 l + 1
     uint32_t longNext[2 * (kMaxDepth + 1)];
 };
 
