@@ -2,7 +2,7 @@
 does: many surfaces side by side, one large surface's tree in subtrees; the same
 trees as a build's."""
 import os
-import threading
+import time
 
 import numpy as np
 import pytest
@@ -29,8 +29,8 @@ def store(name):
 def test_walk_trees_of_a_loaded_store_are_built_by_all_cores(name, tmp_path):
     torch = pytest.importorskip("torch")
     from cgspline_gb300 import rt
-    if (os.cpu_count() or 1) < 4:
-        pytest.skip("needs four cores")
+    if (os.cpu_count() or 1) < 8:
+        pytest.skip("needs eight cores")
     sc = store(name)
     g = rt.GpuScene(sc)
     cam = S.camera_c2() if name == "large" else S.Camera(rotation=S.look_at((34.0, -30.0, 40.0), (34.0, 34.0, 0.0)),
@@ -43,23 +43,13 @@ def test_walk_trees_of_a_loaded_store_are_built_by_all_cores(name, tmp_path):
     g.save(path)
     g.close()
     rt.GpuScene.load(path).close()
-    tasks, stop = [], threading.Event()
-
-    def watch():
-        while not stop.is_set():
-            tasks.append(len(os.listdir("/proc/self/task")))
-
-    t = threading.Thread(target=watch)
-    t.start()
-    try:
-        before = len(os.listdir("/proc/self/task"))
-        h = rt.GpuScene.load(path)
-    finally:
-        stop.set()
-        t.join()
+    # processor time over elapsed time: 1.0 and 1.2 where one thread does it, 2.8 and 3.9 on 16 cores
+    wall, cpu = time.perf_counter(), time.process_time()
+    h = rt.GpuScene.load(path)
+    wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
     got = {k: v.cpu().numpy() for k, v in h.intersect(rays).items()}
     assert h.counters()["nodes"] == nodes
     h.close()
     for k in want:
         assert np.array_equal(got[k], want[k]), k
-    assert max(tasks) >= before + 3, (max(tasks), before)
+    assert cpu >= 1.7 * wall, (cpu, wall)
